@@ -486,6 +486,11 @@ int mul_dev_len(const u32* a, long long la, const u32* b, long long lb, u32* h, 
         lh = n;
     }
     const u32 root = canonical_root(pc, logn);
+    if (logn <= kMaxLatencyLog) {
+        bool launched = false;
+        err = latency_mul(pc, logn, dev, ProdJob{a, b, h, (int)la, (int)lb, (int)lh, 0}, st, &launched);
+        if (err != OK || launched) return err;
+    }
     if (logn <= kMaxSmallLog && logn < single_large_min_log()) {
         SmallArgs A;
         if ((err = small_args(pc, root, logn, dev, &A)) != OK) return err;

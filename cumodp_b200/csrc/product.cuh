@@ -1,6 +1,7 @@
 // Host-side product dispatch shared by the C entry points.
 #pragma once
 #include "large_product.cuh"
+#include "latency_product.cuh"
 #include "runtime.cuh"
 
 namespace cmb {
@@ -41,6 +42,23 @@ bool launch_col_fwd_pipe(const LargeArgs& a, int njobs, cudaStream_t st);
 bool launch_col_fwd_pipe1(const LargeArgs& a, int njobs, cudaStream_t st);
 void launch_small(int logn, const SmallArgs& a, int njobs, cudaStream_t st);
 void launch_large(const LargeArgs& a, int njobs, cudaStream_t st);
+
+// A single product of transform length 2^logn (kMinLog <= logn <=
+// kMaxLatencyLog) in one launch (latency_product.cuh); *launched = false when
+// the device cannot run it (no room for a cluster of 16 CTAs) and the caller
+// takes the other kernels.  The limit is what a cluster's shared memory holds;
+// at 2^16 the one launch takes 11.5 us and the three-pass kernels 14.8.
+constexpr int kMaxLatencyLog = 16;
+int latency_mul(const PrimeCtx& pc, int logn, int dev, const ProdJob& job, cudaStream_t st, bool* launched);
+// Products of the same lengths mod np (3 or 4) primes: prime r's operands at
+// a + r astride, b + r bstride, its la + lb - 1 residues at h + r hstride.
+int latency_mul_primes(const u32* primes, int np, int dev, const u32* a, int la, long long astride, const u32* b, int lb,
+                       long long bstride, u32* h, long long hstride, cudaStream_t st, bool* launched);
+// The same for two signed 64-bit operands mod np (2 or 3) primes in one
+// launch: prime r's la + lb - 1 residues at h + r (la + lb - 1).  *launched =
+// false past 2^kMaxLatencyLog too.
+int latency_mul_i64(const u32* primes, int np, int dev, const long long* a, int la, const long long* b, int lb, u32* h,
+                    cudaStream_t st, bool* launched);
 
 // Sets the shared-memory limits of every product kernel once (must run
 // before any launch is captured into a graph).

@@ -8,6 +8,8 @@
 // scratch buffers grow once and are reused.
 #include "runtime.cuh"
 
+#include "latency_product.cuh"
+
 #include <atomic>
 #include <cstdio>
 #include <map>
@@ -259,6 +261,58 @@ static cudaError_t upload_now(void* d, const void* h, size_t bytes) {
     cudaError_t e = cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     return e;
+}
+
+namespace {
+
+// One level's entries in the layout [slot j][task o < tasks]: w^(o bitrev(j)),
+// row by row with one product per entry.
+void push_slot_major(std::vector<Tw>& t, u32 w, int logr, int tasks, u32 p) {
+    for (int j = 0; j < 1 << logr; ++j) {
+        const u32 step = powmod_exact(w, bitrev((u32)j, logr), p);
+        u32 v = 1;
+        for (int o = 0; o < tasks; ++o) {
+            t.push_back(tw_of(v, p));
+            v = mulmod_exact(v, step, p);
+        }
+    }
+}
+
+}  // namespace
+
+const Tw* latency_tables(int dev, u32 p, u32 root, int logn, int logl, int* err) {
+    Caches& C = caches();
+    std::lock_guard<std::mutex> g(C.m);
+    auto key = std::make_tuple(dev, p, root, logn, 2);
+    auto it = C.tables.find(key);
+    if (it != C.tables.end()) return it->second;
+    const LevelPlan pl = lat_plan(logl);
+    std::vector<Tw> t;
+    const u32 rinv = powmod_exact(root, (1ull << logn) - 1, p);
+    for (u32 w : {root, rinv}) {
+        int lb = logl;
+        for (int i = 0; i + 1 < pl.nlev; ++i) {
+            push_slot_major(t, powmod_exact(w, 1ull << (logn - lb), p), pl.logr[i], 1 << (lb - pl.logr[i]), p);
+            lb -= pl.logr[i];
+        }
+    }
+    if (logl < logn)
+        for (u32 w : {root, rinv}) push_slot_major(t, w, logn - logl, 1 << logl, p);
+    Tw* d = nullptr;
+    if (dev_malloc((void**)&d, t.size() * sizeof(Tw)) != cudaSuccess) {
+        cudaGetLastError();
+        *err = OUT_OF_MEMORY;
+        return nullptr;
+    }
+    if (upload_now(d, t.data(), t.size() * sizeof(Tw)) != cudaSuccess) {
+        cudaGetLastError();
+        cudaFree(d);
+        *err = FFT_ERROR;
+        return nullptr;
+    }
+    C.bytes += (long long)(t.size() * sizeof(Tw));
+    C.tables[key] = d;
+    return d;
 }
 
 static const Tw* level_tables(int dev, u32 p, u32 root, int logl, int kind, int* err) {

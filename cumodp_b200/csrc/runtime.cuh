@@ -55,6 +55,10 @@ Tw tw_of(u32 w, u32 p);
 const Tw* row_tables(int dev, u32 p, u32 root, int logl, int* err);
 // Same for the interleaved-column plan.
 const Tw* col_tables(int dev, u32 p, u32 root, int logl, int* err);
+// Tables of the one-launch product of length 2^logn (latency_product.cuh):
+// the block tables of 2^logl words (forward, inverse), then, when logl <
+// logn, the leading level's 2 x 2^logn entries.
+const Tw* latency_tables(int dev, u32 p, u32 root, int logn, int logl, int* err);
 // Inter-pass twiddle seeds for a two-pass transform of length 2^logn:
 // lo[e] = w^e (e < 2^12) and hi[e] = w^(e << 12) (e < 2^(logn-12)), both in
 // Montgomery form times R (w^e * 2^64 mod p) so that one Montgomery product

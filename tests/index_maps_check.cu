@@ -17,6 +17,8 @@
 //            its two entries inside the table, the two digits recompose the
 //            task index, and the row kernels' shared memory fits the SM;
 //   pipelined column pass: stage, tile and twiddle indexes in bounds;
+//   one-launch products: padded addresses in bounds and distinct, level tasks cover
+//            each block once, twiddle reads in bounds, shared memory fits;
 //   Shoup quotients from the double estimate equal floor(w 2^32 / p);
 //   the quad-interleaved row spectrum is a permutation with warp-contiguous runs;
 //   the natural-order reorder buffer's swizzle is a bijection without store conflicts.
@@ -25,6 +27,7 @@
 #include <vector>
 
 #include "../cumodp_b200/csrc/large_product.cuh"
+#include "../cumodp_b200/csrc/latency_product.cuh"
 
 using namespace cmb;
 
@@ -324,7 +327,62 @@ void shoup_quot_check() {
     }
 }
 
+template <int LOGL>
+void latency_check(int cluster) {
+    constexpr int L = 1 << LOGL;
+    const LevelPlan pl = lat_plan(LOGL);
+    std::vector<int> used((size_t)lat_words(LOGL), 0);
+    for (int i = 0; i < L; ++i) {
+        CHECK(lat_pad(i) < lat_words(LOGL), "latency L=%d pad out of range", LOGL);
+        CHECK(used[(size_t)lat_pad(i)]++ == 0, "latency L=%d pad collides", LOGL);
+    }
+    int lb = LOGL, off = 0;
+    for (int lev = 0; lev < pl.nlev; ++lev) {
+        const int R = 1 << pl.logr[lev], B = 1 << lb, TB = B / R;
+        std::vector<int> seen((size_t)L, 0);
+        for (int id = 0; id < L / R; ++id) {
+            const int o = id % TB, base = (id / TB) * B + o;
+            for (int m = 0; m < R; ++m) {
+                CHECK(base + TB * m < L, "latency L=%d level %d out of range", LOGL, lev);
+                ++seen[(size_t)(base + TB * m)];
+                if (lev + 1 < pl.nlev) CHECK(off + m * TB + o < lat_entries(LOGL), "latency L=%d twiddle", LOGL);
+            }
+        }
+        for (int v : seen) CHECK(v == 1, "latency L=%d level %d coverage", LOGL, lev);
+        if (lev + 1 < pl.nlev) off += B;
+        lb -= pl.logr[lev];
+    }
+    CHECK(lb == 0 && pl.logr[pl.nlev - 1] == 3 && off == lat_entries(LOGL), "latency L=%d plan", LOGL);
+    CHECK(lat_smem(LOGL, cluster) <= 227 * 1024, "latency L=%d shared memory", LOGL);
+    CHECK(2 * L % lat_threads(LOGL) == 0, "latency L=%d load loop", LOGL);
+    if (cluster > 1) {
+        // words on their way home: block j's word i reaches CTA i / CH at j CH + i % CH
+        const int CH = L / kClusterCtas;
+        CHECK(2 * CH <= lat_threads(LOGL), "latency L=%d leading tasks", LOGL);
+        std::vector<int> home((size_t)kClusterCtas * L, 0);
+        for (int j = 0; j < kClusterCtas; ++j)
+            for (int i = 0; i < L; ++i) {
+                const int at = j * CH + i % CH;
+                CHECK(at < L, "latency L=%d home", LOGL);
+                ++home[(size_t)(i / CH) * L + at];
+            }
+        for (int v : home) CHECK(v == 1, "latency L=%d home coverage", LOGL);
+    }
+}
+
 int main() {
+    latency_check<5>(1);
+    latency_check<6>(1);
+    latency_check<7>(1);
+    latency_check<8>(1);
+    latency_check<9>(1);
+    latency_check<10>(1);
+    latency_check<11>(1);
+    latency_check<8>(16);
+    latency_check<9>(16);
+    latency_check<10>(16);
+    latency_check<11>(16);
+    latency_check<12>(16);
     row_plan_check<5>();
     row_plan_check<6>();
     row_plan_check<7>();
