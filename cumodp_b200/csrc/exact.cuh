@@ -28,6 +28,11 @@ int twoconv_plan(int ba, int bb, long long la, long long lb, bool force_two_prim
 int twoconv_mul_dev(const long long* a, long long la, const long long* b, long long lb, long long* c, int ba,
                     int bb, bool force_two_prime, cudaStream_t st, TwoConvPlan* used, const TwoConvBufs* bufs);
 
+// The signed 128-bit integers (lo, hi pairs) whose residues mod p[r] < 2^30, r
+// < np <= 3, are c[r lc + i]; pdl: the launch may be scheduled while the
+// kernel before it on st finishes (programmatic dependent launch).
+int launch_lift(const u32* c, long long lc, const u32* p, int np, long long* out, bool pdl, cudaStream_t st);
+
 // The same product for lengths past the reference primes' transforms
 // (twoconv_plan: FFT_SIZE_TOO_LARGE): the big-coefficient path with one
 // 64-bit word per input coefficient and two per output coefficient, over

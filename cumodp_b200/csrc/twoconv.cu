@@ -19,11 +19,16 @@
 //      points), so the x-convolutions become 2K independent y-products;
 //   2. the y-products: one batched call per prime (fused single-CTA or
 //      three-pass kernels, graph-launched);
+//      (K = 1 products of up to 2^16 points: steps 1 and 2 are one launch,
+//      latency_mul_i64, a cluster of CTAs per prime reducing the operands as
+//      it reads them: degree 8191 in 9.1 us; before, two splits, three graph
+//      launches on side streams and the lift took 40.2)
 //   3. k_crt_recombine: per output coefficient, the inverse 2K-point
 //      x-transform, u and v, (u+v) and (u-v) mod each prime, the signed CRT
 //      lift, evaluation at 2^M and the final shift, stored as a signed
 //      128-bit integer (lo, hi words).
-// K = 1 is the degenerate case with no limb split (u = v = the product).
+// K = 1 is the degenerate case with no limb split (u = v = the product): its
+// residues (k_residues) and signed lift (k_lift) are kernels of their own.
 // The planner picks the cheapest (K, M, primes) whose exactness bound holds.
 #include <algorithm>
 #include <cmath>
@@ -44,8 +49,7 @@ static const u32 kTwoConvPrimes[3] = {962592769u, 950009857u, 940572673u};
 struct SplitArgs {
     const long long* x;
     int len;
-    int K, M;
-    int npts;            // evaluation points: 2K, or 1 when K = 1
+    int K, M;            // K = 2 or 4
     int nprimes;
     u32 p[3];
     u32 zeta_pow[3][8];  // zeta^t, t < 2K (K <= 4)
@@ -58,7 +62,7 @@ __global__ void k_split_eval(const __grid_constant__ SplitArgs A) {
     const long long v = A.x[i];
     const bool neg = v < 0;
     const unsigned long long m = neg ? 0ull - (unsigned long long)v : (unsigned long long)v;
-    const int twoK = 2 * A.K, npts = A.npts;
+    const int twoK = 2 * A.K;
     const unsigned long long mask = A.M >= 64 ? ~0ull : ((1ull << A.M) - 1);
     for (int r = 0; r < A.nprimes; ++r) {
         const u32 p = A.p[r];
@@ -68,10 +72,10 @@ __global__ void k_split_eval(const __grid_constant__ SplitArgs A) {
             const u32 lr = (u32)(l % p);
             limb[j] = (neg && lr) ? p - lr : lr;
         }
-        for (int s = 0; s < npts; ++s) {
+        for (int s = 0; s < twoK; ++s) {
             u64 acc = 0;
             for (int j = 0; j < A.K; ++j) acc += (u64)limb[j] * A.zeta_pow[r][(j * s) % twoK] % p;
-            A.out[((size_t)r * npts + s) * A.len + i] = (u32)(acc % p);
+            A.out[((size_t)r * twoK + s) * A.len + i] = (u32)(acc % p);
         }
     }
 }
@@ -80,7 +84,6 @@ struct CrtArgs {
     const u32* c;   // [prime][s][lc]
     int lc;
     int K, M, nprimes;
-    int npts;
     u32 p[3];
     u32 zinv_pow[3][8];  // zeta^-t
     u32 inv2k[3];        // (2K)^-1 mod p
@@ -113,23 +116,18 @@ __device__ __forceinline__ __int128 crt_signed(const u32* r, const CrtArgs& A) {
 __global__ void k_crt_recombine(const __grid_constant__ CrtArgs A) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= A.lc) return;
-    const int K = A.K, twoK = 2 * K, npts = A.npts;
+    const int K = A.K, twoK = 2 * K;
     u32 S[3][4], D[3][4];
     for (int r = 0; r < A.nprimes; ++r) {
         const u32 p = A.p[r];
         u32 cs[8], c[8];
-        for (int s = 0; s < npts; ++s) cs[s] = A.c[((size_t)r * npts + s) * A.lc + i];
-        if (K == 1) {  // no limb split: the single product is c_0, and c_1 = 0
-            c[0] = cs[0];
-            c[1] = 0;
-        } else {
-            // inverse 2K-point x-transform: c_j = (2K)^-1 sum_s cs_s zeta^-js
-            // (the acyclic x-product, degree 2K-2)
-            for (int j = 0; j < twoK; ++j) {
-                u64 acc = 0;
-                for (int s = 0; s < twoK; ++s) acc += (u64)cs[s] * A.zinv_pow[r][(j * s) % twoK] % p;
-                c[j] = (u32)((acc % p) * A.inv2k[r] % p);
-            }
+        for (int s = 0; s < twoK; ++s) cs[s] = A.c[((size_t)r * twoK + s) * A.lc + i];
+        // inverse 2K-point x-transform: c_j = (2K)^-1 sum_s cs_s zeta^-js
+        // (the acyclic x-product, degree 2K-2)
+        for (int j = 0; j < twoK; ++j) {
+            u64 acc = 0;
+            for (int s = 0; s < twoK; ++s) acc += (u64)cs[s] * A.zinv_pow[r][(j * s) % twoK] % p;
+            c[j] = (u32)((acc % p) * A.inv2k[r] % p);
         }
         for (int j = 0; j < K; ++j) {
             // cyclic u_j = c_j + c_{j+K}, negacyclic v_j = c_j - c_{j+K};
@@ -153,6 +151,84 @@ __global__ void k_crt_recombine(const __grid_constant__ CrtArgs A) {
     const __int128 prod = acc / 2;  // exact: acc is even
     A.out[2 * (size_t)i] = (long long)(unsigned long long)(unsigned __int128)prod;
     A.out[2 * (size_t)i + 1] = (long long)(prod >> 64);
+}
+
+// One limb (K = 1, one evaluation point): both operands' residues in one
+// launch, out[r len + i] for a then [r len + i] for b.  A residue is two Shoup
+// products (the 32-bit halves), not a 64-bit division.
+struct ResidueArgs {
+    const long long *a, *b;
+    int la, lb, nprimes;
+    u32 p[3], oneq[3];
+    Tw r32[3];  // 2^32 mod p
+    u32 *ea, *eb;
+};
+
+__global__ void __launch_bounds__(256) k_residues(const __grid_constant__ ResidueArgs A) {
+    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (t >= (long long)A.la + A.lb) return;
+    const bool second = t >= A.la;
+    const int i = (int)(second ? t - A.la : t), len = second ? A.lb : A.la;
+    const long long v = (second ? A.b : A.a)[i];
+    const u64 m = v < 0 ? 0ull - (u64)v : (u64)v;
+    u32* out = (second ? A.eb : A.ea) + i;
+    for (int r = 0; r < A.nprimes; ++r) {
+        const u32 p = A.p[r];
+        const u32 x = mul_shoup((u32)m, 1u, A.oneq[r], p) + mul_shoup((u32)(m >> 32), A.r32[r].w, A.r32[r].wq, p);
+        const u32 c = red1(red2(x, 2 * p), p);
+        out[(size_t)r * len] = v < 0 && c ? p - c : c;
+    }
+}
+
+// Signed lift of NP residues (c[r lc + i], canonical) to 128 bits, one
+// coefficient per thread: Garner's digits by Shoup products, then
+// v0 + v1 p0 + v2 p0 p1 in 128 bits, less P above P / 2; no division.
+struct LiftArgs {
+    const u32* c;
+    long long* out;  // (lo, hi) per coefficient
+    int lc;
+    u32 p[3], oneq[3];
+    Tw g1;      // p0^-1 mod p1
+    Tw g2;      // (p0 p1)^-1 mod p2
+    Tw p0m2;    // p0 mod p2
+    u64 p01;    // p0 p1
+    u64 half_lo, half_hi, full_lo, full_hi;  // floor(P / 2) and P
+};
+
+template <int NP>
+__global__ void __launch_bounds__(256) k_lift(const __grid_constant__ LiftArgs A) {
+    pdl_wait();  // the products
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= A.lc) return;
+    const u32 v0 = A.c[i];
+    u64 lo = v0, hi = 0;
+    if constexpr (NP >= 2) {
+        const u32 p1 = A.p[1];
+        // v1 = (r1 - v0) / p0 mod p1; v0 reduced below p1 first
+        const u32 d = A.c[(size_t)A.lc + i] + p1 - red1(mul_shoup(v0, 1u, A.oneq[1], p1), p1);
+        const u32 v1 = red1(mul_shoup(d, A.g1.w, A.g1.wq, p1), p1);
+        lo += (u64)v1 * A.p[0];  // < p0 p1 < 2^60
+        if constexpr (NP == 3) {
+            const u32 p2 = A.p[2];
+            // v2 = (r2 - v0 - v1 p0) / (p0 p1) mod p2
+            const u32 s = red1(mul_shoup(v0, 1u, A.oneq[2], p2), p2) + red1(mul_shoup(v1, A.p0m2.w, A.p0m2.wq, p2), p2);
+            const u32 e = A.c[2 * (size_t)A.lc + i] + 2 * p2 - s;  // in (0, 3 p2) < 2^32
+            const u32 v2 = red1(mul_shoup(e, A.g2.w, A.g2.wq, p2), p2);
+            const u64 ml = (u64)v2 * A.p01, mh = __umul64hi((u64)v2, A.p01);
+            lo += ml;
+            hi = mh + (lo < ml);
+        }
+    }
+    if (hi > A.half_hi || (hi == A.half_hi && lo > A.half_lo)) {
+        hi = hi - A.full_hi - (lo < A.full_lo);
+        lo -= A.full_lo;
+    }
+    if ((reinterpret_cast<uintptr_t>(A.out) & 15) == 0) {
+        reinterpret_cast<ulonglong2*>(A.out)[i] = make_ulonglong2(lo, hi);
+    } else {
+        A.out[2 * (size_t)i] = (long long)lo;
+        A.out[2 * (size_t)i + 1] = (long long)hi;
+    }
 }
 
 namespace {
@@ -223,6 +299,110 @@ void twoconv_buffer_sizes(long long la, long long lb, size_t* eval_words, size_t
     *job_bytes = (size_t)np * direct_job_bytes(npts);
 }
 
+int launch_lift(const u32* ec, long long lc, const u32* p, int np, long long* c, bool pdl, cudaStream_t st) {
+    LiftArgs A;
+    memset(&A, 0, sizeof(A));
+    A.c = ec;
+    A.out = c;
+    A.lc = (int)lc;
+    for (int r = 0; r < np; ++r) {
+        A.p[r] = p[r];
+        A.oneq[r] = shoup_quot(1, p[r]);
+    }
+    if (np >= 2) {
+        A.g1 = tw_of(powmod_exact(p[0] % p[1], p[1] - 2, p[1]), p[1]);
+        A.p01 = (u64)p[0] * p[1];
+    }
+    if (np == 3) {
+        A.g2 = tw_of(powmod_exact((u32)(A.p01 % p[2]), p[2] - 2, p[2]), p[2]);
+        A.p0m2 = tw_of(p[0] % p[2], p[2]);
+    }
+    unsigned __int128 P = 1;
+    for (int r = 0; r < np; ++r) P *= p[r];
+    A.full_lo = (u64)P;
+    A.full_hi = (u64)(P >> 64);
+    A.half_lo = (u64)(P >> 1);
+    A.half_hi = (u64)(P >> 65);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)((lc + 255) / 256));
+    cfg.blockDim = dim3(256);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl ? 1 : 0;
+    return cuda_err(cudaLaunchKernelEx(&cfg, np == 3 ? k_lift<3> : np == 2 ? k_lift<2> : k_lift<1>, A));
+}
+
+namespace {
+
+// K > 1: the launch arguments of the split and recombine kernels, and both
+// operands' evaluations.
+int split_operands(const TwoConvPlan& pl, const long long* a, long long la, const long long* b, long long lb, u32* ea,
+                   u32* eb, SplitArgs* sa, CrtArgs* ca, cudaStream_t st) {
+    const int twoK = 2 * pl.K, np = pl.nprimes;
+    int err = OK;
+    memset(sa, 0, sizeof(*sa));
+    sa->K = pl.K;
+    sa->M = pl.M;
+    sa->nprimes = np;
+    memset(ca, 0, sizeof(*ca));
+    ca->K = pl.K;
+    ca->M = pl.M;
+    ca->nprimes = np;
+    for (int r = 0; r < np; ++r) {
+        const u32 p = kTwoConvPrimes[r];
+        const PrimeCtx* pc = prime_ctx(p, &err);
+        if (!pc) return err;
+        const u32 zeta = canonical_root(*pc, twoK == 2 ? 1 : (twoK == 4 ? 2 : 3));
+        const u32 zinv = powmod_exact(zeta, twoK - 1, p);
+        sa->p[r] = ca->p[r] = p;
+        for (int t = 0; t < twoK; ++t) {
+            sa->zeta_pow[r][t] = powmod_exact(zeta, t, p);
+            ca->zinv_pow[r][t] = powmod_exact(zinv, t, p);
+        }
+        ca->inv2k[r] = powmod_exact(twoK, p - 2, p);
+    }
+    ca->garner1 = powmod_exact(kTwoConvPrimes[0] % kTwoConvPrimes[1], kTwoConvPrimes[1] - 2, kTwoConvPrimes[1]);
+    ca->garner2 = powmod_exact(
+        (u32)((u64)kTwoConvPrimes[0] * kTwoConvPrimes[1] % kTwoConvPrimes[2]), kTwoConvPrimes[2] - 2,
+        kTwoConvPrimes[2]);
+    sa->x = a;
+    sa->len = (int)la;
+    sa->out = ea;
+    k_split_eval<<<(unsigned)((la + 255) / 256), 256, 0, st>>>(*sa);
+    sa->x = b;
+    sa->len = (int)lb;
+    sa->out = eb;
+    k_split_eval<<<(unsigned)((lb + 255) / 256), 256, 0, st>>>(*sa);
+    return cuda_err(cudaGetLastError());
+}
+
+// K = 1: both operands' residues.
+int launch_residues(const long long* a, long long la, const long long* b, long long lb, int np, u32* ea, u32* eb,
+                    cudaStream_t st) {
+    ResidueArgs A;
+    memset(&A, 0, sizeof(A));
+    A.a = a;
+    A.b = b;
+    A.la = (int)la;
+    A.lb = (int)lb;
+    A.nprimes = np;
+    for (int r = 0; r < np; ++r) {
+        const u32 p = kTwoConvPrimes[r];
+        A.p[r] = p;
+        A.oneq[r] = shoup_quot(1, p);
+        A.r32[r] = tw_of((u32)((1ull << 32) % p), p);
+    }
+    A.ea = ea;
+    A.eb = eb;
+    k_residues<<<(unsigned)((la + lb + 255) / 256), 256, 0, st>>>(A);
+    return cuda_err(cudaGetLastError());
+}
+
+}  // namespace
+
 // c (lo, hi pairs, la+lb-1 coefficients) = a * b exactly; device pointers.
 // bufs == nullptr: library workspace and graph-launched batches.
 int twoconv_mul_dev(const long long* a, long long la, const long long* b, long long lb, long long* c, int ba,
@@ -244,43 +424,18 @@ int twoconv_mul_dev(const long long* a, long long la, const long long* b, long l
     u32* ea = ws;
     u32* eb = ea + (size_t)np * npts * la;
     u32* ec = eb + (size_t)np * npts * lb;
+    bool products_done = false;
     SplitArgs sa;
-    memset(&sa, 0, sizeof(sa));
-    sa.K = pl.K;
-    sa.M = pl.M;
-    sa.npts = npts;
-    sa.nprimes = np;
     CrtArgs ca;
-    memset(&ca, 0, sizeof(ca));
-    ca.K = pl.K;
-    ca.M = pl.M;
-    ca.npts = npts;
-    ca.nprimes = np;
-    for (int r = 0; r < np; ++r) {
-        const u32 p = kTwoConvPrimes[r];
-        const PrimeCtx* pc = prime_ctx(p, &err);
-        if (!pc) return err;
-        const u32 zeta = canonical_root(*pc, twoK == 2 ? 1 : (twoK == 4 ? 2 : 3));
-        const u32 zinv = powmod_exact(zeta, twoK - 1, p);
-        sa.p[r] = ca.p[r] = p;
-        for (int t = 0; t < twoK; ++t) {
-            sa.zeta_pow[r][t] = powmod_exact(zeta, t, p);
-            ca.zinv_pow[r][t] = powmod_exact(zinv, t, p);
-        }
-        ca.inv2k[r] = powmod_exact(twoK, p - 2, p);
+    if (pl.K == 1) {
+        // up to 2^16 points one launch reduces both operands and multiplies
+        // them mod every prime; otherwise the residues go through memory
+        err = latency_mul_i64(kTwoConvPrimes, np, dev, a, (int)la, b, (int)lb, ec, st, &products_done);
+        if (err != OK) return err;
+        if (!products_done && (err = launch_residues(a, la, b, lb, np, ea, eb, st)) != OK) return err;
+    } else {
+        if ((err = split_operands(pl, a, la, b, lb, ea, eb, &sa, &ca, st)) != OK) return err;
     }
-    ca.garner1 = powmod_exact(kTwoConvPrimes[0] % kTwoConvPrimes[1], kTwoConvPrimes[1] - 2, kTwoConvPrimes[1]);
-    ca.garner2 = powmod_exact(
-        (u32)((u64)kTwoConvPrimes[0] * kTwoConvPrimes[1] % kTwoConvPrimes[2]), kTwoConvPrimes[2] - 2,
-        kTwoConvPrimes[2]);
-    sa.x = a;
-    sa.len = (int)la;
-    sa.out = ea;
-    k_split_eval<<<(unsigned)((la + 255) / 256), 256, 0, st>>>(sa);
-    sa.x = b;
-    sa.len = (int)lb;
-    sa.out = eb;
-    k_split_eval<<<(unsigned)((lb + 255) / 256), 256, 0, st>>>(sa);
     // y-products: one per evaluation point and prime
     std::vector<sfixn> df(npts, (sfixn)(la - 1)), dg(npts, (sfixn)(lb - 1));
     std::vector<int64_t> fo(npts), go(npts), ho(npts);
@@ -289,7 +444,9 @@ int twoconv_mul_dev(const long long* a, long long la, const long long* b, long l
         go[s] = (int64_t)s * lb;
         ho[s] = (int64_t)s * lc;
     }
-    if (!bufs) {
+    if (products_done) {
+        // residues of every prime are in ec
+    } else if (!bufs) {
         // the primes are independent: one side stream each (each batch plan
         // owns its workspace), joined before the CRT
         aux_fork(dev, st, np);
@@ -321,6 +478,7 @@ int twoconv_mul_dev(const long long* a, long long la, const long long* b, long l
             if (err != OK) return err;
         }
     }
+    if (pl.K == 1) return launch_lift(ec, lc, kTwoConvPrimes, np, c, products_done, st);
     ca.c = ec;
     ca.lc = (int)lc;
     ca.out = c;
