@@ -13,20 +13,19 @@
 // Here the coefficients travel as fixed-width two's-complement words (no GMP
 // on either side of the boundary) and the whole computation stays on the
 // GPU:
-//   1. k_big_abs: |a_j| and its sign, one thread per coefficient;
-//   2. k_big_split: per prime, the Kronecker layout A_p[j*(2K-1) + i] =
-//      sign_j * limb_i(|a_j|) mod p for i < K and 0 for K <= i < 2K-1, one
-//      thread per word.  The zero tail of every block keeps the
+//   1. k_big_split: per prime, the Kronecker layout A_p[j*(2K-1) + i] =
+//      sign_j * limb_i(|a_j|) mod p for i < K and 0 for K <= i < 2K-1, both
+//      operands in one launch, one thread per word.  The zero tail of every block keeps the
 //      (2K-1)-coefficient linear x-convolution of two K-limb numbers inside
 //      its block, so one univariate product per prime equals the bivariate
 //      product (about the total transform length of a cyclic plus a
 //      negacyclic convolution of length K);
-//   3. one univariate product per prime (fused single-CTA or three-pass
-//      kernels);
-//   4. k_big_crt: per output coefficient, Garner's CRT of every x-coefficient
-//      to a signed 128-bit integer and the sum of them shifted by M*i bits,
-//      in separate positive and negative multiword accumulators, stored as
-//      out_words two's-complement words.
+//   2. one univariate product per prime (one launch for all of them up to
+//      2^16 points, else three-pass kernels);
+//   3. k_big_sum (one warp per output coefficient) or k_big_crt (one thread,
+//      few limbs): Garner's CRT of every x-coefficient to a signed 128-bit
+//      integer and the sum of them shifted by M*i bits, stored as out_words
+//      two's-complement words; a single limb over three primes is k_lift.
 // The planner picks the number of primes (3 or 4) and the limb width M with
 // the cheapest transform such that every x-coefficient satisfies
 // K * min(la, lb) * (2^M - 1)^2 < P / 2.
@@ -117,65 +116,53 @@ int big_out_words(long long na, long long nb, int bw) {
     return (bits + 63) / 64;
 }
 
-// |x_j| (in_words words) and sign, one coefficient per thread and step of a
-// grid-stride loop (the grid is capped by grid_of).
-__global__ void k_big_abs(const unsigned long long* __restrict__ x, long long len, int words,
-                          unsigned long long* __restrict__ mag, unsigned char* __restrict__ neg) {
-    for (long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x; j < len;
-         j += (long long)gridDim.x * blockDim.x) {
-        const unsigned long long* w = x + j * words;
-        unsigned long long* m = mag + j * words;
-        const bool s = (long long)w[words - 1] < 0;
-        unsigned long long carry = 1;
-        for (int i = 0; i < words; ++i) {
-            if (s) {
-                const unsigned long long v = ~w[i] + carry;
-                carry = (carry && v == 0) ? 1 : 0;
-                m[i] = v;
-            } else {
-                m[i] = w[i];
-            }
-        }
-        neg[j] = s ? 1 : 0;
-    }
-}
-
 struct BigSplitArgs {
-    const unsigned long long* mag;
-    const unsigned char* neg;
-    long long len;  // coefficients
+    const unsigned long long *xa, *xb;  // coefficients of in-words two's-complement words
+    u32 ta, tb;                         // layout words of each operand
     int words, K, M, nprimes;
-    u32 p[kBigMaxPrimes];
-    u32* out[kBigMaxPrimes];  // (2K - 1)(len - 1) + K words each
+    u32 p[kBigMaxPrimes], oneq[kBigMaxPrimes];
+    Tw r32[kBigMaxPrimes];  // 2^32 mod p
+    u32 *outa[kBigMaxPrimes], *outb[kBigMaxPrimes];
 };
 
 // out_p[j*(2K-1) + i] = sign_j * (bits [M i, M i + M) of |x_j|) mod p, i < K;
-// 0 for K <= i < 2K-1 (the last block is cut at K words).
-__global__ void k_big_split(const __grid_constant__ BigSplitArgs A) {
-    const int blk = 2 * A.K - 1;
-    const long long total = (long long)blk * (A.len - 1) + A.K;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-         t += (long long)gridDim.x * blockDim.x) {
-        const long long j = t / blk;
-        const int i = (int)(t % blk);
-        unsigned long long limb = 0;
-        if (i < A.K) {
-            const long long s = (long long)A.M * i;
-            const int w = (int)(s >> 6), b = (int)(s & 63);
-            const unsigned long long* m = A.mag + j * A.words;
-            if (w < A.words) {
-                limb = m[w] >> b;
-                if (b && w + 1 < A.words) limb |= m[w + 1] << (64 - b);
-                if (A.M < 64) limb &= (1ull << A.M) - 1;
+// 0 for K <= i < 2K-1 (the last block is cut at K words); both operands in
+// one launch, one layout word per thread.  |x| of a negative x is ~x + 1: the
+// 1 reaches word w when every lower word of x is zero, which the first lower
+// word nearly always settles.  A limb's residue is two Shoup products.
+__global__ void __launch_bounds__(256) k_big_split(const __grid_constant__ BigSplitArgs A) {
+    u32 t = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool second = t >= A.ta;
+    if (second) t -= A.ta;
+    if (second && t >= A.tb) return;
+    const u32 blk = 2 * A.K - 1, j = t / blk;
+    const int i = (int)(t - j * blk);
+    const unsigned long long* x = (second ? A.xb : A.xa) + (size_t)j * A.words;
+    const bool neg = (long long)x[A.words - 1] < 0;
+    unsigned long long limb = 0;
+    if (i < A.K) {
+        const int s = A.M * i, w = s >> 6, b = s & 63;
+        if (w < A.words) {
+            unsigned long long m0 = x[w], m1 = w + 1 < A.words ? x[w + 1] : (neg ? ~0ull : 0ull);
+            if (neg) {
+                int k = 0;
+                while (k < w && x[k] == 0) ++k;
+                const unsigned long long c0 = k == w;
+                m1 = ~m1 + (c0 && m0 == 0);
+                m0 = ~m0 + c0;
             }
+            limb = m0 >> b;
+            if (b) limb |= m1 << (64 - b);
+            limb &= (1ull << A.M) - 1;  // M <= 62
         }
-        const bool ng = A.neg[j] != 0;
-        for (int k = 0; k < A.nprimes; ++k) {
-            const u32 p = A.p[k];
-            u32 r = (u32)(limb % p);
-            if (ng && r) r = p - r;
-            A.out[k][t] = r;
-        }
+    }
+    for (int k = 0; k < A.nprimes; ++k) {
+        const u32 p = A.p[k];
+        const u32 r = red1(red2(mul_shoup((u32)limb, 1u, A.oneq[k], p) +
+                                    mul_shoup((u32)(limb >> 32), A.r32[k].w, A.r32[k].wq, p),
+                                2 * p),
+                           p);
+        (second ? A.outb[k] : A.outa[k])[t] = neg && r ? p - r : r;
     }
 }
 
@@ -257,28 +244,167 @@ __global__ void k_big_crt(const __grid_constant__ BigCrtArgs A) {
     }
 }
 
+// The same sums with one warp per output coefficient (K > kBigThreadK): lane
+// by lane the 2K-1 lifted values y_i + P in (P/2, 3P/2) go to shared memory,
+// then lane by lane each 32-bit word of sum_i (y_i + P) 2^(M i) - P sum_i 2^(M i)
+// (the second sum's negative is `negcorr`, the same for every coefficient)
+// gathers the few values that overlap it, and the words' carries are resolved
+// 32 at a time with ballots.  One thread per coefficient ran a serial chain of
+// 2K-1 lifts with 64-bit divisions and two accumulators in local memory; with
+// this sum and the split in one launch the 1024-term 1024-bit product went
+// from 194 to 42 us (its three 2^17-point products, 17 us each on side
+// streams, are most of what is left).
+constexpr int kBigThreadK = 4;
+constexpr int kBigWarps = 4;
+constexpr int kBigMaxAcc32 = 2 * kBigMaxAccWords;
+
+struct BigSumArgs {
+    const u32* prod[kBigMaxPrimes];  // (2K - 1) lc words each
+    u32 lc;
+    int K, M, out_words;
+    u32 p[kBigMaxPrimes], oneq[kBigMaxPrimes];
+    Tw inv[kBigMaxPrimes][kBigMaxPrimes];  // inv[a][b] = p_a^-1 mod p_b (a < b)
+    u64 half_lo, half_hi, full_lo, full_hi;
+    unsigned long long* c;
+    u32 negcorr[kBigMaxAcc32];
+};
+
+template <int NP>
+__global__ void __launch_bounds__(32 * kBigWarps) k_big_sum(const __grid_constant__ BigSumArgs A) {
+    extern __shared__ __align__(16) u32 ysm[];  // per warp: 2K-1 values of four words
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nv = 2 * A.K - 1;
+    const u32 j = blockIdx.x * kBigWarps + warp;
+    if (j >= A.lc) return;  // whole warps
+    uint4* y = reinterpret_cast<uint4*>(ysm) + (size_t)warp * nv;
+    for (int i = lane; i < nv; i += 32) {
+        const size_t at = (size_t)j * nv + i;
+        u32 v[NP];
+#pragma unroll
+        for (int k = 0; k < NP; ++k) {
+            const u32 pk = A.p[k];
+            u32 t = A.prod[k][at];
+#pragma unroll
+            for (int a = 0; a < k; ++a) {
+                // t = (t - v_a) / p_a mod p_k
+                const u32 d = t + pk - red1(mul_shoup(v[a], 1u, A.oneq[k], pk), pk);
+                t = red1(mul_shoup(d, A.inv[a][k].w, A.inv[a][k].wq, pk), pk);
+            }
+            v[k] = t;
+        }
+        unsigned __int128 x = v[NP - 1];
+#pragma unroll
+        for (int k = NP - 2; k >= 0; --k) x = x * A.p[k] + v[k];
+        const unsigned __int128 half = ((unsigned __int128)A.half_hi << 64) | A.half_lo;
+        if (x <= half) x += ((unsigned __int128)A.full_hi << 64) | A.full_lo;
+        y[i] = make_uint4((u32)x, (u32)(x >> 32), (u32)(x >> 64), (u32)(x >> 96));
+    }
+    __syncwarp();
+    const u32* yw = reinterpret_cast<const u32*>(y);
+    u32* out = reinterpret_cast<u32*>(A.c + (size_t)j * A.out_words);
+    const int nw = 2 * A.out_words;
+    u32 high = 0, cin = 0;  // into the chunk's first word: the previous word's excess, and a carry
+    for (int w0 = 0; w0 < nw; w0 += 32) {
+        const int w = w0 + lane;
+        u64 s = 0;
+        if (w < nw) {
+            s = w < kBigMaxAcc32 ? A.negcorr[w] : 0xffffffffu;
+            // values with M i < 32 w + 32 and M i + 128 > 32 w
+            const int lo = 32 * w >= 128 ? (32 * w - 128) / A.M + 1 : 0, hi = min(nv - 1, (32 * w + 31) / A.M);
+            for (int i = lo; i <= hi; ++i) {
+                const int sh = 32 * w - A.M * i;  // bit of y_i at this word's bit 0, in (-32, 128)
+                if (sh >= 0) {
+                    const int q = sh >> 5;
+                    s += __funnelshift_r(yw[4 * i + q], q < 3 ? yw[4 * i + q + 1] : 0u, sh & 31);
+                } else {
+                    s += (u32)(yw[4 * i] << -sh);
+                }
+            }
+        }
+        const u32 up = (u32)(s >> 32);
+        u32 prev = __shfl_up_sync(~0u, up, 1);
+        if (lane == 0) prev = high;
+        const u64 t = (u64)(u32)s + prev;
+        const u32 gen = __ballot_sync(~0u, (t >> 32) != 0), prop = __ballot_sync(~0u, (u32)t == 0xffffffffu);
+        const u64 carry = ((((u64)gen << 1) | cin) + prop) ^ prop;  // bit l: a carry enters word l
+        if (w < nw) out[w] = (u32)t + (u32)((carry >> lane) & 1);
+        cin = (u32)(carry >> 32) & 1;
+        high = __shfl_sync(~0u, up, 31);
+    }
+}
+
 int grid_of(long long n) { return (int)std::max<long long>(1, std::min<long long>((n + 255) / 256, 148 * 32)); }
 
 }  // namespace
 
-// Scratch of one product (bigconv_mul_dev with caller buffers): the
-// magnitudes, signs, split operands and products per prime, then the
-// products' workspace and job tables (as direct_batch takes them).
+// Scratch of one product (bigconv_mul_dev with caller buffers): the split
+// operands and products per prime, then the products' workspace and job
+// tables (as direct_batch takes them).
 struct BigSizes {
-    size_t mag_bytes, sign_bytes, words, ws_words, job_bytes;
+    size_t words, ws_words, job_bytes;
 };
 
-BigSizes big_sizes(const BigPlan& pl, long long na, long long nb, int in_words) {
+BigSizes big_sizes(const BigPlan& pl, long long na, long long nb) {
     const long long la = (2ll * pl.K - 1) * (na - 1) + pl.K, lb = (2ll * pl.K - 1) * (nb - 1) + pl.K;
     BigSizes z;
-    z.mag_bytes = ((size_t)(na + nb) * in_words * 8 + 255) & ~(size_t)255;
-    z.sign_bytes = ((size_t)(na + nb) + 255) & ~(size_t)255;
     z.words = (size_t)pl.nprimes * (la + lb + la + lb - 1);
     const long long LA[1] = {la}, LB[1] = {lb};
     z.ws_words = (size_t)pl.nprimes * direct_ws_words(1, LA, LB);
     z.job_bytes = (size_t)pl.nprimes * ((direct_job_bytes(1) + 255) & ~(size_t)255);
     return z;
 }
+
+namespace {
+
+// k_big_sum for the products cp of a plan with more than kBigThreadK limbs.
+int big_sum(const BigPlan& pl, u32* const* cp, long long lc, int out_words, unsigned long long* c, cudaStream_t st) {
+    const int r = pl.nprimes, nv = 2 * pl.K - 1;
+    BigSumArgs A;
+    memset(&A, 0, sizeof(A));
+    unsigned __int128 P = 1;
+    for (int k = 0; k < r; ++k) {
+        A.prod[k] = cp[k];
+        A.p[k] = pl.p[k];
+        A.oneq[k] = shoup_quot(1, pl.p[k]);
+        for (int a = 0; a < k; ++a)
+            A.inv[a][k] = tw_of(powmod_exact(pl.p[a] % pl.p[k], pl.p[k] - 2, pl.p[k]), pl.p[k]);
+        P *= pl.p[k];
+    }
+    A.lc = (u32)lc;
+    A.K = pl.K;
+    A.M = pl.M;
+    A.out_words = out_words;
+    A.full_lo = (u64)P;
+    A.full_hi = (u64)(P >> 64);
+    A.half_lo = (u64)(P >> 1);
+    A.half_hi = (u64)(P >> 65);
+    A.c = c;
+    // -P sum_i 2^(M i) mod 2^(32 kBigMaxAcc32); the sum stays below it (8,704
+    // bits for values of at most 2 * 4096 + 200), so words past it are all ones
+    std::vector<u64> col(kBigMaxAcc32 + 8, 0);
+    for (int i = 0; i < nv; ++i) {
+        const int s = pl.M * i, w = s >> 5, b = s & 31;
+        for (int q = 0; q < 5; ++q) {
+            const u32 lo = q < 4 ? (u32)(P >> (32 * q)) : 0u, below = q > 0 ? (u32)(P >> (32 * (q - 1))) : 0u;
+            const u32 piece = b ? (lo << b) | (below >> (32 - b)) : lo;
+            if (w + q < kBigMaxAcc32) col[w + q] += piece;
+        }
+    }
+    u64 carry = 0, plus = 1;
+    for (int w = 0; w < kBigMaxAcc32; ++w) {
+        const u64 v = col[w] + carry;
+        carry = v >> 32;
+        const u64 n = (u64)(u32)~(u32)v + plus;  // two's complement of the sum
+        A.negcorr[w] = (u32)n;
+        plus = n >> 32;
+    }
+    const unsigned blocks = (unsigned)((lc + kBigWarps - 1) / kBigWarps);
+    const size_t smem = (size_t)kBigWarps * nv * 16;
+    if (r == 3) k_big_sum<3><<<blocks, 32 * kBigWarps, smem, st>>>(A);
+    else k_big_sum<4><<<blocks, 32 * kBigWarps, smem, st>>>(A);
+    return cuda_err(cudaGetLastError());
+}
+
+}  // namespace
 
 // c (lc = na + nb - 1 coefficients of out_words words) = a * b exactly;
 // device pointers, coefficients of in_words two's-complement words, bw the
@@ -299,44 +425,45 @@ int bigconv_mul_dev(const unsigned long long* a, long long na, const unsigned lo
     const long long la = (2ll * pl.K - 1) * (na - 1) + pl.K, lb = (2ll * pl.K - 1) * (nb - 1) + pl.K;
     const long long lp = la + lb - 1;
     const int r = pl.nprimes;
-    // scratch: |a|, |b| (64-bit words), signs, split operands and products per prime
-    const BigSizes z = big_sizes(pl, na, nb, in_words);
-    const size_t mag_bytes = z.mag_bytes, sign_bytes = z.sign_bytes, words = z.words;
+    // scratch: split operands and products, prime by prime
+    const BigSizes z = big_sizes(pl, na, nb);
     const int dev = current_device();
-    char* ws = bufs ? (char*)bufs->eval : (char*)workspace(dev, kWsBig, mag_bytes + sign_bytes + words * 4, &err);
-    if (!ws) return err;
-    unsigned long long* mag = (unsigned long long*)ws;
-    unsigned char* sg = (unsigned char*)(ws + mag_bytes);
-    u32* w32 = (u32*)(ws + mag_bytes + sign_bytes);
-    k_big_abs<<<grid_of(na), 256, 0, st>>>(a, na, in_words, mag, sg);
-    k_big_abs<<<grid_of(nb), 256, 0, st>>>(b, nb, in_words, mag + (size_t)na * in_words, sg + na);
+    u32* w32 = bufs ? bufs->eval : (u32*)workspace(dev, kWsBig, z.words * 4, &err);
+    if (!w32) return err;
     u32 *ap[kBigMaxPrimes], *bp[kBigMaxPrimes], *cp[kBigMaxPrimes];
     for (int k = 0; k < r; ++k) {
-        ap[k] = w32 + (size_t)k * (la + lb + lp);
-        bp[k] = ap[k] + la;
-        cp[k] = bp[k] + lb;
+        ap[k] = w32 + (size_t)k * la;
+        bp[k] = w32 + (size_t)r * la + (size_t)k * lb;
+        cp[k] = w32 + (size_t)r * (la + lb) + (size_t)k * lp;
     }
     BigSplitArgs S;
     memset(&S, 0, sizeof(S));
+    S.xa = a;
+    S.xb = b;
+    S.ta = (u32)la;
+    S.tb = (u32)lb;
     S.words = in_words;
     S.K = pl.K;
     S.M = pl.M;
     S.nprimes = r;
-    for (int k = 0; k < r; ++k) S.p[k] = pl.p[k];
-    S.mag = mag;
-    S.neg = sg;
-    S.len = na;
-    for (int k = 0; k < r; ++k) S.out[k] = ap[k];
-    k_big_split<<<grid_of(la), 256, 0, st>>>(S);
-    S.mag = mag + (size_t)na * in_words;
-    S.neg = sg + na;
-    S.len = nb;
-    for (int k = 0; k < r; ++k) S.out[k] = bp[k];
-    k_big_split<<<grid_of(lb), 256, 0, st>>>(S);
+    for (int k = 0; k < r; ++k) {
+        const u32 p = pl.p[k];
+        S.p[k] = p;
+        S.oneq[k] = shoup_quot(1, p);
+        S.r32[k] = tw_of((u32)((1ull << 32) % p), p);
+        S.outa[k] = ap[k];
+        S.outb[k] = bp[k];
+    }
+    k_big_split<<<(unsigned)((la + lb + 255) / 256), 256, 0, st>>>(S);
     if ((err = cuda_err(cudaGetLastError())) != OK) return err;
-    // one product per prime, on side streams (each batch plan owns its
+    // up to 2^16 points every prime's product is one launch for all of them
+    bool done = false;
+    if ((err = latency_mul_primes(pl.p, r, dev, ap[0], (int)la, la, bp[0], (int)lb, lb, cp[0], lp, st, &done)) != OK)
+        return err;
+    // else one product per prime, on side streams (each batch plan owns its
     // workspace), joined before the CRT
-    if (!bufs) {
+    if (done) {
+    } else if (!bufs) {
         const sfixn df = (sfixn)(la - 1), dg = (sfixn)(lb - 1);
         const int64_t zero = 0;
         aux_fork(dev, st, r);
@@ -356,6 +483,9 @@ int bigconv_mul_dev(const unsigned long long* a, long long na, const unsigned lo
             if (err != OK) return err;
         }
     }
+    if (pl.K == 1 && r == 3 && out_words == 2)
+        return launch_lift(cp[0], lc, pl.p, r, (long long*)c, false, st);
+    if (pl.K > kBigThreadK) return big_sum(pl, cp, lc, out_words, c, st);
     BigCrtArgs C;
     memset(&C, 0, sizeof(C));
     for (int k = 0; k < r; ++k) {
@@ -387,8 +517,8 @@ void exact_i64_long_sizes(long long la, long long lb, int bw, size_t* eval_words
         *eval_words = *ws_words = *job_bytes = 0;
         return;
     }
-    const BigSizes z = big_sizes(pl, la, lb, 1);
-    *eval_words = (z.mag_bytes + z.sign_bytes) / 4 + z.words;
+    const BigSizes z = big_sizes(pl, la, lb);
+    *eval_words = z.words;
     *ws_words = z.ws_words;
     *job_bytes = z.job_bytes;
 }
@@ -423,7 +553,8 @@ bool exact_i64_long_one_limb(int bw, long long la, long long lb, u32* primes) {
 namespace {
 
 struct Prime3 {
-    u32 p[3];
+    u32 p[3], oneq[3];
+    Tw r32[3];  // 2^32 mod p
 };
 
 // r_k[j] = x[j] mod p_k in [0, p_k), one word per thread and step.
@@ -436,41 +567,16 @@ __global__ void k_i64_residues(const long long* __restrict__ x, long long n, Pri
         u32 r[3];
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-            const u32 t = (u32)(m % P.p[k]);
-            r[k] = (v < 0 && t) ? P.p[k] - t : t;
+            const u32 p = P.p[k];
+            const u32 t = red1(red2(mul_shoup((u32)m, 1u, P.oneq[k], p) +
+                                        mul_shoup((u32)(m >> 32), P.r32[k].w, P.r32[k].wq, p),
+                                    2 * p),
+                               p);
+            r[k] = (v < 0 && t) ? p - t : t;
         }
         r0[j] = r[0];
         r1[j] = r[1];
         r2[j] = r[2];
-    }
-}
-
-struct Crt3Args {
-    const u32* prod[3];  // canonical residues of each output coefficient
-    long long n;
-    u32 p[3];
-    u32 inv01, inv02, inv12;  // p0^-1 mod p1, p0^-1 mod p2, p1^-1 mod p2
-    long long* c;             // lo, hi words of each signed 128-bit result
-};
-
-// Garner's CRT of three residues to the x in [0, P), stored as the signed
-// value x - P when x > P / 2 (128-bit two's complement); one coefficient per
-// thread and step.  The big-coefficient CRT (k_big_crt) with one limb.
-__global__ void k_crt3_i128(const __grid_constant__ Crt3Args A) {
-    const unsigned __int128 P01 = (unsigned __int128)A.p[0] * A.p[1];
-    const unsigned __int128 P = P01 * A.p[2];
-    const unsigned __int128 half = P >> 1;
-    for (long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x; j < A.n;
-         j += (long long)gridDim.x * blockDim.x) {
-        const u32 v0 = A.prod[0][j];
-        const u32 r1 = A.prod[1][j], r2 = A.prod[2][j];
-        const u32 v1 = (u32)((u64)((r1 + A.p[1] - v0 % A.p[1]) % A.p[1]) * A.inv01 % A.p[1]);
-        const u64 t2 = (u64)((r2 + A.p[2] - v0 % A.p[2]) % A.p[2]) * A.inv02 % A.p[2];
-        const u32 v2 = (u32)((t2 + A.p[2] - v1 % A.p[2]) % A.p[2] * A.inv12 % A.p[2]);
-        unsigned __int128 x = (unsigned __int128)v0 + (unsigned __int128)v1 * A.p[0] + (unsigned __int128)v2 * P01;
-        if (x > half) x -= P;  // wraps to the two's complement of x - P
-        A.c[2 * j] = (long long)(unsigned long long)x;
-        A.c[2 * j + 1] = (long long)(unsigned long long)(x >> 64);
     }
 }
 
@@ -510,7 +616,11 @@ int exact_i64_long_batch(int cnt, const long long* x, const long long* la, const
         prod[k] = B.eval + 3 * (size_t)nin + (size_t)k * nout;
     }
     Prime3 P3;
-    for (int k = 0; k < 3; ++k) P3.p[k] = primes[k];
+    for (int k = 0; k < 3; ++k) {
+        P3.p[k] = primes[k];
+        P3.oneq[k] = shoup_quot(1, primes[k]);
+        P3.r32[k] = tw_of((u32)((1ull << 32) % primes[k]), primes[k]);
+    }
     k_i64_residues<<<grid_of(nin), 256, 0, st>>>(x, nin, P3, res[0], res[1], res[2]);
     int err = cuda_err(cudaGetLastError());
     if (err != OK) return err;
@@ -529,18 +639,7 @@ int exact_i64_long_batch(int cnt, const long long* x, const long long* la, const
                            (char*)B.djobs + k * jb, (char*)B.hjobs + k * jb, st, false);
         if (err != OK) return err;
     }
-    Crt3Args C;
-    for (int k = 0; k < 3; ++k) {
-        C.prod[k] = prod[k];
-        C.p[k] = primes[k];
-    }
-    C.n = nout;
-    C.inv01 = powmod_exact(primes[0] % primes[1], primes[1] - 2, primes[1]);
-    C.inv02 = powmod_exact(primes[0] % primes[2], primes[2] - 2, primes[2]);
-    C.inv12 = powmod_exact(primes[1] % primes[2], primes[2] - 2, primes[2]);
-    C.c = c;
-    k_crt3_i128<<<grid_of(nout), 256, 0, st>>>(C);
-    return cuda_err(cudaGetLastError());
+    return launch_lift(prod[0], nout, primes, 3, c, false, st);
 }
 
 }  // namespace cmb
