@@ -789,9 +789,9 @@ int cyclic_mul_compose(u32* f, const u32* g, int e, u32 p, cudaStream_t st) {
 
 // F <- DFT^-1(DFT F * DFT G) on a 2^em x 2^en row-major grid (rows: y, of
 // length 2^en in x): the 2-D cyclic convolution, i.e. the bivariate product
-// when both operands are zero-padded to the product's size.  Grids within
-// the fused 2-D transform's limits use it (column pass + row pass per
-// transform).  Otherwise: row transforms,
+// when both operands are zero-padded to the product's size.  Grids of up to
+// 2^13 rows run as the three passes of a long product (grid_mul_dev).
+// Otherwise: row transforms,
 // a transpose, column transforms (as rows) give both spectra in transposed
 // order; the pointwise product and the inverse steps run in that order, so
 // nothing is permuted back before the last transpose.  G is overwritten.
@@ -804,8 +804,10 @@ int bivariate_mul_dev(u32* F, u32* G, int em, int en, u32 p, cudaStream_t st) {
     if (em > pc->info.two_adic || en > pc->info.two_adic || em + en > 30) return FFT_SIZE_TOO_LARGE;
     const long long m = 1ll << em, n = 1ll << en, total = m * n;
     const u32 wm = em ? canonical_root(*pc, em) : 1u, wn = en ? canonical_root(*pc, en) : 1u;
+    int l1, e;
+    if (grid_split(em, en, &l1, &e)) return grid_mul_dev(F, G, em, en, p, st);
     if (en >= 6 && en <= kMaxRowLog && em <= kMaxColLog) {
-        // grids the fused 2-D transform covers: two passes per transform, no transposes
+        // one row, or a grid of less than 2^11 words
         if ((err = bivariate_dev(F, em, wm, en, wn, p, false, st)) != OK) return err;
         if ((err = bivariate_dev(G, em, wm, en, wn, p, false, st)) != OK) return err;
         k_pointwise_mod<<<grid_for(total), 256, 0, st>>>(F, G, total, p, pc->info.pinv_neg, pc->info.r2);

@@ -381,26 +381,33 @@ bool launch_col_fwd_pipe1(const LargeArgs& a, int njobs, cudaStream_t st) {
     return true;
 }
 
-void launch_large(const LargeArgs& a, int njobs, cudaStream_t st) {
-    const int n1 = 1 << a.l1, n2 = 1 << a.l2;
-    NvtxRange range(kRowFName[a.l2]);  // the product's three passes, named by its dominant kernel
+void launch_col_fwd(const LargeArgs& a, int njobs, cudaStream_t st) {
     cudaEvent_t e0;
-    bool tr = pass_timing_begin(st, &e0);
-    if (!launch_col_fwd_pipe(a, njobs, st)) kColFwd[a.l1](a, dim3(n2 / col_tile_cols_rt(a.l1, false), 2, njobs), st);
+    const bool tr = pass_timing_begin(st, &e0);
+    if (!launch_col_fwd_pipe(a, njobs, st))
+        kColFwd[a.l1](a, dim3((1 << a.l2) / col_tile_cols_rt(a.l1, false), 2, njobs), st);
     if (tr) pass_timing_end(st, kColFwdName[a.l1], e0);
-    if (a.row_fused) {
-        tr = pass_timing_begin(st, &e0);
-        kRow[a.l2](a, dim3(n1, njobs, 1), st);
-        if (tr) pass_timing_end(st, kRowName[a.l2], e0);
-    } else {
-        tr = pass_timing_begin(st, &e0);
-        kRowG[a.l2](a, dim3(n1, njobs, 1), st);
-        if (tr) pass_timing_end(st, kRowGName[a.l2], e0);
-        tr = pass_timing_begin(st, &e0);
-        kRowF[a.l2](a, dim3(n1, njobs, 1), st);
-        if (tr) pass_timing_end(st, kRowFName[a.l2], e0);
+}
+
+void launch_col_fwd_full(const LargeArgs& a, cudaStream_t st) {
+    if (a.l1 != 10) {
+        launch_col_fwd(a, 1, st);
+        return;
     }
-    tr = pass_timing_begin(st, &e0);
+    LargeArgs b = a;
+    b.job0.a = a.job0.b;
+    b.job0.la = a.job0.lb;
+    b.job0.wa = a.job0.wb;
+    cudaEvent_t e0;
+    const bool tr = pass_timing_begin(st, &e0);
+    if (!launch_col_fwd_pipe1(a, 1, st) || !launch_col_fwd_pipe1(b, 1, st)) launch_col_fwd(a, 1, st);
+    if (tr) pass_timing_end(st, kColFwdName[a.l1], e0);
+}
+
+void launch_col_inv(const LargeArgs& a, int njobs, cudaStream_t st) {
+    const int n2 = 1 << a.l2;
+    cudaEvent_t e0;
+    const bool tr = pass_timing_begin(st, &e0);
     if (col_pipe_ok(a.l1) && col_pipe_enabled()) {
         const int ntiles = (n2 / col_tile_cols_rt(a.l1, true)) * njobs;
         if (a.l1 == 10) launch_col_inv_pipe_t<10>(a, ntiles, st);
@@ -409,6 +416,25 @@ void launch_large(const LargeArgs& a, int njobs, cudaStream_t st) {
         kColInv[a.l1](a, dim3(n2 / col_tile_cols_rt(a.l1, true), 1, njobs), st);
     }
     if (tr) pass_timing_end(st, kColInvName[a.l1], e0);
+}
+
+void launch_large(const LargeArgs& a, int njobs, cudaStream_t st) {
+    const int n1 = 1 << a.l1;
+    NvtxRange range(kRowFName[a.l2]);  // the product's three passes, named by its dominant kernel
+    cudaEvent_t e0;
+    launch_col_fwd(a, njobs, st);
+    bool tr = pass_timing_begin(st, &e0);
+    if (a.row_fused) {
+        kRow[a.l2](a, dim3(n1, njobs, 1), st);
+        if (tr) pass_timing_end(st, kRowName[a.l2], e0);
+    } else {
+        kRowG[a.l2](a, dim3(n1, njobs, 1), st);
+        if (tr) pass_timing_end(st, kRowGName[a.l2], e0);
+        tr = pass_timing_begin(st, &e0);
+        kRowF[a.l2](a, dim3(n1, njobs, 1), st);
+        if (tr) pass_timing_end(st, kRowFName[a.l2], e0);
+    }
+    launch_col_inv(a, njobs, st);
 }
 
 // h[i] = (h[i] + t[i]) mod p for i < len; both in [0, p).

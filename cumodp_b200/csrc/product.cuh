@@ -40,6 +40,11 @@ bool launch_col_fwd_pipe(const LargeArgs& a, int njobs, cudaStream_t st);
 // A natural-order transform's column pass (operand a of each job, over wa)
 // through k_col_fwd_pipe1 when the columns have 2^10 rows; false otherwise.
 bool launch_col_fwd_pipe1(const LargeArgs& a, int njobs, cudaStream_t st);
+// The forward column pass of every job's two operands, the same for job0 with
+// operands as long as the transform (no zero half), the inverse column pass.
+void launch_col_fwd(const LargeArgs& a, int njobs, cudaStream_t st);
+void launch_col_fwd_full(const LargeArgs& a, cudaStream_t st);
+void launch_col_inv(const LargeArgs& a, int njobs, cudaStream_t st);
 void launch_small(int logn, const SmallArgs& a, int njobs, cudaStream_t st);
 void launch_large(const LargeArgs& a, int njobs, cudaStream_t st);
 
@@ -80,6 +85,14 @@ size_t mul_ws_words(int logn);
 // h[0..lh) = a[0..la) * b[0..lb) mod p on device pointers, on stream st.
 int mul_dev(const u32* a, long long la, const u32* b, long long lb, u32* h, long long lh, u32 p,
             cudaStream_t st);
+
+// Whether the bivariate product of 2^em x 2^en grids runs on the three-pass
+// kernels (grid_product.cuh): columns of 2^l1 rows, the other e bits of y in
+// the row passes.
+bool grid_split(int em, int en, int* l1, int* e);
+// F <- the 2-D cyclic convolution of F and G (grids within grid_split's range,
+// 16-byte aligned; em and en within p's 2-adic order).
+int grid_mul_dev(u32* F, u32* G, int em, int en, u32 p, cudaStream_t st);
 
 // f <- f * g mod (x^(2^e) - 1, p), the length-2^e cyclic convolution, on
 // device arrays of 2^e words (f may not overlap g): the product kernels on

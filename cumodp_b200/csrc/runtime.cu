@@ -8,6 +8,7 @@
 // scratch buffers grow once and are reused.
 #include "runtime.cuh"
 
+#include "large_product.cuh"
 #include "latency_product.cuh"
 
 #include <atomic>
@@ -265,6 +266,25 @@ static cudaError_t upload_now(void* d, const void* h, size_t bytes) {
 
 namespace {
 
+// Uploads t and keeps it under key (C.m held).
+const Tw* keep_table(Caches& C, const std::tuple<int, u32, u32, int, int>& key, const std::vector<Tw>& t, int* err) {
+    Tw* d = nullptr;
+    if (dev_malloc((void**)&d, t.size() * sizeof(Tw)) != cudaSuccess) {
+        cudaGetLastError();
+        *err = OUT_OF_MEMORY;
+        return nullptr;
+    }
+    if (upload_now(d, t.data(), t.size() * sizeof(Tw)) != cudaSuccess) {
+        cudaGetLastError();
+        cudaFree(d);
+        *err = FFT_ERROR;
+        return nullptr;
+    }
+    C.bytes += (long long)(t.size() * sizeof(Tw));
+    C.tables[key] = d;
+    return d;
+}
+
 // One level's entries in the layout [slot j][task o < tasks]: w^(o bitrev(j)),
 // row by row with one product per entry.
 void push_slot_major(std::vector<Tw>& t, u32 w, int logr, int tasks, u32 p) {
@@ -298,21 +318,28 @@ const Tw* latency_tables(int dev, u32 p, u32 root, int logn, int logl, int* err)
     }
     if (logl < logn)
         for (u32 w : {root, rinv}) push_slot_major(t, w, logn - logl, 1 << logl, p);
-    Tw* d = nullptr;
-    if (dev_malloc((void**)&d, t.size() * sizeof(Tw)) != cudaSuccess) {
-        cudaGetLastError();
-        *err = OUT_OF_MEMORY;
-        return nullptr;
-    }
-    if (upload_now(d, t.data(), t.size() * sizeof(Tw)) != cudaSuccess) {
-        cudaGetLastError();
-        cudaFree(d);
-        *err = FFT_ERROR;
-        return nullptr;
-    }
-    C.bytes += (long long)(t.size() * sizeof(Tw));
-    C.tables[key] = d;
-    return d;
+    return keep_table(C, key, t, err);
+}
+
+const Tw* grid_lead_tables(int dev, u32 p, u32 wm, int em, int en, int l1, u32 scale, int* err) {
+    Caches& C = caches();
+    std::lock_guard<std::mutex> g(C.m);
+    auto key = std::make_tuple(dev, p, wm, en * 64 + l1, 3);
+    auto it = C.tables.find(key);
+    if (it != C.tables.end()) return it->second;
+    const LevelPlan pl = col_plan(l1);
+    const u32 wmi = powmod_exact(wm, (1ull << em) - 1, p);
+    std::vector<Tw> t;
+    for (int inv = 0; inv < 2; ++inv)
+        for (u32 s = 0; s < 1u << l1; ++s) {
+            const u32 f = powmod_exact(inv ? wmi : wm, col_slot_to_k1(s, pl, l1), p);
+            u32 v = inv ? scale : 1u;
+            for (int m = 0; m < 4; ++m) {
+                t.push_back(tw_of(v, p));
+                v = mulmod_exact(v, f, p);
+            }
+        }
+    return keep_table(C, key, t, err);
 }
 
 static const Tw* level_tables(int dev, u32 p, u32 root, int logl, int kind, int* err) {

@@ -345,7 +345,7 @@ cumodp_err cumodp_list_fft_dev(sfixn *X, sfixn m, sfixn k, sfixn w, sfixn p, int
  * j, of 2^en words, holds the coefficients of y^j; x^i at column i):
  * F <- DFT^-1(DFT F * DFT G), the 2-D cyclic convolution, which is the
  * bivariate product when both operands are zero-padded to the product's
- * size.  G is overwritten; F and G 16-byte aligned.  Counterpart of the reference's C++
+ * size.  G may be overwritten; F and G 16-byte aligned.  Counterpart of the reference's C++
  * bi_stockham_poly_mul_dev (src/list_stockham.cu:1317-1348, declared in
  * include/list_stockham.h:103-104; include/list_stockham_b200.h gives that
  * signature), for any em, en within the prime's 2-adic order (em + en <= 30).
