@@ -672,7 +672,8 @@ __global__ void k_monic_level_fixup(const u32* __restrict__ in, u32* __restrict_
 
 // One level of a subproduct tree of monic polynomials stored without their
 // leading coefficient: out[j] = in[2j] * in[2j+1] (degree l each, l words;
-// the product has degree 2l, 2l words).  The products a b run as one batch
+// the product has degree 2l, 2l words).  Transforms of up to 2^12 words are
+// one launch (k_monic_level).  Longer ones: the products a b run as one batch
 // of equal-size pairs (the graph-captured batch path), then one kernel adds
 // the x^l (a + b) term.
 int subproduct_level_dev(long long l, long long npairs, const u32* in, u32* out, u32 p, cudaStream_t st) {
@@ -680,6 +681,11 @@ int subproduct_level_dev(long long l, long long npairs, const u32* in, u32* out,
     if (npairs == 0) return OK;
     if (!in || !out) return ASSUMPTION_ERROR;
     if (out < in + 2 * npairs * l && in < out + 2 * npairs * l) return ASSUMPTION_ERROR;  // no aliasing
+    if (2 * l <= 1 << kMaxLevelLog) {
+        int e = OK;
+        const PrimeCtx* pc = prime_ctx(p, &e);
+        return pc ? monic_level_dev(*pc, (int)l, (int)npairs, in, out, st) : e;
+    }
     const int cnt = (int)npairs;
     std::vector<sfixn> d(cnt, (sfixn)(l - 1));
     std::vector<int64_t> fo(cnt), go(cnt), ho(cnt);

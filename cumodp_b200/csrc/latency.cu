@@ -1,4 +1,5 @@
 // Host side of the one-launch products (latency_product.cuh).
+#include <algorithm>
 #include <map>
 #include <mutex>
 #include <tuple>
@@ -198,6 +199,51 @@ int latency_mul_i64(const u32* primes, int np, int dev, const long long* a, int 
     if (tr) pass_timing_end(st, kName[logn - kMinLog], e0);
     *launched = ce == cudaSuccess;
     return cuda_err(ce);
+}
+
+namespace {
+
+template <int LOGL>
+void launch_level_t(const LevelArgs& a, int sms, cudaStream_t st) {
+    constexpr size_t smem = lat_smem(LOGL, 1);
+    static const bool attr = [] {
+        cudaFuncSetAttribute(k_monic_level<LOGL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        return true;
+    }();
+    (void)attr;
+    const int grid = std::min(a.npairs, sms * level_ctas(LOGL));
+    k_monic_level<LOGL><<<grid, level_threads(LOGL), smem, st>>>(a);
+}
+typedef void (*LevelFn)(const LevelArgs&, int, cudaStream_t);
+const LevelFn kLevel[] = {launch_level_t<5>, launch_level_t<6>,  launch_level_t<7>,  launch_level_t<8>,
+                          launch_level_t<9>, launch_level_t<10>, launch_level_t<11>, launch_level_t<12>};
+
+}  // namespace
+
+int monic_level_dev(const PrimeCtx& pc, int l, int npairs, const u32* in, u32* out, cudaStream_t st) {
+    int logn = kMinLog, err = OK;
+    while ((1 << logn) < 2 * l) ++logn;
+    if (logn > kMaxLevelLog) return ASSUMPTION_ERROR;
+    if (logn > pc.info.two_adic) return FFT_SIZE_TOO_LARGE;
+    const int dev = current_device();
+    const u32 p = pc.info.p, root = canonical_root(pc, logn);
+    LevelArgs a{};
+    // these lengths' block tables are those of the one-launch product where it
+    // has one CTA; 2^12 has a table of its own
+    a.pr.tw = latency_tables(dev, p, root, logn, logn, &err);
+    if (!a.pr.tw) return err;
+    const u32 ninv = powmod_exact((u32)((1ull << logn) % p), p - 2, p);
+    a.pr.pk = pc.pk;
+    a.pr.scale = tw_of(mulmod_exact(ninv, pc.info.r1, p), p);
+    a.in = in;
+    a.out = out;
+    a.l = l;
+    a.npairs = npairs;
+    cudaEvent_t e0;
+    const bool tr = pass_timing_begin(st, &e0);
+    kLevel[logn - kMinLog](a, sm_count(dev), st);
+    if (tr) pass_timing_end(st, "monic_level", e0);
+    return cuda_err(cudaGetLastError());
 }
 
 }  // namespace cmb

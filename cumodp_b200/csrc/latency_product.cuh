@@ -338,6 +338,93 @@ __global__ void __launch_bounds__(lat_threads(LOGL), 1) k_latency_product(const 
     }
 }
 
+// One level of a subproduct tree (cumodp_subproduct_level_dev) for transforms
+// of 2^LOGL = n >= 2l words: pair j's monic polynomials x^l + a and x^l + b
+// (l words each, consecutive) go in with their leading coefficient, and their
+// product mod x^n - 1 has the 2l words wanted, except that for n = 2l the
+// leading x^(2l) wraps onto the constant term.  So the x^l (a + b) term costs
+// nothing, and no job table is made or uploaded: a job is its index.
+// Persistent CTAs (the twiddles are copied once); the next pair's words are
+// loaded while the current pair is transformed.  One operand per task and
+// radix 8 last keep a thread's data in 16 registers: the batch kernel's
+// radix-32 level holds 64 and spends as long on it as on the rest.  Bound by
+// integer issue (68 % of the issue slots).  Measured on B200, with the batch
+// kernel, its job upload and the fix-up pass before: 2048 pairs of degree 512
+// 41 -> 23 us, 32768 of them 583 -> 263 us, 65536 pairs of degree 16 1102 -> 39
+// us (a job table a call).
+struct LevelArgs {
+    LatPrime pr;
+    const u32* in;
+    u32* out;
+    int l, npairs;
+};
+__host__ __device__ constexpr int level_threads(int logl) { return logl <= 8 ? 32 : 1 << (logl - 3); }
+__host__ __device__ constexpr int level_ctas(int logl) { return logl <= 8 ? 24 : logl <= 10 ? 1024 / level_threads(logl) : logl == 11 ? 4 : 2; }
+
+template <int LOGL>
+__global__ void __launch_bounds__(level_threads(LOGL), level_ctas(LOGL)) k_monic_level(const __grid_constant__ LevelArgs A) {
+    constexpr int L = 1 << LOGL, T = level_threads(LOGL), W = (lat_words(LOGL) + 3) & ~3;
+    constexpr LevelPlan PL = lat_plan(LOGL);
+    constexpr int NE = lat_entries(LOGL), NV = 2 * L / T;
+    extern __shared__ __align__(16) u32 sm[];  // F, G, twiddles
+    Tw* tws = reinterpret_cast<Tw*>(sm + 2 * W);
+    const LatPrime& P = A.pr;
+    const u32 p = P.pk.p, p2 = P.pk.p2;
+    for (int i = threadIdx.x; i < NE; i += T) {
+        const unsigned d = (unsigned)__cvta_generic_to_shared(tws + 2 * i);
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(P.tw + 2 * i) : "memory");
+    }
+    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
+    u32 v[NV];
+    auto load = [&](u32 j) {
+        const u32* src = A.in + (size_t)2 * j * A.l;
+#pragma unroll
+        for (int u = 0; u < NV; ++u) {
+            const int idx = threadIdx.x + u * T, i = idx % L, at = (idx >= L ? A.l : 0) + i;
+            v[u] = i < A.l ? __ldg(src + at) : i == A.l ? 1u : 0u;
+        }
+    };
+    u32 j = blockIdx.x;
+    const u32 npairs = A.npairs;
+    if (j < npairs) load(j);
+    for (; j < npairs; j += gridDim.x) {
+#pragma unroll
+        for (int u = 0; u < NV; ++u) {
+            const int idx = threadIdx.x + u * T;
+            sm[(idx / L) * W + lat_pad(idx % L)] = mul_shoup(v[u], 1u, P.pk.one_q, p);
+        }
+        __syncthreads();
+        if (j + gridDim.x < npairs) load(j + gridDim.x);
+        lat_fwd_levels<LOGL, 0, T>(sm, tws, P.pk);
+        for (int id = threadIdx.x; id < L / 8; id += T) {
+            u32 f[8], g[8];
+#pragma unroll
+            for (int m = 0; m < 8; ++m) {
+                f[m] = sm[lat_pad(8 * id + m)];
+                g[m] = sm[W + lat_pad(8 * id + m)];
+            }
+            dif_regs<8>(f, P.pk.rc.f, p, p2);
+            dif_regs<8>(g, P.pk.rc.f, p, p2);
+#pragma unroll
+            for (int m = 0; m < 8; ++m)
+                f[m] = mul_shoup(mul_mont(f[m], g[m], p, P.pk.pinv_neg), P.scale.w, P.scale.wq, p);
+            dit_regs<8>(f, P.pk.rc.i, p, p2);
+#pragma unroll
+            for (int m = 0; m < 8; ++m) sm[lat_pad(8 * id + m)] = f[m];
+        }
+        __syncthreads();
+        u32* out = A.out + (size_t)2 * j * A.l;
+        lat_inv_levels<LOGL, PL.nlev - 2, T>(sm, tws + NE, P.pk, [&](int i, u32 x) {
+            if (i < 2 * A.l) {
+                u32 c = red1(red2(x, p2), p);
+                if (i == 0 && 2 * A.l == L) c = c ? c - 1 : p - 1;
+                out[i] = c;
+            }
+        });
+        __syncthreads();  // the last inverse level has read its words
+    }
+}
+
 #endif  // __CUDACC__
 
 }  // namespace cmb

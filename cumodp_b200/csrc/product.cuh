@@ -65,6 +65,13 @@ int latency_mul_primes(const u32* primes, int np, int dev, const u32* a, int la,
 int latency_mul_i64(const u32* primes, int np, int dev, const long long* a, int la, const long long* b, int lb, u32* h,
                     cudaStream_t st, bool* launched);
 
+// One level of a subproduct tree, 2l <= 2^kMaxLevelLog (k_monic_level): the
+// npairs products of consecutive monic polynomials of degree l.  Longer levels
+// have few pairs for their size and run as batches (2^13 words are two
+// operands and twiddles of more than one CTA's shared memory).
+constexpr int kMaxLevelLog = 12;
+int monic_level_dev(const PrimeCtx& pc, int l, int npairs, const u32* in, u32* out, cudaStream_t st);
+
 // Sets the shared-memory limits of every product kernel once (must run
 // before any launch is captured into a graph).
 void ensure_kernel_attrs();

@@ -303,7 +303,7 @@ void push_slot_major(std::vector<Tw>& t, u32 w, int logr, int tasks, u32 p) {
 const Tw* latency_tables(int dev, u32 p, u32 root, int logn, int logl, int* err) {
     Caches& C = caches();
     std::lock_guard<std::mutex> g(C.m);
-    auto key = std::make_tuple(dev, p, root, logn, 2);
+    auto key = std::make_tuple(dev, p, root, logn, 16 + logl);
     auto it = C.tables.find(key);
     if (it != C.tables.end()) return it->second;
     const LevelPlan pl = lat_plan(logl);
