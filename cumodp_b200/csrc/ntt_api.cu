@@ -7,8 +7,8 @@
 // (src/list_stockham.cu:1224-1245) computes the row-column 2-D DFT
 // (DFT_m (x) I_n)(I_m (x) DFT_n) of a row-major 2^em x 2^en array.
 //
-// Here a transform of length <= 2^14 is one CTA (levels in shared memory,
-// then an in-CTA reorder to natural order).  Longer 1-D transforms use the
+// Here a transform of length <= 2^14 is one CTA's row (k_row_nat, natural
+// order for free).  Longer 1-D transforms use the
 // four-step split of the product path: a column pass (k_col_fwd), a row
 // pass that applies w_n^(k1*c), transforms the row and writes it back in
 // natural order as row k1, and a tiled transpose.  The 2-D transform is the
@@ -20,20 +20,20 @@
 
 #include "../../include/cumodp.h"
 #include "product.cuh"
+#include "row_natural.cuh"
 
 namespace cmb {
 
 struct RowNttArgs {
     PrimeK pk;
     const Tw* __restrict__ twr;
-    const u32* __restrict__ seeds;  // inter-pass twiddles w_n^(k1 c) (nullptr: none)
+    const u32* __restrict__ seeds;  // inter-pass twiddles w_n^(k1 c)
     int nlo, nhi;
-    int l1;                         // rows come from a column pass of length 2^l1 (0: none)
+    int l1;                         // rows come from a column pass of length 2^l1
     LevelPlan colpl;
     const u32* src;                 // row slot s at src + s * n2
     u32* dst;                       // natural row k1 at dst + k1 * n2
     Tw scale;                       // applied to every output (folded into level 0's input factors)
-    int rows_in_place;              // 1: independent rows, row s written to dst row s
     const Tw* __restrict__ rowtab;  // per-slot level-0 factor tables (RowTab, forward direction), or nullptr
     long long job_stride;           // words between the transforms of grid row blockIdx.y (list transforms)
 };
@@ -43,10 +43,9 @@ __device__ __forceinline__ u32 seed_mont_at(const u32* __restrict__ seeds, int n
 }
 
 
-// One row of the natural-order transform per CTA: the row (a column-pass
-// output row, or an independent row) is copied into shared memory with
-// cp.async, level 0 applies the inter-pass twiddle w_n^(k1 c) (or reduces
-// the input), the remaining levels run as in the product kernels, and the
+// One row of a four-step transform per CTA: the row (a column-pass output
+// row) is copied into shared memory with cp.async, level 0 applies the
+// inter-pass twiddle w_n^(k1 c), the remaining levels run as in the product kernels, and the
 // last level leaves each thread one 32-word group in registers; after a
 // barrier the groups are written back at their natural positions in the same
 // buffer, and the row is stored with 16-byte accesses.  With the prebuilt
@@ -78,13 +77,11 @@ __global__ void __launch_bounds__(QOUT ? rowsplit_threads(L2) : ntt_row_threads(
     __shared__ Tw bf[R0];
 
     const u32 s = blockIdx.x;
-    const u32 k1 = A.l1 ? col_slot_to_k1(s, A.colpl, A.l1) : 0u;
-    const u32 out_row = A.rows_in_place ? s : k1;
-    const bool twid = A.seeds != nullptr;
+    const u32 k1 = col_slot_to_k1(s, A.colpl, A.l1);
     const u32 nmask = (1u << (A.l1 + L2)) - 1;
     const u32 p = A.pk.p, p2 = A.pk.p2, pinv = A.pk.pinv_neg;
     using RT = RowTab<L2>;
-    const bool tabbed = RT::USE && twid && A.rowtab;
+    const bool tabbed = RT::USE && A.rowtab;
     const bool scaled = A.scale.w != 1u;
     Tw* tab = reinterpret_cast<Tw*>(sm + n2);
     const size_t joff = (size_t)blockIdx.y * (size_t)A.job_stride;
@@ -96,7 +93,7 @@ __global__ void __launch_bounds__(QOUT ? rowsplit_threads(L2) : ntt_row_threads(
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src + 2 * i) : "memory");
         }
         asm volatile("cp.async.commit_group;\n" ::: "memory");
-    } else if (twid && threadIdx.x < R0) {
+    } else if (threadIdx.x < R0) {
         const u32 e = (k1 * (u32)TB0 * threadIdx.x) & nmask;
         u32 v = red1(mul_mont(seed_mont_at(A.seeds, A.nlo, e, p, pinv), 1u, p, pinv), p);
         if (scaled) v = mulmod_exact(v, A.scale.w, p);
@@ -139,14 +136,12 @@ __global__ void __launch_bounds__(QOUT ? rowsplit_threads(L2) : ntt_row_threads(
     }
     for (int o = threadIdx.x; o < (tabbed ? 0 : TB0); o += T) {
         u32 x[R0];
-        const u32 mo = twid ? seed_mont_at(A.seeds, A.nlo, (k1 * (u32)o) & nmask, p, pinv) : 0u;
+        const u32 mo = seed_mont_at(A.seeds, A.nlo, (k1 * (u32)o) & nmask, p, pinv);
         const int bs = swz(o);
 #pragma unroll
         for (int m = 0; m < R0; ++m) {
             const u32 v = sm[swz_task<TB0, n2>(o, bs, m)];
-            if (twid) x[m] = mul_mont(v, mul_shoup(mo, bf[m].w, bf[m].wq, p), p, pinv);
-            else if (scaled) x[m] = mul_shoup(v, A.scale.w, A.scale.wq, p);
-            else x[m] = mul_shoup(v, 1u, A.pk.one_q, p);
+            x[m] = mul_mont(v, mul_shoup(mo, bf[m].w, bf[m].wq, p), p, pinv);
         }
         dif_regs<R0, true>(x, A.pk.rc.f, p, p2);
         Tw t[R0];
@@ -160,7 +155,7 @@ __global__ void __launch_bounds__(QOUT ? rowsplit_threads(L2) : ntt_row_threads(
     fwd1_levels<L2, 1, T>(sm, A.pk, A.twr);
 
     if constexpr (QOUT) {
-        u32* out = A.dst + joff + (size_t)out_row * n2;
+        u32* out = A.dst + joff + (size_t)k1 * n2;
         for (int r = threadIdx.x; r < n2 / 32; r += T) {
             u32 x[32];
             load_row32(x, sm, r * 32);
@@ -190,7 +185,7 @@ __global__ void __launch_bounds__(QOUT ? rowsplit_threads(L2) : ntt_row_threads(
         for (int j = 0; j < 32; ++j) sm[swz_nat((int)row_pos_to_freq<L2>((u32)(r * 32 + j)))] = x[j];
     }
     __syncthreads();
-    u32* out = A.dst + joff + (size_t)out_row * n2;
+    u32* out = A.dst + joff + (size_t)k1 * n2;
 #pragma unroll 4
     for (int i = threadIdx.x; i < n2; i += T) out[i] = sm[swz_nat(i)];
 }
@@ -326,9 +321,50 @@ void row_ntt_q_and_transpose(const RowNttArgs& a, int rows, u32* x_out, cudaStre
 }
 typedef void (*RowNttFn)(const RowNttArgs&, int, cudaStream_t, int);
 const RowNttFn kRowNtt[15] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
-                              launch_row_ntt_t<6>, launch_row_ntt_t<7>, launch_row_ntt_t<8>,
-                              launch_row_ntt_t<9>, launch_row_ntt_t<10>, launch_row_ntt_t<11>,
+                              nullptr, nullptr, nullptr, nullptr, launch_row_ntt_t<10>, launch_row_ntt_t<11>,
                               launch_row_ntt_t<12>, launch_row_ntt_t<13>, launch_row_ntt_t<14>};
+
+// `rows` independent natural-order row transforms of 2^k words, 6 <= k <= 14
+// (root: the transform's own, scale applied to every output): src row s to
+// dst row s, or to row k1(s) when the rows are slots of a column pass of 2^l1.
+template <int L2>
+void launch_row_nat_t(const RowNatArgs& a, cudaStream_t st) {
+    static const bool attr = [] {
+        cudaFuncSetAttribute(k_row_nat<L2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)nat_smem(L2));
+        return true;
+    }();
+    (void)attr;
+    const u32 grid = (u32)(((u64)a.rows + nat_rows(L2) - 1) / nat_rows(L2));
+    k_row_nat<L2><<<grid, nat_threads(L2), nat_smem(L2), st>>>(a);
+}
+typedef void (*RowNatFn)(const RowNatArgs&, cudaStream_t);
+const RowNatFn kRowNat[15] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
+                              launch_row_nat_t<6>, launch_row_nat_t<7>, launch_row_nat_t<8>,
+                              launch_row_nat_t<9>, launch_row_nat_t<10>, launch_row_nat_t<11>,
+                              launch_row_nat_t<12>, launch_row_nat_t<13>, launch_row_nat_t<14>};
+
+int row_nat(const PrimeCtx& pc, const u32* src, u32* dst, long long rows, int k, u32 root, u32 scale, int l1, int dev,
+            cudaStream_t st) {
+    int err = OK;
+    RowNatArgs A;
+    memset(&A, 0, sizeof(A));
+    A.tw = nat_tables(dev, pc.info.p, root, k, scale, &err);
+    if (!A.tw) return err;
+    A.pk = make_prime_k_for(pc.info, root, k);
+    A.scaled = scale != 1u;
+    A.l1 = l1;
+    if (l1) A.colpl = col_plan(l1);
+    cudaEvent_t e0;
+    const bool tr = pass_timing_begin(st, &e0);
+    for (long long r0 = 0; r0 < rows; r0 += 1ll << 30) {  // one launch when l1 > 0
+        A.src = src + (r0 << k);
+        A.dst = dst + (r0 << k);
+        A.rows = (u32)std::min<long long>(1ll << 30, rows - r0);
+        kRowNat[k](A, st);
+    }
+    if (tr) pass_timing_end(st, "ntt_row", e0);
+    return cuda_err(cudaGetLastError());
+}
 
 // Forward-column launchers shared with the product path (single operand).
 template <int L1>
@@ -484,22 +520,7 @@ int ntt_natural_dev(const u32* x_in, u32* x_out, int k, u32 w, u32 p, bool inver
         k_tiny_dft<<<1, 1 << k, 0, st>>>(x_in, x_out, 1 << k, root, p, sc);
         return cuda_err(cudaGetLastError());
     }
-    if (k <= kMaxSmallLog) {
-        RowNttArgs A;
-        memset(&A, 0, sizeof(A));
-        const Tw* twr = row_tables(dev, p, root, k, &err);
-        if (!twr) return err;
-        A.pk = make_prime_k_for(pc->info, root, k);
-        A.twr = twr;
-        A.src = x_in;
-        A.dst = x_out;
-        A.scale = tw_of(sc, p);
-        cudaEvent_t e0;
-        const bool tr = pass_timing_begin(st, &e0);
-        kRowNtt[k](A, 1, st, 1);
-        if (tr) pass_timing_end(st, "ntt_row", e0);
-        return cuda_err(cudaGetLastError());
-    }
+    if (k <= kMaxSmallLog) return row_nat(*pc, x_in, x_out, 1, k, root, sc, 0, dev, st);
     const int l1 = std::max(5, k - kMaxRowLog), l2 = k - l1;
     const long long n = 1ll << k;
     u32* ws = (u32*)workspace(dev, kWsNtt, (size_t)2 * n * sizeof(u32), &err);
@@ -631,23 +652,7 @@ int list_ntt_dev(u32* x, long long m, int k, u32 w, u32 p, bool inverse, cudaStr
         }
         return cuda_err(cudaGetLastError());
     }
-    if (k <= kMaxSmallLog) {
-        const int dev = current_device();
-        const Tw* twr = row_tables(dev, p, root, k, &err);
-        if (!twr) return err;
-        RowNttArgs A;
-        memset(&A, 0, sizeof(A));
-        A.pk = make_prime_k_for(pc->info, root, k);
-        A.twr = twr;
-        A.scale = tw_of(sc, p);
-        A.rows_in_place = 1;
-        for (long long r0 = 0; r0 < m; r0 += (1ll << 30)) {
-            A.src = x + (r0 << k);
-            A.dst = x + (r0 << k);
-            kRowNtt[k](A, (int)std::min<long long>(1ll << 30, m - r0), st, 1);
-        }
-        return cuda_err(cudaGetLastError());
-    }
+    if (k <= kMaxSmallLog) return row_nat(*pc, x, x, m, k, root, sc, 0, current_device(), st);
     if (k <= kMaxLog) return list_ntt_four_step(*pc, x, m, k, root, sc, st);
     for (long long r = 0; r < m; ++r)
         if ((err = ntt_natural_dev(x + (r << k), x + (r << k), k, w, p, inverse, st)) != OK) return err;
@@ -714,27 +719,11 @@ int bivariate_dev(u32* x, int em, u32 wm, int en, u32 wn, u32 p, bool inverse, c
     const u32 rm = inverse ? inv_of(wm, p) : wm, rn = inverse ? inv_of(wn, p) : wn;
     const u32 sc = inverse ? inv_of((u32)((1ull << (em + en)) % p), p) : 1u;
     const long long total = 1ll << (em + en);
-    const Tw* twr = row_tables(dev, p, rn, en, &err);
-    if (!twr) return err;
-    RowNttArgs A;
-    memset(&A, 0, sizeof(A));
-    A.pk = make_prime_k_for(pc->info, rn, en);
-    A.twr = twr;
-    A.scale = tw_of(sc, p);
-    A.dst = x;
-    if (em == 0) {
-        A.src = x;
-        kRowNtt[en](A, 1, st, 1);
-        return cuda_err(cudaGetLastError());
-    }
+    if (em == 0) return row_nat(*pc, x, x, 1, en, rn, sc, 0, dev, st);
     u32* w1 = (u32*)workspace(dev, kWsNtt, (size_t)total * sizeof(u32), &err);
     if (!w1) return err;
     if ((err = column_pass(*pc, rm, em, en, x, total, w1, dev, st)) != OK) return err;
-    A.l1 = em;
-    A.colpl = col_plan(em);
-    A.src = w1;
-    kRowNtt[en](A, 1 << em, st, 1);
-    return cuda_err(cudaGetLastError());
+    return row_nat(*pc, w1, x, 1ll << em, en, rn, sc, em, dev, st);
 }
 
 // a[i] = a[i] * b[i] mod p (inputs in [0, p)): a Montgomery product

@@ -10,6 +10,7 @@
 
 #include "large_product.cuh"
 #include "latency_product.cuh"
+#include "row_natural.cuh"
 
 #include <atomic>
 #include <cstdio>
@@ -339,6 +340,32 @@ const Tw* grid_lead_tables(int dev, u32 p, u32 wm, int em, int en, int l1, u32 s
                 v = mulmod_exact(v, f, p);
             }
         }
+    return keep_table(C, key, t, err);
+}
+
+const Tw* nat_tables(int dev, u32 p, u32 root, int logl, u32 scale, int* err) {
+    Caches& C = caches();
+    std::lock_guard<std::mutex> g(C.m);
+    // scale is 1 or the inverse of the length, alone or with a column pass's
+    auto key = std::make_tuple(dev, p, root, logl, (int)(64 + scale));
+    auto it = C.tables.find(key);
+    if (it != C.tables.end()) return it->second;
+    const LevelPlan pl = nat_plan(logl);
+    std::vector<Tw> t;
+    t.reserve((size_t)nat_entries(logl));
+    int lb = logl;
+    for (int i = 0; i + 1 < pl.nlev; ++i) {
+        const u32 w = powmod_exact(root, 1ull << (logl - lb), p);
+        for (int k = 0; k < 1 << pl.logr[i]; ++k) {
+            const u32 step = powmod_exact(w, k, p);
+            u32 v = i == 0 ? scale : 1u;
+            for (int o = 0; o < 1 << (lb - pl.logr[i]); ++o) {
+                t.push_back(tw_of(v, p));
+                v = mulmod_exact(v, step, p);
+            }
+        }
+        lb -= pl.logr[i];
+    }
     return keep_table(C, key, t, err);
 }
 

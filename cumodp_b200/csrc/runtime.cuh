@@ -63,6 +63,9 @@ const Tw* latency_tables(int dev, u32 p, u32 root, int logn, int logl, int* err)
 // 2^em x 2^en grid with columns of 2^l1 rows; wm: the primitive 2^em-th root,
 // scale: the factor of the inverse ones.
 const Tw* grid_lead_tables(int dev, u32 p, u32 wm, int em, int en, int l1, u32 scale, int* err);
+// Twiddles of the natural-order row kernel (row_natural.cuh) for rows of
+// 2^logl words with the primitive 2^logl-th root `root`, outputs times `scale`.
+const Tw* nat_tables(int dev, u32 p, u32 root, int logl, u32 scale, int* err);
 // Inter-pass twiddle seeds for a two-pass transform of length 2^logn:
 // lo[e] = w^e (e < 2^12) and hi[e] = w^(e << 12) (e < 2^(logn-12)), both in
 // Montgomery form times R (w^e * 2^64 mod p) so that one Montgomery product
