@@ -99,7 +99,7 @@ int grid_mul_dev(u32* F, u32* G, int em, int en, u32 p, cudaStream_t st) {
     A.wb = ws + words;
     if (E > 0 && !(A.lead = grid_lead_tables(dev, p, wm, em, en, l1, scale, &err))) return err;
     C.job0 = LargeJob{F, G, F, (int)words, (int)words, (int)words, 0, A.wa, A.wb};
-    launch_col_fwd_full(C, st);
+    launch_col_fwd(C, 1, st);
     kRows[E][en](A, words, st);
     launch_col_inv(C, 1, st);
     return cuda_err(cudaGetLastError());

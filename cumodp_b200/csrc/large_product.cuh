@@ -5,17 +5,15 @@
 // four-step split x[r*n2 + c]: a length-n1 DFT down every column, a twiddle
 // w_n^(c*k1), and a length-n2 DFT along every row.  The whole product needs
 // three passes over HBM:
-//   A  column DFTs of both operands: k_col_fwd_pipe (persistent, the next
-//      tile staged while the current one is transformed) for 2^9- and
-//      2^10-row columns, k_col_fwd (one tile per CTA) otherwise; the zero
-//      pad is never read;
+//   A  column DFTs of both operands: k_cold_fwd (col_direct.cuh) for columns
+//      of up to 2^10 rows, k_col_fwd for 2^11; the zero pad is never read;
 //   B  per row: twiddle, row DFT of both operands, pointwise product,
 //      inverse row DFT, inverse twiddle with the 1/n scale folded in: the
 //      split pair k_row_fwd_g + k_row_mul_f (one operand row per CTA; level
 //      0 reads per-slot factor tables built once by k_rowtab_build), or
 //      k_row_fused (both rows in one CTA, for comparison);
-//   C  inverse column DFTs, truncation, canonical residues: k_col_inv_pipe
-//      or k_col_inv, as for pass A.
+//   C  inverse column DFTs, truncation, canonical residues: k_cold_inv or
+//      k_col_inv, as for pass A.
 // Rows leave pass A in digit-reversed order of k1 and are consumed in that
 // order by passes B and C, so nothing is ever permuted.
 #pragma once
@@ -324,355 +322,6 @@ __global__ void __launch_bounds__(NW * 32, col_ctas(L1, KIND)) k_col_fwd(const _
     __syncthreads();
     col_fwd_levels<L1, 0, NW, KIND>(tile, A.pkc, tws);
     tile_store<L1, KIND, NW * 32>(tile, dst, 1ll << (L1 + A.l2), c0, n2, false, A.pkc);
-}
-
-// Pass A as a persistent, software-pipelined kernel for the two-level
-// column plans (n1 = 2^9, 2^10), on tiles of the layout `KIND` (0: 32
-// columns, one per lane; 2: 16 columns, one task per half-warp, padded rows).
-// Each CTA walks the tiles gridDim.x apart; while it transforms one tile,
-// rows [0, n1/2) of its next tile are already on their way into a staging
-// buffer (cp.async, zero-filled past the operand's end), so the SM does not
-// wait for HBM between tiles.  A product's operands are usually at most n/2
-// words long: their rows [n1/2, n1) are zero and the first level skips that
-// half.  Level 0 reads the stage and writes the tile; the last level reads
-// the tile and stores its outputs straight to HBM (each warp store covers
-// whole row segments).  A longer operand also has rows [n1/2, n1) copied
-// into the tile before level 0, which then reads them there.  Sources that
-// are not 16-byte aligned are copied word by word.  Results are those of
-// k_col_fwd (same levels, same output layout).
-template <int L1, int KIND, int NW>
-__global__ void __launch_bounds__(NW * 32, col_pipe_ctas(L1)) k_col_fwd_pipe(const __grid_constant__ LargeArgs A) {
-    constexpr LevelPlan PL = col_plan(L1);
-    static_assert(PL.nlev == 2, "two-level column plans only");
-    constexpr int n1 = 1 << L1, HALF = n1 / 2, T = NW * 32;
-    constexpr int R0 = 1 << PL.logr[0], R1 = 1 << PL.logr[1];  // n1 = R0 * R1; level-0 tasks: R1
-    constexpr int TC = col_tile_cols(L1, KIND), SUB = 32 / TC, QR = TC / 4;
-    extern __shared__ __align__(16) u32 smem[];
-    u32* tile = smem;                                                   // n1 rows
-    u32* stage = smem + col_tile_words(L1, KIND);                       // rows [0, HALF)
-    Tw* tws = reinterpret_cast<Tw*>(stage + tile_row<L1, KIND>(HALF));  // level-0 twiddles (n1 entries)
-    const int n2 = 1 << A.l2, ct = n2 / TC;
-    const int ntiles = ct * 2 * A.njobs;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int col = lane % TC;
-    const u32 p = A.pkc.p, p2 = A.pkc.p2, oneq = A.pkc.one_q;
-    for (int i = threadIdx.x; i < n1; i += T) tws[i] = A.twc[i];
-
-    // tile t -> job, operand, first column
-    auto decode = [&](int t, const u32*& src, long long& len, u32*& dst, int& c0) {
-        const LargeJob& J = A.jobs ? A.jobs[t / (2 * ct)] : A.job0;
-        const int op = (t / ct) & 1;
-        src = op ? J.b : J.a;
-        len = op ? J.lb : J.la;
-        dst = op ? J.wb : J.wa;
-        c0 = (t % ct) * TC;
-    };
-    // rows [r0, r1) x TC columns of the operand into buf at the tile layout
-    // (one commit group); words at or past len read as 0
-    auto rows_issue = [&](u32* buf, const u32* src, long long len, int c0, int r0, int r1) {
-        if ((reinterpret_cast<uintptr_t>(src) & 15) == 0) {
-            // a thread keeps one quad column q and walks rows T / QR apart
-            // (running index: 64-bit adds, no multiply per copy)
-            static_assert(T % QR == 0, "whole rows per thread round");
-            const int q = threadIdx.x % QR;
-            const long long step = (long long)(T / QR) * n2;
-            long long gi = (long long)(r0 + threadIdx.x / QR) * n2 + c0 + 4 * q;
-#pragma unroll 4
-            for (int r = r0 + threadIdx.x / QR; r < r1; r += T / QR, gi += step) {
-                const long long rem = len - gi;
-                const int bytes = rem >= 4 ? 16 : (rem > 0 ? (int)rem * 4 : 0);
-                const u32* g = bytes ? src + gi : src;
-                const unsigned d = (unsigned)__cvta_generic_to_shared(buf + tile_row<L1, KIND>(r) + 4 * q);
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(g), "r"(bytes) : "memory");
-            }
-        } else {
-            for (int idx = r0 * TC + threadIdx.x; idx < r1 * TC; idx += T) {
-                const int r = idx / TC, c = idx % TC;
-                const long long gi = (long long)r * n2 + c0 + c;
-                const int bytes = gi < len ? 4 : 0;
-                const u32* g = bytes ? src + gi : src;
-                const unsigned d = (unsigned)__cvta_generic_to_shared(buf + tile_row<L1, KIND>(r) + c);
-                asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(d), "l"(g), "r"(bytes) : "memory");
-            }
-        }
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
-    };
-
-    int t = blockIdx.x;
-    if (t < ntiles) {
-        const u32* src; long long len; u32* dst; int c0;
-        decode(t, src, len, dst, c0);
-        rows_issue(stage, src, len, c0, 0, HALF);
-    }
-    for (; t < ntiles; t += gridDim.x) {
-        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-        __syncthreads();  // stage and twiddles visible; the previous tile's last level is done with `tile`
-        bool full;
-        {
-            const u32* src; long long len; u32* dst; int c0;
-            decode(t, src, len, dst, c0);
-            full = len > (long long)HALF * n2;
-            if (full) {  // the upper rows of a long operand, into the tile
-                rows_issue(tile, src, len, c0, HALF, n1);
-                asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-                __syncthreads();
-            }
-        }
-
-        // level 0: task o (rows o + R1 m)
-        for (int o = warp * SUB + lane / TC; o < R1; o += NW * SUB) {
-            u32 x[R0];
-            const int off = tile_row<L1, KIND>(o) + col;
-#pragma unroll
-            for (int m = 0; m < R0 / 2; ++m) x[m] = stage[off + tile_step<L1, KIND, R1>(m)];
-            if (!full) {
-                dif_regs_halfzero<R0, true>(x, A.pkc.rc.f, p, p2, oneq);
-            } else {
-#pragma unroll
-                for (int m = 0; m < R0; ++m)
-                    x[m] = mul_shoup(m < R0 / 2 ? x[m] : tile[off + tile_step<L1, KIND, R1>(m)], 1u, oneq, p);
-                dif_regs<R0, true>(x, A.pkc.rc.f, p, p2);
-            }
-#pragma unroll
-            for (int j = 1; j < R0; ++j) {
-                const Tw w = tws[o * R0 + j];  // broadcast to the (half-)warp
-                x[j] = mul_shoup(x[j], w.w, w.wq, p);
-            }
-#pragma unroll
-            for (int m = 0; m < R0; ++m) tile[off + tile_step<L1, KIND, R1>(m)] = x[m];
-        }
-        __syncthreads();  // tile complete; the stage is free
-
-        if (t + (int)gridDim.x < ntiles) {
-            const u32* src; long long len; u32* dst; int c0;
-            decode(t + gridDim.x, src, len, dst, c0);
-            rows_issue(stage, src, len, c0, 0, HALF);
-        }
-
-        // level 1 (last): block blk = rows blk * R1 + m, straight to HBM
-        const u32* src; long long len; u32* dst; int c0;
-        decode(t, src, len, dst, c0);
-        for (int blk = warp * SUB + lane / TC; blk < R0; blk += NW * SUB) {
-            u32 x[R1];
-            const int off = tile_row<L1, KIND>(blk * R1) + col;
-#pragma unroll
-            for (int m = 0; m < R1; ++m) x[m] = tile[off + tile_step<L1, KIND, 1>(m)];
-            dif_regs<R1>(x, A.pkc.rc.f, p, p2);
-            // running pointer: 64-bit adds on the ALU pipe, not a multiply per store
-            u32* out = dst + (size_t)(blk * R1) * n2 + c0 + col;
-#pragma unroll
-            for (int m = 0; m < R1; ++m, out += n2) *out = x[m];
-        }
-    }
-}
-
-// Pass A of a natural-order transform (one full-length operand per job,
-// written over wa) as a persistent, software-pipelined kernel for 2^10-row
-// columns on 16-column tiles: the whole next tile is staged by cp.async
-// (zero-filled past the operand's end; word by word for an unaligned
-// source) while the current one is transformed.  Level 0 reads and reduces
-// the stage and writes the tile; level 1 stores straight to HBM.  Results
-// are those of k_col_fwd<L1, NW, 2>.
-template <int L1, int NW>
-__global__ void __launch_bounds__(NW * 32, 1) k_col_fwd_pipe1(const __grid_constant__ LargeArgs A) {
-    constexpr LevelPlan PL = col_plan(L1);
-    static_assert(PL.nlev == 2, "two-level column plans only");
-    constexpr int KIND = 2, n1 = 1 << L1, T = NW * 32;
-    constexpr int R0 = 1 << PL.logr[0], R1 = 1 << PL.logr[1];  // n1 = R0 * R1
-    constexpr int TC = col_tile_cols(L1, KIND), SUB = 32 / TC, QR = TC / 4;
-    constexpr int TW = col_tile_words(L1, KIND);
-    extern __shared__ __align__(16) u32 smem[];
-    u32* tile = smem;
-    u32* stage = smem + TW;
-    Tw* tws = reinterpret_cast<Tw*>(stage + TW);  // level-0 twiddles (n1 entries)
-    const int n2 = 1 << A.l2, ct = n2 / TC;
-    const int ntiles = ct * A.njobs;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int col = lane % TC;
-    const u32 p = A.pkc.p, p2 = A.pkc.p2, oneq = A.pkc.one_q;
-    for (int i = threadIdx.x; i < n1; i += T) tws[i] = A.twc[i];
-
-    // all n1 rows x TC columns of tile t into the stage (one commit group);
-    // words at or past the operand's length read as 0
-    auto stage_issue = [&](int t) {
-        const LargeJob& J = A.jobs ? A.jobs[t / ct] : A.job0;
-        const u32* src = J.a;
-        const long long len = J.la;
-        const int c0 = (t % ct) * TC;
-        if ((reinterpret_cast<uintptr_t>(src) & 15) == 0) {
-            static_assert(T % QR == 0, "whole rows per thread round");
-            const int q = threadIdx.x % QR;
-            const long long step = (long long)(T / QR) * n2;
-            long long gi = (long long)(threadIdx.x / QR) * n2 + c0 + 4 * q;
-#pragma unroll 4
-            for (int r = threadIdx.x / QR; r < n1; r += T / QR, gi += step) {
-                const long long rem = len - gi;
-                const int bytes = rem >= 4 ? 16 : (rem > 0 ? (int)rem * 4 : 0);
-                const u32* g = bytes ? src + gi : src;
-                const unsigned d = (unsigned)__cvta_generic_to_shared(stage + tile_row<L1, KIND>(r) + 4 * q);
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(g), "r"(bytes) : "memory");
-            }
-        } else {
-            for (int idx = threadIdx.x; idx < n1 * TC; idx += T) {
-                const int r = idx / TC, c = idx % TC;
-                const long long gi = (long long)r * n2 + c0 + c;
-                const int bytes = gi < len ? 4 : 0;
-                const u32* g = bytes ? src + gi : src;
-                const unsigned d = (unsigned)__cvta_generic_to_shared(stage + tile_row<L1, KIND>(r) + c);
-                asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(d), "l"(g), "r"(bytes) : "memory");
-            }
-        }
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
-    };
-
-    int t = blockIdx.x;
-    if (t < ntiles) stage_issue(t);
-    for (; t < ntiles; t += gridDim.x) {
-        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-        __syncthreads();  // stage and twiddles visible; the previous tile's level 1 is done with `tile`
-
-        // level 0: task o (rows o + R1 m), inputs reduced, DIF, twiddles, stage -> tile
-        for (int o = warp * SUB + lane / TC; o < R1; o += NW * SUB) {
-            u32 x[R0];
-            const int off = tile_row<L1, KIND>(o) + col;
-#pragma unroll
-            for (int m = 0; m < R0; ++m) x[m] = mul_shoup(stage[off + tile_step<L1, KIND, R1>(m)], 1u, oneq, p);
-            dif_regs<R0, true>(x, A.pkc.rc.f, p, p2);
-#pragma unroll
-            for (int j = 1; j < R0; ++j) {
-                const Tw w = tws[o * R0 + j];
-                x[j] = mul_shoup(x[j], w.w, w.wq, p);
-            }
-#pragma unroll
-            for (int m = 0; m < R0; ++m) tile[off + tile_step<L1, KIND, R1>(m)] = x[m];
-        }
-        __syncthreads();  // tile complete; the stage is free
-        if (t + (int)gridDim.x < ntiles) stage_issue(t + gridDim.x);
-
-        // level 1 (last): block blk = rows blk * R1 + m, straight to HBM
-        const LargeJob& J = A.jobs ? A.jobs[t / ct] : A.job0;
-        const int c0 = (t % ct) * TC;
-        for (int blk = warp * SUB + lane / TC; blk < R0; blk += NW * SUB) {
-            u32 x[R1];
-            const int off = tile_row<L1, KIND>(blk * R1) + col;
-#pragma unroll
-            for (int m = 0; m < R1; ++m) x[m] = tile[off + tile_step<L1, KIND, 1>(m)];
-            dif_regs<R1>(x, A.pkc.rc.f, p, p2);
-            u32* out = J.wa + (size_t)(blk * R1) * n2 + c0 + col;
-#pragma unroll
-            for (int m = 0; m < R1; ++m, out += n2) *out = x[m];
-        }
-    }
-}
-
-// Pass C as a persistent, software-pipelined kernel for the two-level
-// column plans (n1 = 2^9: 32-column tiles, n1 = 2^10: 16-column tiles, the
-// inverse pass's layouts).  Each CTA walks the tiles gridDim.x apart; the
-// whole next tile is copied into a stage buffer (cp.async) while the current
-// one is transformed: each warp refills the stage rows of its own blocks as
-// soon as its deepest-level tasks have consumed them.  The deepest level
-// reads the stage and writes the tile; level 0 reads the tile and stores the
-// canonical residues straight to the output, truncated at lh.  Results are
-// those of k_col_inv.
-template <int L1, int NW>
-__global__ void __launch_bounds__(NW * 32, 1) k_col_inv_pipe(const __grid_constant__ LargeArgs A) {
-    constexpr LevelPlan PL = col_plan(L1);
-    static_assert(PL.nlev == 2, "two-level column plans only");
-    constexpr int INV = 1, T = NW * 32;
-    constexpr int TC = col_tile_cols(L1, INV), SUB = 32 / TC, QR = TC / 4;
-    constexpr int n1 = 1 << L1, R0 = 1 << PL.logr[0], R1 = 1 << PL.logr[1];  // n1 = R0 * R1
-    constexpr int TW = col_tile_words(L1, INV);
-    extern __shared__ __align__(16) u32 smem[];
-    u32* tile = smem;
-    u32* stage = smem + TW;
-    Tw* tws = reinterpret_cast<Tw*>(stage + TW);  // inverse level-0 twiddles (n1 entries)
-    const int n2 = 1 << A.l2, ct = n2 / TC;
-    const int ntiles = ct * A.njobs;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int col = lane % TC;
-    const u32 p = A.pkc.p, p2 = A.pkc.p2;
-    for (int i = threadIdx.x; i < n1; i += T) tws[i] = A.twc[A.twc_inv + i];
-
-    // the whole tile t (all n1 rows of the row pass's output) into the stage
-    // (the first tile; later ones are refilled per warp)
-    auto stage_issue = [&](int t) {
-        const LargeJob& J = A.jobs ? A.jobs[t / ct] : A.job0;
-        // a thread keeps one quad column q and walks rows T / QR apart
-        static_assert(T % QR == 0, "whole rows per thread round");
-        const int q = threadIdx.x % QR;
-        const u32* src = J.wa + (t % ct) * TC + (size_t)(threadIdx.x / QR) * n2 + 4 * q;
-        const size_t step = (size_t)(T / QR) * n2;
-#pragma unroll 4
-        for (int r = threadIdx.x / QR; r < n1; r += T / QR, src += step) {
-            const unsigned d = (unsigned)__cvta_generic_to_shared(stage + tile_row<L1, INV>(r) + 4 * q);
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src) : "memory");
-        }
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
-    };
-
-    pdl_wait();  // pass B's output
-    int t = blockIdx.x;
-    if (t < ntiles) stage_issue(t);
-    for (; t < ntiles; t += gridDim.x) {
-        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-        __syncthreads();  // stage and twiddles visible; the previous tile's level 0 is done with `tile`
-
-        // deepest level: blocks of R1 consecutive rows, DIT, stage -> tile
-        for (int id = warp * SUB + lane / TC; id < R0; id += NW * SUB) {
-            u32 x[R1];
-            const int off = tile_row<L1, INV>(id * R1) + col;
-#pragma unroll
-            for (int m = 0; m < R1; ++m) x[m] = stage[off + tile_step<L1, INV, 1>(m)];
-            dit_regs<R1, false>(x, A.pkc.rc.i, p, p2);
-#pragma unroll
-            for (int m = 0; m < R1; ++m) tile[off + tile_step<L1, INV, 1>(m)] = x[m];
-        }
-        // this warp's blocks (rows [warp SUB R1, (warp + 1) SUB R1)) have been
-        // read (their words reached the tile), so the warp refills those stage
-        // rows with the next tile's at once, half a tile earlier than a
-        // CTA-wide refill after the barrier
-        static_assert(NW * SUB == R0, "one block set per warp");
-        __syncwarp();
-        if (t + (int)gridDim.x < ntiles) {
-            const int tn = t + gridDim.x;
-            const LargeJob& Jn = A.jobs ? A.jobs[tn / ct] : A.job0;
-            const int q = lane % QR;
-            const int r0 = warp * SUB * R1 + lane / QR;
-            const u32* src = Jn.wa + (tn % ct) * TC + (size_t)r0 * n2 + 4 * q;
-            const size_t step = (size_t)(32 / QR) * n2;
-#pragma unroll 4
-            for (int r = r0; r < (warp + 1) * SUB * R1; r += 32 / QR, src += step) {
-                const unsigned d = (unsigned)__cvta_generic_to_shared(stage + tile_row<L1, INV>(r) + 4 * q);
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src) : "memory");
-            }
-        }
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
-        __syncthreads();  // tile complete
-
-        // level 0: task o (rows o + R1 m), pre-twiddle, DIT, canonical residues out
-        const LargeJob& J = A.jobs ? A.jobs[t / ct] : A.job0;
-        const long long lh = J.lh;
-        const int c0 = (t % ct) * TC;
-        for (int o = warp * SUB + lane / TC; o < R1; o += NW * SUB) {
-            u32 x[R0];
-            const int off = tile_row<L1, INV>(o) + col;
-#pragma unroll
-            for (int m = 0; m < R0; ++m) x[m] = tile[off + tile_step<L1, INV, R1>(m)];
-#pragma unroll
-            for (int j = 1; j < R0; ++j) {
-                const Tw w = tws[o * R0 + j];
-                x[j] = mul_shoup(x[j], w.w, w.wq, p);
-            }
-            dit_regs<R0, true>(x, A.pkc.rc.i, p, p2);
-            // running index and pointer (64-bit adds on the ALU pipe)
-            long long gi = (long long)o * n2 + c0 + col;
-            u32* out = J.h + gi;
-            const long long step = (long long)R1 * n2;
-#pragma unroll
-            for (int m = 0; m < R0; ++m, gi += step, out += step)
-                if (gi < lh) *out = red1(red2(x[m], p2), p);
-        }
-    }
 }
 
 // pass C, grid: (n2/TC column tiles, 1, jobs)

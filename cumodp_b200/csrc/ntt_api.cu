@@ -378,12 +378,6 @@ void launch_colfwd1_t(const LargeArgs& a, int tiles, cudaStream_t st) {
     }
     k_col_fwd<L1, col_warps(L1, 2), 2><<<dim3(tiles, 1, a.njobs), col_warps(L1, 2) * 32, smem, st>>>(a);
 }
-typedef void (*ColFn)(const LargeArgs&, int, cudaStream_t);
-const ColFn kColFwd1[12] = {nullptr, launch_colfwd1_t<1>, launch_colfwd1_t<2>, launch_colfwd1_t<3>,
-                            launch_colfwd1_t<4>, launch_colfwd1_t<5>, launch_colfwd1_t<6>,
-                            launch_colfwd1_t<7>, launch_colfwd1_t<8>, launch_colfwd1_t<9>,
-                            launch_colfwd1_t<10>, launch_colfwd1_t<11>};
-
 // w is a primitive 2^k-th root of unity mod p.
 bool root_has_order(u32 w, int k, u32 p) {
     if (w == 0 || w >= p) return false;
@@ -411,7 +405,7 @@ int column_pass(const PrimeCtx& pc, u32 root_c, int l1, int l2, const u32* src, 
     A.job0 = LargeJob{src, nullptr, nullptr, (int)std::min<long long>(len, 1ll << 30), 0, 0, 0, dst, nullptr};
     A.jobs = djobs;  // a device job table (a list of transforms), or nullptr: job0
     A.njobs = njobs;
-    if (!launch_col_fwd_pipe1(A, njobs, st)) kColFwd1[l1](A, (1 << l2) / col_tile_cols_rt(l1, 2), st);
+    if (!launch_col_fwd1(A, njobs, st)) launch_colfwd1_t<kMaxColLog>(A, (1 << l2) / col_tile_cols(kMaxColLog, 2), st);
     return OK;
 }
 

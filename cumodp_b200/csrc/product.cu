@@ -1,4 +1,5 @@
 // Product dispatch: size classes, kernel instantiation tables, launches.
+#include "col_direct.cuh"
 #include "product.cuh"
 
 #include <algorithm>
@@ -74,30 +75,6 @@ int sm_count(int dev) {
 }
 
 namespace {
-
-// Whether pass A uses the persistent pipelined kernel where it applies
-// (CUMODP_COL_PIPE=0 selects the one-tile-per-CTA kernel, for comparison).
-bool col_pipe_enabled() {
-    static const bool on = [] {
-        const char* e = getenv("CUMODP_COL_PIPE");
-        return !(e && e[0] == '0');
-    }();
-    return on;
-}
-
-template <int L1>
-void launch_col_fwd_pipe_t(const LargeArgs& a, int ntiles, cudaStream_t st) {
-    constexpr int smem = col_pipe_smem_bytes(L1);
-    const int grid = std::min(ntiles, sm_count(current_device()) * col_pipe_ctas(L1));
-    k_col_fwd_pipe<L1, col_pipe_kind(L1), col_pipe_warps(L1)><<<grid, col_pipe_warps(L1) * 32, smem, st>>>(a);
-}
-
-template <int L1>
-void launch_col_inv_pipe_t(const LargeArgs& a, int ntiles, cudaStream_t st) {
-    const int grid = std::min(ntiles, sm_count(current_device()));
-    launch_pdl(k_col_inv_pipe<L1, col_inv_pipe_warps(L1)>, dim3(grid), col_inv_pipe_warps(L1) * 32,
-               (size_t)col_inv_pipe_smem_bytes(L1), st, a);
-}
 
 template <int L1>
 void launch_col_inv_t(const LargeArgs& a, dim3 grid, cudaStream_t st) {
@@ -195,15 +172,33 @@ void launch_row_f_t(const LargeArgs& a, dim3 grid, cudaStream_t st) {
     launch_pdl(k_row_mul_f<L2>, grid, rowsplit_threads(L2), rowsplit_smem<L2>(), st, a);
 }
 
+// The register column passes (col_direct.cuh): njobs jobs of `ops` operands.
+template <int L1>
+void launch_cold_fwd_t(const LargeArgs& a, int ops, int njobs, cudaStream_t st) {
+    const int n2 = 1 << a.l2;
+    k_cold_fwd<L1><<<dim3((n2 + cold_cols(L1) - 1) / cold_cols(L1), ops, njobs), cold_threads(L1), cold_smem(L1), st>>>(a);
+}
+template <int L1>
+void launch_cold_inv_t(const LargeArgs& a, int njobs, cudaStream_t st) {
+    const int n2 = 1 << a.l2;
+    launch_pdl(k_cold_inv<L1>, dim3((n2 + cold_cols(L1) - 1) / cold_cols(L1), 1, njobs), cold_threads(L1), cold_smem(L1),
+               st, a);
+}
+template <int L1>
+void attr_cold() {
+    cudaFuncSetAttribute(k_cold_fwd<L1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cold_smem(L1));
+    cudaFuncSetAttribute(k_cold_inv<L1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cold_smem(L1));
+}
+typedef void (*ColdFwdFn)(const LargeArgs&, int, int, cudaStream_t);
+typedef void (*ColdInvFn)(const LargeArgs&, int, cudaStream_t);
+const ColdFwdFn kColdFwd[kMaxDirectColLog + 1] = {
+    nullptr, launch_cold_fwd_t<1>, launch_cold_fwd_t<2>, launch_cold_fwd_t<3>, launch_cold_fwd_t<4>, launch_cold_fwd_t<5>,
+    launch_cold_fwd_t<6>, launch_cold_fwd_t<7>, launch_cold_fwd_t<8>, launch_cold_fwd_t<9>, launch_cold_fwd_t<10>};
+const ColdInvFn kColdInv[kMaxDirectColLog + 1] = {
+    nullptr, launch_cold_inv_t<1>, launch_cold_inv_t<2>, launch_cold_inv_t<3>, launch_cold_inv_t<4>, launch_cold_inv_t<5>,
+    launch_cold_inv_t<6>, launch_cold_inv_t<7>, launch_cold_inv_t<8>, launch_cold_inv_t<9>, launch_cold_inv_t<10>};
+
 typedef void (*PassFn)(const LargeArgs&, dim3, cudaStream_t);
-const PassFn kColFwd[12] = {nullptr, launch_col_fwd_t<1>, launch_col_fwd_t<2>, launch_col_fwd_t<3>,
-                            launch_col_fwd_t<4>, launch_col_fwd_t<5>, launch_col_fwd_t<6>,
-                            launch_col_fwd_t<7>, launch_col_fwd_t<8>, launch_col_fwd_t<9>,
-                            launch_col_fwd_t<10>, launch_col_fwd_t<11>};
-const PassFn kColInv[12] = {nullptr, launch_col_inv_t<1>, launch_col_inv_t<2>, launch_col_inv_t<3>,
-                            launch_col_inv_t<4>, launch_col_inv_t<5>, launch_col_inv_t<6>,
-                            launch_col_inv_t<7>, launch_col_inv_t<8>, launch_col_inv_t<9>,
-                            launch_col_inv_t<10>, launch_col_inv_t<11>};
 const PassFn kRow[15] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
                          launch_row_t<6>, launch_row_t<7>, launch_row_t<8>, launch_row_t<9>,
                          launch_row_t<10>, launch_row_t<11>, launch_row_t<12>, launch_row_t<13>,
@@ -220,17 +215,6 @@ void attr_col() {
                          col_smem_bytes(L1, false));
     cudaFuncSetAttribute(k_col_inv<L1, col_warps(L1, true)>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          col_smem_bytes(L1, true));
-}
-void attr_col_pipe1() {
-    cudaFuncSetAttribute(k_col_fwd_pipe1<10, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         col_pipe1_smem_bytes(10));
-}
-template <int L1>
-void attr_col_pipe() {
-    cudaFuncSetAttribute(k_col_fwd_pipe<L1, col_pipe_kind(L1), col_pipe_warps(L1)>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         col_pipe_smem_bytes(L1));
-    cudaFuncSetAttribute(k_col_inv_pipe<L1, col_inv_pipe_warps(L1)>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         col_inv_pipe_smem_bytes(L1));
 }
 template <int L2>
 void attr_row() {
@@ -267,9 +251,8 @@ void ensure_kernel_attrs() {
     std::call_once(once, [] {
         attr_small<5>(); attr_small<6>(); attr_small<7>(); attr_small<8>(); attr_small<9>();
         attr_small<10>(); attr_small<11>(); attr_small<12>(); attr_small<13>(); attr_small<14>();
-        attr_col<1>(); attr_col<2>(); attr_col<3>(); attr_col<4>(); attr_col<5>();
-        attr_col<6>(); attr_col<7>(); attr_col<8>(); attr_col<9>(); attr_col<10>(); attr_col<11>();
-        attr_col_pipe<9>(); attr_col_pipe<10>(); attr_col_pipe1();
+        attr_col<11>();
+        attr_cold<6>(); attr_cold<7>(); attr_cold<8>(); attr_cold<9>(); attr_cold<10>();
         attr_row<6>(); attr_row<7>(); attr_row<8>(); attr_row<9>(); attr_row<10>();
         attr_row<11>(); attr_row<12>(); attr_row<13>(); attr_row<14>();
         attr_rowsplit<6>(); attr_rowsplit<7>(); attr_rowsplit<8>(); attr_rowsplit<9>(); attr_rowsplit<10>();
@@ -364,56 +347,30 @@ void launch_small(int logn, const SmallArgs& a, int njobs, cudaStream_t st) {
     if (tr) pass_timing_end(st, kSmallName[logn], e0);
 }
 
-bool launch_col_fwd_pipe(const LargeArgs& a, int njobs, cudaStream_t st) {
-    if (!col_pipe_ok(a.l1) || !col_pipe_enabled()) return false;
-    const int ntiles = ((1 << a.l2) / col_tile_cols_rt(a.l1, col_pipe_kind(a.l1))) * 2 * njobs;
-    if (a.l1 == 10) launch_col_fwd_pipe_t<10>(a, ntiles, st);
-    else launch_col_fwd_pipe_t<9>(a, ntiles, st);
-    return true;
-}
-
-bool launch_col_fwd_pipe1(const LargeArgs& a, int njobs, cudaStream_t st) {
-    if (a.l1 != 10 || !col_pipe_enabled()) return false;
-    ensure_kernel_attrs();
-    const int ntiles = ((1 << a.l2) / col_tile_cols_rt(10, 2)) * njobs;
-    const int grid = std::min(ntiles, sm_count(current_device()));
-    k_col_fwd_pipe1<10, 16><<<grid, 16 * 32, col_pipe1_smem_bytes(10), st>>>(a);
-    return true;
-}
-
 void launch_col_fwd(const LargeArgs& a, int njobs, cudaStream_t st) {
     cudaEvent_t e0;
     const bool tr = pass_timing_begin(st, &e0);
-    if (!launch_col_fwd_pipe(a, njobs, st))
-        kColFwd[a.l1](a, dim3((1 << a.l2) / col_tile_cols_rt(a.l1, false), 2, njobs), st);
+    if (a.l1 <= kMaxDirectColLog)
+        kColdFwd[a.l1](a, 2, njobs, st);
+    else
+        launch_col_fwd_t<kMaxColLog>(a, dim3((1 << a.l2) / col_tile_cols(kMaxColLog, false), 2, njobs), st);
     if (tr) pass_timing_end(st, kColFwdName[a.l1], e0);
 }
 
-void launch_col_fwd_full(const LargeArgs& a, cudaStream_t st) {
-    if (a.l1 != 10) {
-        launch_col_fwd(a, 1, st);
-        return;
-    }
-    LargeArgs b = a;
-    b.job0.a = a.job0.b;
-    b.job0.la = a.job0.lb;
-    b.job0.wa = a.job0.wb;
-    cudaEvent_t e0;
-    const bool tr = pass_timing_begin(st, &e0);
-    if (!launch_col_fwd_pipe1(a, 1, st) || !launch_col_fwd_pipe1(b, 1, st)) launch_col_fwd(a, 1, st);
-    if (tr) pass_timing_end(st, kColFwdName[a.l1], e0);
+bool launch_col_fwd1(const LargeArgs& a, int njobs, cudaStream_t st) {
+    if (a.l1 > kMaxDirectColLog) return false;
+    ensure_kernel_attrs();
+    kColdFwd[a.l1](a, 1, njobs, st);
+    return true;
 }
 
 void launch_col_inv(const LargeArgs& a, int njobs, cudaStream_t st) {
-    const int n2 = 1 << a.l2;
     cudaEvent_t e0;
     const bool tr = pass_timing_begin(st, &e0);
-    if (col_pipe_ok(a.l1) && col_pipe_enabled()) {
-        const int ntiles = (n2 / col_tile_cols_rt(a.l1, true)) * njobs;
-        if (a.l1 == 10) launch_col_inv_pipe_t<10>(a, ntiles, st);
-        else launch_col_inv_pipe_t<9>(a, ntiles, st);
+    if (a.l1 <= kMaxDirectColLog) {
+        kColdInv[a.l1](a, njobs, st);
     } else {
-        kColInv[a.l1](a, dim3(n2 / col_tile_cols_rt(a.l1, true), 1, njobs), st);
+        launch_col_inv_t<kMaxColLog>(a, dim3((1 << a.l2) / col_tile_cols(kMaxColLog, true), 1, njobs), st);
     }
     if (tr) pass_timing_end(st, kColInvName[a.l1], e0);
 }

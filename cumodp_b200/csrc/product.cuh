@@ -34,16 +34,10 @@ int default_row_log(int logn);
 
 int small_args(const PrimeCtx& pc, u32 root, int logn, int dev, SmallArgs* a);
 int large_args(const PrimeCtx& pc, u32 root_n, int logn, int l2, int dev, LargeArgs* a);
-// A product's pass A through the persistent pipelined kernel when the column
-// length has one (2^9, 2^10 rows); false when the caller must launch k_col_fwd.
-bool launch_col_fwd_pipe(const LargeArgs& a, int njobs, cudaStream_t st);
-// A natural-order transform's column pass (operand a of each job, over wa)
-// through k_col_fwd_pipe1 when the columns have 2^10 rows; false otherwise.
-bool launch_col_fwd_pipe1(const LargeArgs& a, int njobs, cudaStream_t st);
-// The forward column pass of every job's two operands, the same for job0 with
-// operands as long as the transform (no zero half), the inverse column pass.
+// The forward column pass of every job's two operands; that of operand a alone
+// (false past 2^kMaxDirectColLog rows); the inverse column pass.
 void launch_col_fwd(const LargeArgs& a, int njobs, cudaStream_t st);
-void launch_col_fwd_full(const LargeArgs& a, cudaStream_t st);
+bool launch_col_fwd1(const LargeArgs& a, int njobs, cudaStream_t st);
 void launch_col_inv(const LargeArgs& a, int njobs, cudaStream_t st);
 void launch_small(int logn, const SmallArgs& a, int njobs, cudaStream_t st);
 void launch_large(const LargeArgs& a, int njobs, cudaStream_t st);
