@@ -36,8 +36,8 @@ struct GridArgs {
 
 // Words of one CTA: a whole row, and at least 2^11.
 __host__ __device__ constexpr int grid_log(int e, int l2) { return e + l2 > 11 ? e + l2 : 11; }
-__host__ __device__ constexpr int grid_threads(int lt) { return lt == 14 ? 256 : 1 << (lt - 5); }
-__host__ __device__ constexpr int grid_ctas(int lt) { return lt == 14 ? 3 : 1024 / grid_threads(lt); }
+__host__ __device__ constexpr int grid_threads(int lt) { return 1 << (lt - 5); }
+__host__ __device__ constexpr int grid_ctas(int lt) { return 1024 / grid_threads(lt); }
 
 #ifdef __CUDACC__
 
@@ -56,7 +56,7 @@ __device__ __forceinline__ void grid_fwd_levels(u32* sm, const GridArgs& A) {
             for (int m = 0; m < R; ++m) x[m] = sm[swz_task<TB, B>(base, bs, m)];
             dif_regs<R, true>(x, A.pk.rc.f, p, p2);
             Tw t[R];
-            load_tw<R>(t, A.twr + LV::TWOFF + o * R);
+            load_tw<R, TB>(t, A.twr + LV::TWOFF + o);
 #pragma unroll
             for (int j = 1; j < R; ++j) x[j] = mul_shoup(x[j], t[j].w, t[j].wq, p);
 #pragma unroll
@@ -80,7 +80,7 @@ __device__ __forceinline__ void grid_inv_levels(u32* sm, const GridArgs& A) {
 #pragma unroll
             for (int m = 0; m < R; ++m) x[m] = sm[swz_task<TB, B>(base, bs, m)];
             Tw t[R];
-            load_tw<R>(t, A.twr + A.twr_inv + LV::TWOFF + o * R);
+            load_tw<R, TB>(t, A.twr + A.twr_inv + LV::TWOFF + o);
 #pragma unroll
             for (int j = 1; j < R; ++j) x[j] = mul_shoup(x[j], t[j].w, t[j].wq, p);
             dit_regs<R, true>(x, A.pk.rc.i, p, p2);
@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(grid_threads(grid_log(E, L2)), grid_ctas(grid_
             const int o = id % TB, base = (id / TB) * B + o, bs = swz(base);
             u32 x[R];
             Tw t[R];
-            load_tw<R>(t, A.twr + A.twr_inv + o * R);
+            load_tw<R, TB>(t, A.twr + A.twr_inv + o);
 #pragma unroll
             for (int m = 0; m < R; ++m) {
                 x[m] = sm[swz_task<TB, B>(base, bs, m)];

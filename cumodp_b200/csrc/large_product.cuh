@@ -404,7 +404,7 @@ __global__ void __launch_bounds__(row_threads(L2), 1) k_row_fused(const __grid_c
         dif_regs<R0, true>(xf, A.pk.rc.f, p, p2);
         dif_regs<R0, true>(xg, A.pk.rc.f, p, p2);
         Tw t[R0];
-        load_tw<R0>(t, A.twr + o * R0);
+        load_tw<R0, TB0>(t, A.twr + o);
 #pragma unroll
         for (int j = 1; j < R0; ++j) {
             xf[j] = mul_shoup(xf[j], t[j].w, t[j].wq, p);
@@ -453,7 +453,7 @@ __global__ void __launch_bounds__(row_threads(L2), 1) k_row_fused(const __grid_c
 #pragma unroll
         for (int m = 0; m < R0; ++m) x[m] = sm[swz_task<TB0, n2>(o, swz(o), m)];
         Tw t[R0];
-        load_tw<R0>(t, A.twr + A.twr_inv + o * R0);
+        load_tw<R0, TB0>(t, A.twr + A.twr_inv + o);
 #pragma unroll
         for (int j = 1; j < R0; ++j) x[j] = mul_shoup(x[j], t[j].w, t[j].wq, p);
         dit_regs<R0, true>(x, A.pk.rc.i, p, p2);
@@ -587,7 +587,7 @@ __device__ __forceinline__ void row_wpow_build(u32* wp, const LargeArgs& A, u32 
 }
 
 // The U entries of one direction from the powers wp and that direction's
-// level-0 twiddles twl (entry e R0 + j = w_n2^(+-e rev(j))).  The loop runs
+// level-0 twiddles twl (entry j TB0 + e = w_n2^(+-e rev(j))).  The loop runs
 // j fastest so the twiddle reads are coalesced.
 template <int L2, int T>
 __device__ __forceinline__ void row_tab_build(Tw* tab, const u32* wp, const Tw* __restrict__ twl, const LargeArgs& A) {
@@ -603,7 +603,7 @@ __device__ __forceinline__ void row_tab_build(Tw* tab, const u32* wp, const Tw* 
             const int k = (q - RT::R0 * RT::NA) / RT::R0;
             e = k * RT::NA; w = RT::NA + k; at = RT::R0 * RT::NA + j * RT::NB + k;
         }
-        const u32 v = red1(mul_mont(wp[w], __ldg(&twl[e * RT::R0 + j].w), p, pinv), p);
+        const u32 v = red1(mul_mont(wp[w], __ldg(&twl[j * RT::TB0 + e].w), p, pinv), p);
         tab[at] = Tw{v, shoup_quot_dev(v, p, A.r32p)};
     }
 }
@@ -655,7 +655,7 @@ __device__ __forceinline__ void row_level0_fwd_seeds(u32* sm, const LargeArgs& A
     const u32 p = A.pk.p, p2 = A.pk.p2, pinv = A.pk.pinv_neg;
     for (int o = threadIdx.x; o < TB0; o += T) {
         Tw t[R0];
-        load_tw<R0>(t, A.twr + o * R0);
+        load_tw<R0, TB0>(t, A.twr + o);
         const u32 mo = seed_mont(A, (k1 * (u32)o) & nmask, false);  // w^(k1 o) * 2^32
         u32 x[R0];
 #pragma unroll
@@ -669,35 +669,50 @@ __device__ __forceinline__ void row_level0_fwd_seeds(u32* sm, const LargeArgs& A
     }
 }
 
-// Level 0 forward of one operand: slot factors on the inputs, DIF, the
-// per-row factors U_j^o on the outputs.
+// Level 0 forward of one operand, from global memory (row) into sm: slot
+// factors on the inputs, DIF, the per-row factors U_j^o on the outputs.  A
+// thread's first words are loaded before the factor table is waited for.
 template <int L2, int T>
-__device__ __forceinline__ void row_level0_fwd(u32* sm, const LargeArgs& A, const Tw* tab) {
+__device__ __forceinline__ void row_level0_fwd(u32* sm, const u32* row, const LargeArgs& A, const Tw* tab) {
     using RT = RowTab<L2>;
     constexpr int R0 = RT::R0, TB0 = RT::TB0;
     static_assert(T % RT::NA == 0, "the tasks of a thread share o mod NA");
     const u32 p = A.pk.p, p2 = A.pk.p2;
     // the slot factors and this thread's U_j^(o mod NA) are the same for all
-    // of its tasks: kept in registers
-    Tw vf[R0], af[R0];
+    // of its tasks: kept in registers up to radix 8
+    u32 x[R0];
 #pragma unroll
-    for (int j = 0; j < R0; ++j) {
-        vf[j] = tab[RT::ENTRIES + j];
-        af[j] = tab[j * RT::NA + threadIdx.x % RT::NA];
+    for (int m = 0; m < R0; ++m) x[m] = row[threadIdx.x + TB0 * m];
+    row_load_wait();  // the table
+    __syncthreads();
+    constexpr bool KEEP = R0 <= 8;
+    const Tw* const vt = tab + RT::ENTRIES;
+    const Tw* const at = tab + threadIdx.x % RT::NA;
+    Tw vf[KEEP ? R0 : 1], af[KEEP ? R0 : 1];
+    if constexpr (KEEP) {
+#pragma unroll
+        for (int j = 0; j < R0; ++j) {
+            vf[j] = vt[j];
+            af[j] = at[j * RT::NA];
+        }
     }
+    static_assert(T <= TB0, "every thread has a first task");
     for (int o = threadIdx.x; o < TB0; o += T) {
-        u32 x[R0];
+        if (o != (int)threadIdx.x) {
 #pragma unroll
-        for (int m = 0; m < R0; ++m) {
-            const u32 v = sm[swz_task<TB0, (1 << L2)>(o, swz(o), m)];
-            x[m] = m == 0 ? v : mul_shoup(v, vf[m].w, vf[m].wq, p);
+            for (int m = 0; m < R0; ++m) x[m] = row[o + TB0 * m];
+        }
+#pragma unroll
+        for (int m = 1; m < R0; ++m) {
+            const Tw f = KEEP ? vf[KEEP ? m : 0] : vt[m];
+            x[m] = mul_shoup(x[m], f.w, f.wq, p);
         }
         dif_regs<R0, true>(x, A.pk.rc.f, p, p2);
         const Tw* tb = tab + RT::R0 * RT::NA + o / RT::NA;
 #pragma unroll
         for (int j = 0; j < R0; ++j) {
-            const Tw b = tb[j * RT::NB];
-            x[j] = mul_shoup(mul_shoup(x[j], af[j].w, af[j].wq, p), b.w, b.wq, p);
+            const Tw a = KEEP ? af[KEEP ? j : 0] : at[j * RT::NA], b = tb[j * RT::NB];
+            x[j] = mul_shoup(mul_shoup(x[j], a.w, a.wq, p), b.w, b.wq, p);
         }
 #pragma unroll
         for (int m = 0; m < R0; ++m) sm[swz_task<TB0, (1 << L2)>(o, swz(o), m)] = x[m];
@@ -725,11 +740,13 @@ __global__ void __launch_bounds__(rowsplit_threads(L2), rowsplit_ctas(L2)) k_row
     if constexpr (RowTab<L2>::USE) row_tab_fetch<L2, T>(tab, wp, A, s, k1, false);
     else row_slot_factors<L2>(A, k1, bf, nullptr);
     pdl_wait();  // pass A's columns of G
-    row_load_issue<L2, T>(sm, row);
-    row_load_wait();
-    __syncthreads();
-    if constexpr (RowTab<L2>::USE) row_level0_fwd<L2, T>(sm, A, tab);
-    else row_level0_fwd_seeds<L2, T>(sm, A, k1, bf);
+    if constexpr (RowTab<L2>::USE) {
+        row_level0_fwd<L2, T>(sm, row, A, tab);
+    } else {
+        row_load<L2, T>(sm, row);
+        __syncthreads();
+        row_level0_fwd_seeds<L2, T>(sm, A, k1, bf);
+    }
     __syncthreads();
     fwd1_levels<L2, 1, T>(sm, A.pk, A.twr);
     for (int r = threadIdx.x; r < n2 / 32; r += T) {
@@ -771,13 +788,16 @@ __global__ void __launch_bounds__(rowsplit_threads(L2), rowsplit_ctas(L2)) k_row
     // F's forward row pass depends only on pass A (complete before the
     // previous kernel, G's row pass, started), so it runs while that kernel
     // finishes; G's spectrum is read after pdl_wait
-    row_load_issue<L2, T>(sm, rowF);
-    if constexpr (RowTab<L2>::USE) row_tab_fetch<L2, T>(tab, wp, A, s, k1, false);
-    else row_slot_factors<L2>(A, k1, bf, bi);
-    row_load_wait();
-    __syncthreads();
-    if constexpr (RowTab<L2>::USE) row_level0_fwd<L2, T>(sm, A, tab);
-    else row_level0_fwd_seeds<L2, T>(sm, A, k1, bf);
+    if constexpr (RowTab<L2>::USE) {
+        row_tab_fetch<L2, T>(tab, wp, A, s, k1, false);
+        row_level0_fwd<L2, T>(sm, rowF, A, tab);
+    } else {
+        row_load_issue<L2, T>(sm, rowF);
+        row_slot_factors<L2>(A, k1, bf, bi);
+        row_load_wait();
+        __syncthreads();
+        row_level0_fwd_seeds<L2, T>(sm, A, k1, bf);
+    }
     __syncthreads();
     // level 0's inverse factors replace the forward ones; they are waited
     // for (prebuilt) or visible (built here) after the barriers below
@@ -806,16 +826,20 @@ __global__ void __launch_bounds__(rowsplit_threads(L2), rowsplit_ctas(L2)) k_row
     using RT = RowTab<L2>;
     if constexpr (RT::USE) {
         const Tw* bo = tab + RT::ENTRIES;
-        Tw af[R0];  // this thread's U_j^-(o mod NA), the same for all of its tasks
+        constexpr bool KEEP = R0 <= 8;
+        const Tw* const at = tab + threadIdx.x % RT::NA;
+        Tw af[KEEP ? R0 : 1];  // this thread's U_j^-(o mod NA), the same for all of its tasks
+        if constexpr (KEEP) {
 #pragma unroll
-        for (int j = 0; j < R0; ++j) af[j] = tab[j * RT::NA + threadIdx.x % RT::NA];
+            for (int j = 0; j < R0; ++j) af[j] = at[j * RT::NA];
+        }
         for (int o = threadIdx.x; o < TB0; o += T) {
             u32 x[R0];
             const Tw* tb = tab + RT::R0 * RT::NA + o / RT::NA;
 #pragma unroll
             for (int j = 0; j < R0; ++j) {
-                const Tw b = tb[j * RT::NB];
-                x[j] = mul_shoup(mul_shoup(sm[swz_task<TB0, n2>(o, swz(o), j)], af[j].w, af[j].wq, p), b.w, b.wq, p);
+                const Tw a = KEEP ? af[KEEP ? j : 0] : at[j * RT::NA], b = tb[j * RT::NB];
+                x[j] = mul_shoup(mul_shoup(sm[swz_task<TB0, n2>(o, swz(o), j)], a.w, a.wq, p), b.w, b.wq, p);
             }
             dit_regs<R0, true>(x, A.pk.rc.i, p, p2);
 #pragma unroll
@@ -828,7 +852,7 @@ __global__ void __launch_bounds__(rowsplit_threads(L2), rowsplit_ctas(L2)) k_row
 #pragma unroll
             for (int m = 0; m < R0; ++m) x[m] = sm[swz_task<TB0, n2>(o, swz(o), m)];
             Tw t[R0];
-            load_tw<R0>(t, A.twr + A.twr_inv + o * R0);
+            load_tw<R0, TB0>(t, A.twr + A.twr_inv + o);
 #pragma unroll
             for (int j = 1; j < R0; ++j) x[j] = mul_shoup(x[j], t[j].w, t[j].wq, p);
             dit_regs<R0, true>(x, A.pk.rc.i, p, p2);

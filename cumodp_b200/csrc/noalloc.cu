@@ -61,13 +61,14 @@ std::mutex g_na_m;
 NaDevice g_na[64];
 
 // One plan's level tables (the layout of level_tables_into: per level i,
-// task o and slot j at off_i + o R_i + j hold w_B^(o bitrev(j)) in Shoup
-// form, the forward tables first and the inverse ones nf entries later, then
+// task o and slot j at off_i + j TB_i + o (row plans) or off_i + o R_i + j
+// (column plans) hold w_B^(o bitrev(j)) in Shoup form, the forward tables first and the inverse ones nf entries later, then
 // two zero words), with w_B and w_B^-1 of every level in Montgomery form.
 struct NaPlan {
     Tw* out;
     LevelPlan pl;
     int logl, nf;
+    bool slot_major;  // a row plan's layout
     u32 wb[6], wbi[6];
 };
 
@@ -88,7 +89,8 @@ __device__ __forceinline__ Tw na_level_entry(const NaPlan& P, int t, u32 one_m, 
     for (int i = 0; i + 1 < P.pl.nlev; ++i) {
         const int r = P.pl.logr[i];
         if (t < off + (1 << lb)) {
-            const int q = t - off, o = q >> r, j = q & ((1 << r) - 1);
+            const int q = t - off, lt = lb - r;  // 2^lt tasks
+            const int o = P.slot_major ? q & ((1 << lt) - 1) : q >> r, j = P.slot_major ? q >> lt : q & ((1 << r) - 1);
             const u32 m = na_pow_m(inv ? P.wbi[i] : P.wb[i], (u64)o * rev_bits((u32)j, r), one_m, p, pinv);
             const u32 v = red1(mul_mont(m, 1u, p, pinv), p);
             return Tw{v, shoup_quot(v, p)};
@@ -124,13 +126,14 @@ __global__ void k_na_tables(const NaPlan row, const NaPlan col, u32* seeds, u32 
 }
 
 // The host side of k_na_tables' arguments for one plan (scalars only).
-NaPlan na_plan(Tw* out, const LevelPlan& pl, int logl, u32 root, const PrimeInfo& pi) {
+NaPlan na_plan(Tw* out, const LevelPlan& pl, int logl, u32 root, const PrimeInfo& pi, bool slot_major) {
     NaPlan P;
     memset(&P, 0, sizeof(P));
     P.out = out;
     P.pl = pl;
     P.logl = logl;
     P.nf = plan_tw_entries(pl, logl);
+    P.slot_major = slot_major;
     const u32 p = pi.p;
     const u32 rinv = powmod_exact(root, (1ull << logl) - 1, p);
     int lb = logl;
@@ -178,13 +181,13 @@ int mul_dev_noalloc(const u32* a, long long la, const u32* b, long long lb, u32*
     // of the product's kernels (nothing is carried over from earlier calls)
     {
         const PrimeInfo& pi = pc->info;
-        const NaPlan rowp = na_plan(d_row, row_plan(l2), l2, root_r, pi);
+        const NaPlan rowp = na_plan(d_row, row_plan(l2), l2, root_r, pi, true);
         NaPlan colp;
         memset(&colp, 0, sizeof(colp));
         u32 nlo = 0, nhi = 0, wm = 0, wim = 0, w4m = 0, wi4m = 0;
         if ((size_t)(2 * rowp.nf + 2) > kNaRowTw) return ASSUMPTION_ERROR;  // the array's row-table region
         if (large) {
-            colp = na_plan(d_col, col_plan(l1), l1, powmod_exact(root, 1ull << l2, p), pi);
+            colp = na_plan(d_col, col_plan(l1), l1, powmod_exact(root, 1ull << l2, p), pi, false);
             if ((size_t)(2 * colp.nf + 2) > kNaColTw || seed_words(logn) > kNaSeeds) return ASSUMPTION_ERROR;
             nlo = (u32)std::min<long long>(n, 4096);
             nhi = (u32)std::max<long long>(1, n / 4096);

@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(QOUT ? rowsplit_threads(L2) : ntt_row_threads(
         }
         dif_regs<R0, true>(x, A.pk.rc.f, p, p2);
         Tw t[R0];
-        load_tw<R0>(t, A.twr + o * R0);
+        load_tw<R0, TB0>(t, A.twr + o);
 #pragma unroll
         for (int j = 1; j < R0; ++j) x[j] = mul_shoup(x[j], t[j].w, t[j].wq, p);
 #pragma unroll

@@ -151,14 +151,15 @@ __device__ __forceinline__ void dit_regs(u32 (&x)[R], const Tw* __restrict__ c, 
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-template <int R>
+// Twiddles of one task of a level with TB tasks a block (slots j TB apart; a
+// warp's tasks read consecutive entries).  Slot 0's is 1 and not loaded.
+template <int R, int TB>
 __device__ __forceinline__ void load_tw(Tw (&t)[R], const Tw* __restrict__ src) {
-    const uint4* s4 = reinterpret_cast<const uint4*>(src);
+    t[0] = Tw{1u, 0u};
 #pragma unroll
-    for (int j = 0; j < R / 2; ++j) {
-        uint4 v = __ldg(s4 + j);
-        t[2 * j] = Tw{v.x, v.y};
-        t[2 * j + 1] = Tw{v.z, v.w};
+    for (int j = 1; j < R; ++j) {
+        const uint2 v = __ldg(reinterpret_cast<const uint2*>(src + j * TB));
+        t[j] = Tw{v.x, v.y};
     }
 }
 
@@ -169,7 +170,10 @@ __device__ __forceinline__ void load_tw(Tw (&t)[R], const Tw* __restrict__ src) 
 // Level i acts on blocks of size B_i = L >> (r_1 + ... + r_{i-1}).  Its
 // twiddle table holds, for each task o < B_i / R_i and register slot j < R_i,
 // w_{B_i}^(o * bitrev(j)) (forward) and the inverse root power (inverse), as
-// Tw pairs; the last level needs none (B_m = R_m).
+// Tw pairs; the last level needs none (B_m = R_m).  A row plan's table is
+// slot-major (entry (o, j) at j B_i / R_i + o: a warp's tasks, consecutive o,
+// read consecutive entries), a column plan's task-major (at o R_i + j: a
+// warp shares one task).
 // --------------------------------------------------------------------------
 struct LevelPlan {
     int nlev;

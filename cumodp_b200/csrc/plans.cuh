@@ -8,8 +8,10 @@ namespace cmb {
 // The last level always has radix 32: every earlier level then has at least
 // 32 tasks per block, so 32 lanes touch 32 consecutive words (no bank
 // conflicts), and the last level reads whole 32-word rows with 16-byte
-// accesses through the swizzle.  Earlier levels use radix <= 16 so that a
-// thread can hold both operands of a product (2 x 16 registers).
+// accesses through the swizzle.  From 2^12 on three levels: a fourth costs a
+// Shoup product, a twiddle and a shared-memory exchange per word (2^14-word
+// rows, g + f of a 2^24 product: 56 + 113 us with {3, 3, 3, 5}, 58 + 103 with
+// {4, 5, 5}).
 __host__ __device__ constexpr LevelPlan row_plan(int logl) {
     switch (logl) {
         case 5: return LevelPlan{1, {5}};
@@ -19,9 +21,9 @@ __host__ __device__ constexpr LevelPlan row_plan(int logl) {
         case 9: return LevelPlan{2, {4, 5}};
         case 10: return LevelPlan{3, {2, 3, 5}};
         case 11: return LevelPlan{3, {3, 3, 5}};
-        case 12: return LevelPlan{4, {2, 2, 3, 5}};
-        case 13: return LevelPlan{4, {2, 3, 3, 5}};
-        case 14: return LevelPlan{4, {3, 3, 3, 5}};
+        case 12: return LevelPlan{3, {3, 4, 5}};
+        case 13: return LevelPlan{3, {4, 4, 5}};
+        case 14: return LevelPlan{3, {4, 5, 5}};
         default: return LevelPlan{0, {0}};
     }
 }
@@ -153,18 +155,16 @@ __host__ __device__ constexpr int small_ppc(int logl) { return logl >= 12 ? 1 : 
 __host__ __device__ constexpr int small_ctas(int logl) { return logl <= 12 ? 6 : logl == 13 ? 3 : 1; }
 __host__ __device__ constexpr int row_threads(int logl) { return logl == 14 ? 1024 : small_threads(logl); }
 // Threads of the split row kernels (one operand row per CTA): one per
-// 32-word row of the last level, two CTAs per SM; 2^14-word rows use 256
-// threads (up to 85 registers each) and three CTAs per SM, so that the load,
-// compute and store phases of three rows overlap on every SM.
-__host__ __device__ constexpr int rowsplit_threads(int logl) { return logl == 14 ? 256 : logl >= 10 ? (1 << (logl - 5)) : 32; }
+// 32-word row of the last level.
+__host__ __device__ constexpr int rowsplit_threads(int logl) { return logl >= 10 ? (1 << (logl - 5)) : 32; }
 // Natural-order row transforms (k_row_ntt): one thread per 32-word group of
 // the last level (at least a warp), one row of shared memory per CTA, 1024
 // threads per SM.
 __host__ __device__ constexpr int ntt_row_threads(int logl) { return logl >= 10 ? (1 << (logl - 5)) : 32; }
 __host__ __device__ constexpr int ntt_row_ctas(int logl) { return 1024 / ntt_row_threads(logl) < 32 ? 1024 / ntt_row_threads(logl) : 32; }
 
-// Resident CTAs per SM the split row kernels are compiled for: three for
-// 2^14-word rows, else enough for 1024 threads per SM (64 registers).
-__host__ __device__ constexpr int rowsplit_ctas(int logl) { return logl == 14 ? 3 : (1024 / rowsplit_threads(logl) < 32 ? 1024 / rowsplit_threads(logl) : 32); }
+// Resident CTAs per SM the split row kernels are compiled for: 1024 threads
+// of 64 registers.
+__host__ __device__ constexpr int rowsplit_ctas(int logl) { return (1024 / rowsplit_threads(logl) < 32 ? 1024 / rowsplit_threads(logl) : 32); }
 
 }  // namespace cmb

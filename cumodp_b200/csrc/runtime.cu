@@ -66,7 +66,7 @@ Caches& caches() {
     return *c;
 }
 
-std::vector<Tw> build_level_tables(const LevelPlan& pl, int logl, u32 root, u32 p) {
+std::vector<Tw> build_level_tables(const LevelPlan& pl, int logl, u32 root, u32 p, bool slot_major) {
     const int nf = plan_tw_entries(pl, logl);
     std::vector<Tw> t((size_t)2 * nf + 2);
     const u32 rinv = powmod_exact(root, (1ull << logl) - 1, p);  // root^-1
@@ -78,8 +78,9 @@ std::vector<Tw> build_level_tables(const LevelPlan& pl, int logl, u32 root, u32 
         for (int o = 0; o < TB; ++o)
             for (int j = 0; j < R; ++j) {
                 u64 e = (u64)o * bitrev((u32)j, r);
-                t[off + o * R + j] = tw_of(powmod_exact(wb, e, p), p);
-                t[nf + off + o * R + j] = tw_of(powmod_exact(wbi, e, p), p);
+                const int at = off + (slot_major ? j * TB + o : o * R + j);
+                t[at] = tw_of(powmod_exact(wb, e, p), p);
+                t[nf + at] = tw_of(powmod_exact(wbi, e, p), p);
             }
         off += 1 << lb;
         lb -= r;
@@ -109,8 +110,9 @@ int level_tables_into(int kind, u32 p, u32 root, int logl, Tw* out, size_t cap) 
         for (int o = 0; o < TB; ++o)
             for (int j = 0; j < R; ++j) {
                 u64 e = (u64)o * bitrev((u32)j, r);
-                out[off + o * R + j] = tw_of(powmod_exact(wb, e, p), p);
-                out[nf + off + o * R + j] = tw_of(powmod_exact(wbi, e, p), p);
+                const int at = off + (kind == 0 ? j * TB + o : o * R + j);
+                out[at] = tw_of(powmod_exact(wb, e, p), p);
+                out[nf + at] = tw_of(powmod_exact(wbi, e, p), p);
             }
         off += 1 << lb;
         lb -= r;
@@ -376,7 +378,7 @@ static const Tw* level_tables(int dev, u32 p, u32 root, int logl, int kind, int*
     auto it = C.tables.find(key);
     if (it != C.tables.end()) return it->second;
     const LevelPlan pl = kind == 0 ? row_plan(logl) : col_plan(logl);
-    std::vector<Tw> t = build_level_tables(pl, logl, root, p);
+    std::vector<Tw> t = build_level_tables(pl, logl, root, p, kind == 0);
     Tw* d = nullptr;
     if (dev_malloc((void**)&d, t.size() * sizeof(Tw)) != cudaSuccess) {
         cudaGetLastError();

@@ -113,7 +113,7 @@ __device__ __forceinline__ void small_fwd_level(u32* sm, const Ctx& A) {
         dif_regs<R, true>(xf, A.pk.rc.f, p, p2);
         dif_regs<R, true>(xg, A.pk.rc.f, p, p2);
         Tw t[R];
-        load_tw<R>(t, A.tw + LV::TWOFF + o * R);
+        load_tw<R, TB>(t, A.tw + LV::TWOFF + o);
 #pragma unroll
         for (int j = 1; j < R; ++j) {
             xf[j] = mul_shoup(xf[j], t[j].w, t[j].wq, p);
@@ -144,7 +144,7 @@ __device__ __forceinline__ void small_inv_level(u32* sm, const Ctx& A) {
 #pragma unroll
         for (int m = 0; m < R; ++m) x[m] = sm[swz_task<TB, B>(base, bs, m)];
         Tw t[R];
-        load_tw<R>(t, A.tw + A.tw_inv_off + LV::TWOFF + o * R);
+        load_tw<R, TB>(t, A.tw + A.tw_inv_off + LV::TWOFF + o);
 #pragma unroll
         for (int j = 1; j < R; ++j) x[j] = mul_shoup(x[j], t[j].w, t[j].wq, p);
         dit_regs<R, true>(x, A.pk.rc.i, p, p2);
@@ -189,7 +189,7 @@ __device__ __forceinline__ void fwd1_level(u32* sm, const PrimeK& pk, const Tw* 
         for (int m = 0; m < R; ++m) x[m] = sm[swz_task<TB, B>(base, bs, m)];
         dif_regs<R, true>(x, pk.rc.f, p, p2);
         Tw t[R];
-        load_tw<R>(t, tw + LV::TWOFF + o * R);
+        load_tw<R, TB>(t, tw + LV::TWOFF + o);
 #pragma unroll
         for (int j = 1; j < R; ++j) x[j] = mul_shoup(x[j], t[j].w, t[j].wq, p);
 #pragma unroll
