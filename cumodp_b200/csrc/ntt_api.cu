@@ -24,170 +24,8 @@
 
 namespace cmb {
 
-struct RowNttArgs {
-    PrimeK pk;
-    const Tw* __restrict__ twr;
-    const u32* __restrict__ seeds;  // inter-pass twiddles w_n^(k1 c)
-    int nlo, nhi;
-    int l1;                         // rows come from a column pass of length 2^l1
-    LevelPlan colpl;
-    const u32* src;                 // row slot s at src + s * n2
-    u32* dst;                       // natural row k1 at dst + k1 * n2
-    Tw scale;                       // applied to every output (folded into level 0's input factors)
-    const Tw* __restrict__ rowtab;  // per-slot level-0 factor tables (RowTab, forward direction), or nullptr
-    long long job_stride;           // words between the transforms of grid row blockIdx.y (list transforms)
-};
-
 __device__ __forceinline__ u32 seed_mont_at(const u32* __restrict__ seeds, int nlo, u32 e, u32 p, u32 pinv) {
     return mul_mont(__ldg(seeds + (e & 4095u)), __ldg(seeds + nlo + (e >> 12)), p, pinv);
-}
-
-
-// One row of a four-step transform per CTA: the row (a column-pass output
-// row) is copied into shared memory with cp.async, level 0 applies the
-// inter-pass twiddle w_n^(k1 c), the remaining levels run as in the product kernels, and the
-// last level leaves each thread one 32-word group in registers; after a
-// barrier the groups are written back at their natural positions in the same
-// buffer, and the row is stored with 16-byte accesses.  With the prebuilt
-// per-slot factor tables (rows of 2^11-2^14 words) level 0 is that of the
-// product's row kernels: inputs times W^(TB0 m), DIF, outputs times the two
-// shared-memory factors of U_j^o.  The output scale (the inverse transform's
-// 2^-k) is folded into level 0's input factors, so a transform is linear in
-// it at no cost per word: the last level only reduces to [0, p).
-//
-// QOUT (rows of a four-step transform that a permuting transpose,
-// k_transpose64_q, puts in natural order): the in-row reorder is skipped and
-// each thread stores its last-level groups straight from registers in the
-// layout of the product's row spectra -- digit-reversed positions, quad c of
-// 32-word group r at c n2/8 + 4r, so a warp store covers one contiguous
-// 512-byte run -- with the split row kernels' CTA shape (256 threads, three
-// CTAs per SM for 2^14-word rows).
-template <int L2, bool QOUT = false>
-__global__ void __launch_bounds__(QOUT ? rowsplit_threads(L2) : ntt_row_threads(L2),
-                                  QOUT ? rowsplit_ctas(L2) : ntt_row_ctas(L2))
-    k_row_ntt(const __grid_constant__ RowNttArgs A) {
-    constexpr int n2 = 1 << L2;
-    constexpr int T = QOUT ? rowsplit_threads(L2) : ntt_row_threads(L2);
-    constexpr LevelPlan PL = row_plan(L2);
-    static_assert(PL.nlev >= 2, "row transform needs two levels");
-    static_assert(QOUT || T * 32 >= n2, "one last-level group per thread");
-    using LV0 = SmallLevel<L2, 0>;
-    constexpr int R0 = LV0::R, TB0 = LV0::TB;
-    extern __shared__ __align__(16) u32 sm[];
-    __shared__ Tw bf[R0];
-
-    const u32 s = blockIdx.x;
-    const u32 k1 = col_slot_to_k1(s, A.colpl, A.l1);
-    const u32 nmask = (1u << (A.l1 + L2)) - 1;
-    const u32 p = A.pk.p, p2 = A.pk.p2, pinv = A.pk.pinv_neg;
-    using RT = RowTab<L2>;
-    const bool tabbed = RT::USE && A.rowtab;
-    const bool scaled = A.scale.w != 1u;
-    Tw* tab = reinterpret_cast<Tw*>(sm + n2);
-    const size_t joff = (size_t)blockIdx.y * (size_t)A.job_stride;
-    row_load_issue<L2, T>(sm, A.src + joff + (size_t)s * n2);
-    if (tabbed) {
-        const Tw* src = A.rowtab + (size_t)s * RT::TABW;  // forward direction
-        for (int i = threadIdx.x; i < RT::TABW / 2; i += T) {
-            const unsigned d = (unsigned)__cvta_generic_to_shared(tab + 2 * i);
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src + 2 * i) : "memory");
-        }
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
-    } else if (threadIdx.x < R0) {
-        const u32 e = (k1 * (u32)TB0 * threadIdx.x) & nmask;
-        u32 v = red1(mul_mont(seed_mont_at(A.seeds, A.nlo, e, p, pinv), 1u, p, pinv), p);
-        if (scaled) v = mulmod_exact(v, A.scale.w, p);
-        bf[threadIdx.x] = Tw{v, shoup_quot(v, p)};
-    }
-    row_load_wait();
-    __syncthreads();
-    if (tabbed && scaled) {  // the slot factors times the scale (factor 0 becomes the scale)
-        if (threadIdx.x < R0) {
-            Tw* vf = tab + RT::ENTRIES;
-            const u32 v = threadIdx.x == 0 ? A.scale.w : mulmod_exact(vf[threadIdx.x].w, A.scale.w, p);
-            vf[threadIdx.x] = Tw{v, shoup_quot(v, p)};
-        }
-        __syncthreads();
-    }
-
-    if constexpr (RT::USE) {
-        if (tabbed) {
-            const Tw* vf = tab + RT::ENTRIES;
-            for (int o = threadIdx.x; o < TB0; o += T) {
-                u32 x[R0];
-                const int bs = swz(o);
-#pragma unroll
-                for (int m = 0; m < R0; ++m) {
-                    const u32 v = sm[swz_task<TB0, n2>(o, bs, m)];
-                    x[m] = m == 0 && !scaled ? v : mul_shoup(v, vf[m].w, vf[m].wq, p);
-                }
-                dif_regs<R0, true>(x, A.pk.rc.f, p, p2);
-                const Tw* ta = tab + (o % RT::NA);
-                const Tw* tb = tab + RT::R0 * RT::NA + o / RT::NA;
-#pragma unroll
-                for (int j = 0; j < R0; ++j) {
-                    const Tw a = ta[j * RT::NA], b = tb[j * RT::NB];
-                    x[j] = mul_shoup(mul_shoup(x[j], a.w, a.wq, p), b.w, b.wq, p);
-                }
-#pragma unroll
-                for (int m = 0; m < R0; ++m) sm[swz_task<TB0, n2>(o, bs, m)] = x[m];
-            }
-        }
-    }
-    for (int o = threadIdx.x; o < (tabbed ? 0 : TB0); o += T) {
-        u32 x[R0];
-        const u32 mo = seed_mont_at(A.seeds, A.nlo, (k1 * (u32)o) & nmask, p, pinv);
-        const int bs = swz(o);
-#pragma unroll
-        for (int m = 0; m < R0; ++m) {
-            const u32 v = sm[swz_task<TB0, n2>(o, bs, m)];
-            x[m] = mul_mont(v, mul_shoup(mo, bf[m].w, bf[m].wq, p), p, pinv);
-        }
-        dif_regs<R0, true>(x, A.pk.rc.f, p, p2);
-        Tw t[R0];
-        load_tw<R0, TB0>(t, A.twr + o);
-#pragma unroll
-        for (int j = 1; j < R0; ++j) x[j] = mul_shoup(x[j], t[j].w, t[j].wq, p);
-#pragma unroll
-        for (int m = 0; m < R0; ++m) sm[swz_task<TB0, n2>(o, bs, m)] = x[m];
-    }
-    __syncthreads();
-    fwd1_levels<L2, 1, T>(sm, A.pk, A.twr);
-
-    if constexpr (QOUT) {
-        u32* out = A.dst + joff + (size_t)k1 * n2;
-        for (int r = threadIdx.x; r < n2 / 32; r += T) {
-            u32 x[32];
-            load_row32(x, sm, r * 32);
-            dif_regs<32>(x, A.pk.rc.f, p, p2);
-#pragma unroll
-            for (int c = 0; c < 8; ++c)
-                *reinterpret_cast<uint4*>(out + c * (n2 / 8) + 4 * r) =
-                    make_uint4(red1(x[4 * c], p), red1(x[4 * c + 1], p), red1(x[4 * c + 2], p), red1(x[4 * c + 3], p));
-        }
-        return;
-    }
-    const int r = threadIdx.x;
-    const bool has = r < n2 / 32;
-    u32 x[32];
-    if (has) {
-        load_row32(x, sm, r * 32);
-        dif_regs<32>(x, A.pk.rc.f, p, p2);
-#pragma unroll
-        for (int j = 0; j < 32; ++j) x[j] = red1(x[j], p);
-    }
-    __syncthreads();
-    // natural order through shared memory (swz_nat layout: the reorder's
-    // stores are conflict-free), read out word by word, consecutive lanes on
-    // consecutive words
-    if (has) {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) sm[swz_nat((int)row_pos_to_freq<L2>((u32)(r * 32 + j)))] = x[j];
-    }
-    __syncthreads();
-    u32* out = A.dst + joff + (size_t)k1 * n2;
-#pragma unroll 4
-    for (int i = threadIdx.x; i < n2; i += T) out[i] = sm[swz_nat(i)];
 }
 
 // out[c * rows + r] = in[r * cols + c] for rows and cols multiples of 64:
@@ -217,43 +55,6 @@ __global__ void __launch_bounds__(256) k_transpose64(const u32* __restrict__ in,
         const int cc = ty + 16 * k;
         const uint4 v = make_uint4(t[4 * tx][cc], t[4 * tx + 1][cc], t[4 * tx + 2][cc], t[4 * tx + 3][cc]);
         *reinterpret_cast<uint4*>(dst + (size_t)cc * rows) = v;
-    }
-}
-
-// out[f(c) * rows + r] = in[r * n2 + c] for rows a multiple of 64, where row
-// r of `in` is a row spectrum in the layout k_row_ntt<L2, true> stores and
-// f(c) is the frequency word c holds: word c = q n2/8 + 4 g + e (e < 4,
-// g < n2/32) holds digit-reversed position P = 32 g + 4 q + e, whose
-// frequency is row_pos_to_freq<L2>(P).  64 x 64 tiles through shared
-// memory, 16-byte loads and stores (each of a tile's 64 words is one
-// frequency, whose 64 rows are one 256-byte run of the output).
-template <int L2>
-__global__ void __launch_bounds__(256) k_transpose64_q(const u32* __restrict__ in, u32* __restrict__ out, int rows) {
-    constexpr int n2 = 1 << L2;
-    __shared__ u32 t[64][65];
-    in += (size_t)blockIdx.z * rows * n2;  // transform blockIdx.z of a list
-    out += (size_t)blockIdx.z * rows * n2;
-    const int c0 = blockIdx.x * 64;
-    const size_t r0 = (size_t)blockIdx.y * 64;
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const u32* src = in + r0 * n2 + c0 + 4 * tx;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const int rr = ty + 16 * k;
-        const uint4 v = __ldg(reinterpret_cast<const uint4*>(src + (size_t)rr * n2));
-        t[rr][4 * tx] = v.x;
-        t[rr][4 * tx + 1] = v.y;
-        t[rr][4 * tx + 2] = v.z;
-        t[rr][4 * tx + 3] = v.w;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const int cc = ty + 16 * k;
-        const u32 c = (u32)(c0 + cc), q = c / (n2 / 8), g = (c % (n2 / 8)) / 4, e = c % 4;
-        const u32 f = row_pos_to_freq<L2>(32 * g + 4 * q + e);
-        const uint4 v = make_uint4(t[4 * tx][cc], t[4 * tx + 1][cc], t[4 * tx + 2][cc], t[4 * tx + 3][cc]);
-        *reinterpret_cast<uint4*>(out + (size_t)f * rows + r0 + 4 * tx) = v;
     }
 }
 
@@ -289,59 +90,28 @@ __global__ void k_tiny_dft(const u32* __restrict__ x, u32* __restrict__ y, int n
 
 namespace {
 
-template <int L2>
-void launch_row_ntt_t(const RowNttArgs& a, int rows, cudaStream_t st, int jobs) {
-    const size_t smem = (size_t)(1 << L2) * sizeof(u32) + (size_t)RowTab<L2>::TABW * sizeof(Tw);
-    static bool attr = false;
-    if (!attr) {
-        cudaFuncSetAttribute(k_row_ntt<L2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        attr = true;
-    }
-    k_row_ntt<L2><<<dim3(rows, jobs), ntt_row_threads(L2), smem, st>>>(a);
-}
-
-// The rows of a four-step transform with 2^14-word rows and at least 64 of
-// them: k_row_ntt<14, true> then the permuting transpose into x_out (jobs
-// transforms of rows x 2^14 words, w2 and x_out job_stride words apart).
-void row_ntt_q_and_transpose(const RowNttArgs& a, int rows, u32* x_out, cudaStream_t st, int jobs) {
-    constexpr int L2 = kMaxRowLog;
-    const size_t smem = (size_t)(1 << L2) * sizeof(u32) + (size_t)RowTab<L2>::TABW * sizeof(Tw);
-    static bool attr = false;
-    if (!attr) {
-        cudaFuncSetAttribute(k_row_ntt<L2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        attr = true;
-    }
-    cudaEvent_t e0;
-    bool tr = pass_timing_begin(st, &e0);
-    k_row_ntt<L2, true><<<dim3(rows, jobs), rowsplit_threads(L2), smem, st>>>(a);
-    if (tr) pass_timing_end(st, "ntt_row", e0);
-    tr = pass_timing_begin(st, &e0);
-    k_transpose64_q<L2><<<dim3((1 << L2) / 64, rows / 64, jobs), 256, 0, st>>>(a.dst, x_out, rows);
-    if (tr) pass_timing_end(st, "ntt_transpose", e0);
-}
-typedef void (*RowNttFn)(const RowNttArgs&, int, cudaStream_t, int);
-const RowNttFn kRowNtt[15] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
-                              nullptr, nullptr, nullptr, nullptr, launch_row_ntt_t<10>, launch_row_ntt_t<11>,
-                              launch_row_ntt_t<12>, launch_row_ntt_t<13>, launch_row_ntt_t<14>};
-
 // `rows` independent natural-order row transforms of 2^k words, 6 <= k <= 14
 // (root: the transform's own, scale applied to every output): src row s to
 // dst row s, or to row k1(s) when the rows are slots of a column pass of 2^l1.
-template <int L2>
-void launch_row_nat_t(const RowNatArgs& a, cudaStream_t st) {
+template <int L2, bool SLOT>
+void launch_row_nat_t(const RowNatArgs& a, int jobs, cudaStream_t st) {
     static const bool attr = [] {
-        cudaFuncSetAttribute(k_row_nat<L2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)nat_smem(L2));
+        cudaFuncSetAttribute(k_row_nat<L2, SLOT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)nat_smem(L2));
         return true;
     }();
     (void)attr;
     const u32 grid = (u32)(((u64)a.rows + nat_rows(L2) - 1) / nat_rows(L2));
-    k_row_nat<L2><<<grid, nat_threads(L2), nat_smem(L2), st>>>(a);
+    k_row_nat<L2, SLOT><<<dim3(grid, jobs), nat_threads(L2), nat_smem(L2), st>>>(a);
 }
-typedef void (*RowNatFn)(const RowNatArgs&, cudaStream_t);
+typedef void (*RowNatFn)(const RowNatArgs&, int, cudaStream_t);
 const RowNatFn kRowNat[15] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
-                              launch_row_nat_t<6>, launch_row_nat_t<7>, launch_row_nat_t<8>,
-                              launch_row_nat_t<9>, launch_row_nat_t<10>, launch_row_nat_t<11>,
-                              launch_row_nat_t<12>, launch_row_nat_t<13>, launch_row_nat_t<14>};
+                              launch_row_nat_t<6, false>, launch_row_nat_t<7, false>, launch_row_nat_t<8, false>,
+                              launch_row_nat_t<9, false>, launch_row_nat_t<10, false>, launch_row_nat_t<11, false>,
+                              launch_row_nat_t<12, false>, launch_row_nat_t<13, false>, launch_row_nat_t<14, false>};
+// rows of a four-step transform (2^10 words and more)
+const RowNatFn kRowSlot[15] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
+                               launch_row_nat_t<10, true>, launch_row_nat_t<11, true>, launch_row_nat_t<12, true>,
+                               launch_row_nat_t<13, true>, launch_row_nat_t<14, true>};
 
 int row_nat(const PrimeCtx& pc, const u32* src, u32* dst, long long rows, int k, u32 root, u32 scale, int l1, int dev,
             cudaStream_t st) {
@@ -360,9 +130,42 @@ int row_nat(const PrimeCtx& pc, const u32* src, u32* dst, long long rows, int k,
         A.src = src + (r0 << k);
         A.dst = dst + (r0 << k);
         A.rows = (u32)std::min<long long>(1ll << 30, rows - r0);
-        kRowNat[k](A, st);
+        kRowNat[k](A, 1, st);
     }
     if (tr) pass_timing_end(st, "ntt_row", e0);
+    return cuda_err(cudaGetLastError());
+}
+
+// The rows of four-step transforms of 2^(l1 + l2) words with root `root`, and
+// the transpose that follows: job t's rows (column-pass slots) at w1 + t n, its
+// rows k1 in natural order at w2 + t n, its result at out + t n.
+int rows_and_transpose(const PrimeCtx& pc, const u32* w1, u32* w2, u32* out, int l1, int l2, u32 root, u32 scale,
+                       int jobs, int dev, cudaStream_t st) {
+    int err = OK;
+    const u32 p = pc.info.p, root_r = powmod_exact(root, 1ull << l1, p);
+    RowNatArgs A;
+    memset(&A, 0, sizeof(A));
+    A.tw = nat_tables(dev, p, root_r, l2, scale, &err);
+    A.slot = nat_slot_tables(dev, p, root, l1, l2, &err);
+    if (!A.tw || !A.slot) return err;
+    A.pk = make_prime_k_for(pc.info, root_r, l2);
+    A.scaled = scale != 1u;
+    A.l1 = l1;
+    A.colpl = col_plan(l1);
+    A.src = w1;
+    A.dst = w2;
+    A.rows = 1u << l1;
+    A.job_stride = 1ll << (l1 + l2);
+    cudaEvent_t e0;
+    bool tr = pass_timing_begin(st, &e0);
+    kRowSlot[l2](A, jobs, st);
+    if (tr) pass_timing_end(st, "ntt_row", e0);
+    tr = pass_timing_begin(st, &e0);
+    if (l1 >= 6)
+        k_transpose64<<<dim3((1 << l2) / 64, (1 << l1) / 64, jobs), 256, 0, st>>>(w2, out, 1 << l1, 1 << l2);
+    else
+        k_transpose<<<dim3((1 << l2) / 32, (1 << l1) / 32, jobs), dim3(32, 8), 0, st>>>(w2, out, 1 << l1, 1 << l2);
+    if (tr) pass_timing_end(st, "ntt_transpose", e0);
     return cuda_err(cudaGetLastError());
 }
 
@@ -520,44 +323,12 @@ int ntt_natural_dev(const u32* x_in, u32* x_out, int k, u32 w, u32 p, bool inver
     u32* ws = (u32*)workspace(dev, kWsNtt, (size_t)2 * n * sizeof(u32), &err);
     if (!ws) return err;
     u32 *w1 = ws, *w2 = ws + n;
-    const u32 root_c = powmod_exact(root, 1ull << l2, p), root_r = powmod_exact(root, 1ull << l1, p);
+    const u32 root_c = powmod_exact(root, 1ull << l2, p);
     cudaEvent_t e0;
-    bool tr = pass_timing_begin(st, &e0);
+    const bool tr = pass_timing_begin(st, &e0);
     if ((err = column_pass(*pc, root_c, l1, l2, x_in, n, w1, dev, st)) != OK) return err;
     if (tr) pass_timing_end(st, "ntt_col", e0);
-    RowNttArgs A;
-    memset(&A, 0, sizeof(A));
-    const Tw* twr = row_tables(dev, p, root_r, l2, &err);
-    const u32* seeds = seed_tables(dev, p, root, k, &err);
-    if (!twr || !seeds) return err ? err : OUT_OF_MEMORY;
-    A.pk = make_prime_k_for(pc->info, root_r, l2);
-    A.twr = twr;
-    A.seeds = seeds;
-    A.nlo = (int)std::min<long long>(n, 4096);
-    A.nhi = (int)std::max<long long>(1, n / 4096);
-    A.l1 = l1;
-    A.colpl = col_plan(l1);
-    A.src = w1;
-    A.dst = w2;
-    A.scale = tw_of(sc, p);
-    {
-        LargeArgs LA;  // the level-0 factor tables of this root and shape (built once, cached)
-        if (large_args(*pc, root, k, l2, dev, &LA) == OK) A.rowtab = LA.rowtab;
-    }
-    if (l1 >= 6 && l2 == kMaxRowLog) {
-        row_ntt_q_and_transpose(A, 1 << l1, x_out, st, 1);
-        return cuda_err(cudaGetLastError());
-    }
-    tr = pass_timing_begin(st, &e0);
-    kRowNtt[l2](A, 1 << l1, st, 1);
-    if (tr) pass_timing_end(st, "ntt_row", e0);
-    tr = pass_timing_begin(st, &e0);
-    if (l1 >= 6)
-        k_transpose64<<<dim3((1 << l2) / 64, (1 << l1) / 64), 256, 0, st>>>(w2, x_out, 1 << l1, 1 << l2);
-    else
-        k_transpose<<<dim3((1 << l2) / 32, (1 << l1) / 32), dim3(32, 8), 0, st>>>(w2, x_out, 1 << l1, 1 << l2);
-    if (tr) pass_timing_end(st, "ntt_transpose", e0);
-    return cuda_err(cudaGetLastError());
+    return rows_and_transpose(*pc, w1, w2, x_out, l1, l2, root, sc, 1, dev, st);
 }
 
 namespace {
@@ -579,27 +350,7 @@ int list_ntt_four_step(const PrimeCtx& pc, u32* x, long long m, int k, u32 root,
     LargeJob* dj = (LargeJob*)workspace(dev, kWsListJobs, (size_t)cm * sizeof(LargeJob), &err);
     if (!dj) return err;
     u32 *w1 = ws, *w2 = ws + cm * n;
-    const u32 root_c = powmod_exact(root, 1ull << l2, p), root_r = powmod_exact(root, 1ull << l1, p);
-    RowNttArgs A;
-    memset(&A, 0, sizeof(A));
-    const Tw* twr = row_tables(dev, p, root_r, l2, &err);
-    const u32* seeds = seed_tables(dev, p, root, k, &err);
-    if (!twr || !seeds) return err ? err : OUT_OF_MEMORY;
-    A.pk = make_prime_k_for(pc.info, root_r, l2);
-    A.twr = twr;
-    A.seeds = seeds;
-    A.nlo = (int)std::min<long long>(n, 4096);
-    A.nhi = (int)std::max<long long>(1, n / 4096);
-    A.l1 = l1;
-    A.colpl = col_plan(l1);
-    A.src = w1;
-    A.dst = w2;
-    A.scale = tw_of(sc, p);
-    A.job_stride = n;
-    {
-        LargeArgs LA;
-        if (large_args(pc, root, k, l2, dev, &LA) == OK) A.rowtab = LA.rowtab;
-    }
+    const u32 root_c = powmod_exact(root, 1ull << l2, p);
     std::vector<LargeJob> hj((size_t)cm);
     for (long long r0 = 0; r0 < m; r0 += cm) {
         const int cnt = (int)std::min(cm, m - r0);
@@ -609,17 +360,7 @@ int list_ntt_four_step(const PrimeCtx& pc, u32* x, long long m, int k, u32 root,
         cudaError_t e = cudaMemcpyAsync(dj, hj.data(), (size_t)cnt * sizeof(LargeJob), cudaMemcpyHostToDevice, st);
         if (e != cudaSuccess) return cuda_err(e);
         if ((err = column_pass(pc, root_c, l1, l2, nullptr, n, nullptr, dev, st, dj, cnt)) != OK) return err;
-        u32* out = x + r0 * n;
-        if (l1 >= 6 && l2 == kMaxRowLog) {
-            row_ntt_q_and_transpose(A, 1 << l1, out, st, cnt);
-            continue;
-        }
-        kRowNtt[l2](A, 1 << l1, st, cnt);
-        if (l1 >= 6)
-            k_transpose64<<<dim3((1 << l2) / 64, (1 << l1) / 64, cnt), 256, 0, st>>>(w2, out, 1 << l1, 1 << l2);
-        else
-            k_transpose<<<dim3((1 << l2) / 32, (1 << l1) / 32, cnt), dim3(32, 8), 0, st>>>(w2, out, 1 << l1,
-                                                                                          1 << l2);
+        if ((err = rows_and_transpose(pc, w1, w2, x + r0 * n, l1, l2, root, sc, cnt, dev, st)) != OK) return err;
     }
     return cuda_err(cudaGetLastError());
 }

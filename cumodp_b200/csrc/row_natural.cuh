@@ -1,4 +1,5 @@
-// Natural-order transforms of independent rows of 2^6 .. 2^14 words.
+// Natural-order transforms of rows of 2^6 .. 2^14 words: independent ones, and
+// those of a four-step transform.
 //
 // A row takes two or three levels of radix 8..32, the fewest that fit a
 // thread's registers: level 0 reads its words straight from global memory (task
@@ -9,7 +10,7 @@
 // level's task (k0, k1) holds frequencies k0 + R0 k1 + R0 R1 k2: consecutive
 // tasks are consecutive words, and natural order costs no pass.
 // Bound by integer issue: two exchanges and one Shoup product per word and
-// level boundary where k_row_ntt ran four levels, a copy into shared memory
+// level boundary where the previous kernel ran four levels, a copy into shared memory
 // before them and a reorder through it after them.  Measured on B200, 2^25
 // words of rows, before -> after:
 //   2^6   390 -> 54 us    2^9   115 -> 70 us    2^12  109 -> 70 us
@@ -67,11 +68,19 @@ struct RowNatArgs {
     int scaled;                 // level 0's k0 = 0 twiddles are not 1
     int l1;                     // > 0: rows are slots of a column pass of 2^l1, out(s) = its frequency
     LevelPlan colpl;
+    const Tw* __restrict__ slot;  // SLOT: slot s's nat_slot_entries from s times that on
+    long long job_stride;         // words between the transforms of grid row blockIdx.y
 };
+// Rows of a four-step transform (SLOT): word c of slot s is multiplied by the
+// inter-pass twiddle W^c, W = w^k1(s).  Task o's words are c = o + TB m, so
+// W^c = W^(TB m) W^o: the first is one of R0 factors of the slot, on the way
+// in; the second is the task's own and commutes with the DFT.  Per slot: W^(TB
+// m) for m < R0, then W^o for every task.
+__host__ __device__ constexpr int nat_slot_entries(int logl) { return (1 << nat_plan(logl).logr[0]) + nat_row_threads(logl); }
 
 #ifdef __CUDACC__
 
-template <int L2>
+template <int L2, bool SLOT>
 __global__ void __launch_bounds__(nat_threads(L2), nat_ctas(L2)) k_row_nat(const __grid_constant__ RowNatArgs A) {
     constexpr LevelPlan PL = nat_plan(L2);
     constexpr bool THREE = PL.nlev == 3;
@@ -87,11 +96,23 @@ __global__ void __launch_bounds__(nat_threads(L2), nat_ctas(L2)) k_row_nat(const
     const u32 p = A.pk.p, p2 = A.pk.p2;
     {
         u32 x[R0];
-        const u32* src = A.src + (size_t)(has ? s : 0) * n + t;
+        const size_t job = SLOT ? blockIdx.y * (size_t)A.job_stride : 0;
+        const u32* src = A.src + job + (size_t)(has ? s : 0) * n + t;
 #pragma unroll
         for (int m = 0; m < R0; ++m) x[m] = src[TB0 * m];  // (may be the rows written below)
+        uint2 wo = make_uint2(1u, 0u);
+        if constexpr (SLOT) {  // a column pass's words, below 2p
+            const uint2* f = reinterpret_cast<const uint2*>(A.slot + (size_t)(has ? s : 0) * nat_slot_entries(L2));
+            wo = __ldg(f + R0 + t);
 #pragma unroll
-        for (int m = 0; m < R0; ++m) x[m] = mul_shoup(x[m], 1u, A.pk.one_q, p);
+            for (int m = 1; m < R0; ++m) {
+                const uint2 w = __ldg(f + m);
+                x[m] = mul_shoup(x[m], w.x, w.y, p);
+            }
+        } else {
+#pragma unroll
+            for (int m = 0; m < R0; ++m) x[m] = mul_shoup(x[m], 1u, A.pk.one_q, p);
+        }
         dif_regs<R0, true>(x, A.pk.rc.f, p, p2);
         const Tw* tw = A.tw + t;
 #pragma unroll
@@ -101,6 +122,7 @@ __global__ void __launch_bounds__(nat_threads(L2), nat_ctas(L2)) k_row_nat(const
                 const uint2 w = __ldg(reinterpret_cast<const uint2*>(tw + TB0 * k));
                 x[j] = mul_shoup(x[j], w.x, w.y, p);
             }
+            if constexpr (SLOT) x[j] = mul_shoup(x[j], wo.x, wo.y, p);
             sm[S * k + t] = x[j];
         }
     }
@@ -128,7 +150,7 @@ __global__ void __launch_bounds__(nat_threads(L2), nat_ctas(L2)) k_row_nat(const
     }
     if (!has) return;
     const u32 row = A.l1 ? col_slot_to_k1(s, A.colpl, A.l1) : s;
-    u32* out = A.dst + (size_t)row * n;
+    u32* out = A.dst + (SLOT ? blockIdx.y * (size_t)A.job_stride : 0) + (size_t)row * n;
     for (int id = t; id < n / RL; id += TPR) {
         const u32* b = sm + S * (id % R0) + RL * (id / R0);
         u32 x[RL];

@@ -371,6 +371,31 @@ const Tw* nat_tables(int dev, u32 p, u32 root, int logl, u32 scale, int* err) {
     return keep_table(C, key, t, err);
 }
 
+const Tw* nat_slot_tables(int dev, u32 p, u32 w, int l1, int l2, int* err) {
+    Caches& C = caches();
+    std::lock_guard<std::mutex> g(C.m);
+    auto key = std::make_tuple(dev, p, w, l1 * 64 + l2, 4);
+    auto it = C.tables.find(key);
+    if (it != C.tables.end()) return it->second;
+    const LevelPlan pl = col_plan(l1);
+    const int r0 = 1 << nat_plan(l2).logr[0], tb = nat_row_threads(l2);
+    std::vector<Tw> t;
+    t.reserve((size_t)nat_slot_entries(l2) << l1);
+    auto powers = [&](u32 b, int count) {
+        u32 v = 1;
+        for (int i = 0; i < count; ++i) {
+            t.push_back(tw_of(v, p));
+            v = mulmod_exact(v, b, p);
+        }
+    };
+    for (u32 s = 0; s < 1u << l1; ++s) {
+        const u32 W = powmod_exact(w, col_slot_to_k1(s, pl, l1), p);
+        powers(powmod_exact(W, tb, p), r0);
+        powers(W, tb);
+    }
+    return keep_table(C, key, t, err);
+}
+
 static const Tw* level_tables(int dev, u32 p, u32 root, int logl, int kind, int* err) {
     Caches& C = caches();
     std::lock_guard<std::mutex> g(C.m);

@@ -66,6 +66,9 @@ const Tw* grid_lead_tables(int dev, u32 p, u32 wm, int em, int en, int l1, u32 s
 // Twiddles of the natural-order row kernel (row_natural.cuh) for rows of
 // 2^logl words with the primitive 2^logl-th root `root`, outputs times `scale`.
 const Tw* nat_tables(int dev, u32 p, u32 root, int logl, u32 scale, int* err);
+// A four-step transform's slot factors (row_natural.cuh, SLOT): 2^l1 slots of
+// rows of 2^l2 words, w the transform's primitive 2^(l1 + l2)-th root.
+const Tw* nat_slot_tables(int dev, u32 p, u32 w, int l1, int l2, int* err);
 // Inter-pass twiddle seeds for a two-pass transform of length 2^logn:
 // lo[e] = w^e (e < 2^12) and hi[e] = w^(e << 12) (e < 2^(logn-12)), both in
 // Montgomery form times R (w^e * 2^64 mod p) so that one Montgomery product
