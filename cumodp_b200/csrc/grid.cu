@@ -57,7 +57,7 @@ const RowsFn kRows[3][kMaxRowLog + 1] = {
 
 bool grid_split(int em, int en, int* l1, int* e) {
     if (em < 1 || en < kMinRowLog || em + en < 11) return false;
-    // columns of 2^10 rows (pipelined kernels) first, then of 2^11
+    // columns of 2^10 rows (the register kernels) first, then of 2^11
     for (const int c : {(int)kDefaultColLog, (int)kMaxColLog}) {
         *e = em > c ? em - c : 0;
         *l1 = em - *e;

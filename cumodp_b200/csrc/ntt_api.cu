@@ -8,12 +8,11 @@
 // (DFT_m (x) I_n)(I_m (x) DFT_n) of a row-major 2^em x 2^en array.
 //
 // Here a transform of length <= 2^14 is one CTA's row (k_row_nat, natural
-// order for free).  Longer 1-D transforms use the
-// four-step split of the product path: a column pass (k_col_fwd), a row
-// pass that applies w_n^(k1*c), transforms the row and writes it back in
-// natural order as row k1, and a tiled transpose.  The 2-D transform is the
-// column pass plus the row pass with no inter-pass twiddle: its rows land
-// directly in natural order.
+// order for free).  Longer 1-D transforms use the four-step split of the
+// product path: a column pass (k_cold_fwd), the row pass (k_row_nat, SLOT),
+// which applies w_n^(k1*c) and writes slot s as row k1(s) in natural order,
+// and a tiled transpose.  The 2-D transform is the column pass plus the row
+// pass with no inter-pass twiddle: its rows land directly in natural order.
 #include <algorithm>
 #include <cstring>
 #include <vector>
@@ -529,9 +528,14 @@ int bivariate_mul_dev(u32* F, u32* G, int em, int en, u32 p, cudaStream_t st) {
     const long long m = 1ll << em, n = 1ll << en, total = m * n;
     const u32 wm = em ? canonical_root(*pc, em) : 1u, wn = en ? canonical_root(*pc, en) : 1u;
     int l1, e;
-    if (grid_split(em, en, &l1, &e)) return grid_mul_dev(F, G, em, en, p, st);
+    if (grid_split(em, en, &l1, &e)) {
+        // needs two grids of workspace; without them the paths below, which
+        // leave the operands as they are until their own workspace is there
+        err = grid_mul_dev(F, G, em, en, p, st);
+        if (err != OUT_OF_MEMORY) return err;
+    }
     if (en >= 6 && en <= kMaxRowLog && em <= kMaxColLog) {
-        // one row, or a grid of less than 2^11 words
+        // one row, a grid of less than 2^11 words, or no room for two grids
         if ((err = bivariate_dev(F, em, wm, en, wn, p, false, st)) != OK) return err;
         if ((err = bivariate_dev(G, em, wm, en, wn, p, false, st)) != OK) return err;
         k_pointwise_mod<<<grid_for(total), 256, 0, st>>>(F, G, total, p, pc->info.pinv_neg, pc->info.r2);

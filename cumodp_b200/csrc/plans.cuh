@@ -56,19 +56,15 @@ __host__ __device__ constexpr int col_tw_entries(int logl) {
     for (int i = 0; i + 1 < pl.nlev; ++i) { n += 1 << lb; lb -= pl.logr[i]; }
     return n;
 }
-// Column tiles: col_tile_cols adjacent columns x 2^logl rows in shared
-// memory, processed by col_warps warps, col_ctas resident CTAs per SM, each
-// chosen per kind of pass (0: the product's forward pass, whose operands are
-// half zero padding; 1: the inverse pass; 2: the forward pass of a
-// natural-order transform).  32-column tiles put
-// one column on each lane; 16-column tiles put two tasks on each warp (one
-// per half-warp) and insert a 16-word pad after every 2^col_pad_log rows (the
-// plan's last radix), so that the two half-warps always read opposite halves
-// of the banks.  Short tiles (2^5, 2^6 rows: the column side of products of
-// 2^15-2^17) run on one or two warps, so many CTAs share an SM.  Kinds 1 and
-// 2 over 2^10-row tiles use 16 columns and two
-// CTAs per SM (their load, compute and store phases overlap); kind 0 keeps
-// 32 columns (its loads skip the zero-padded half).
+// Column tiles in shared memory (k_col_fwd, k_col_inv: 2^11-row columns;
+// shorter ones are col_direct.cuh's): col_tile_cols adjacent columns x 2^logl
+// rows, processed by col_warps warps, col_ctas resident CTAs per SM, per kind
+// of pass (0: the product's forward pass, 1: the inverse pass, 2: the forward
+// pass of a natural-order transform).  32-column tiles put one column on each
+// lane; 16-column tiles put two tasks on each warp (one per half-warp) and
+// insert a 16-word pad after every 2^col_pad_log rows (the plan's last
+// radix), so that the two half-warps always read opposite halves of the
+// banks.
 __host__ __device__ constexpr int col_tile_cols(int logl, int kind) { return (kind != 0 && logl == 10) || logl >= 11 ? 16 : 32; }
 __host__ __device__ constexpr int col_warps(int logl, int kind) { return logl == 10 && kind == 0 ? 32 : (logl <= 5 ? 1 : (logl <= 6 ? 2 : 16)); }
 __host__ __device__ constexpr int col_ctas(int logl, int kind) { return kind != 0 && logl == 10 ? 2 : 1; }
@@ -81,32 +77,15 @@ __host__ __device__ constexpr int col_tile_words(int logl, int kind) {
 // Whether a column CTA stages its twiddles in shared memory next to the
 // tile (else the levels read them from global memory, as broadcasts).
 __host__ __device__ constexpr bool col_tw_smem(int logl, int kind) { return true; }
-// col_tile_cols for a run-time logl.
-__host__ __device__ inline int col_tile_cols_rt(int logl, int kind) {
-    constexpr int t[3][13] = {
-        {col_tile_cols(0, 0), col_tile_cols(1, 0), col_tile_cols(2, 0), col_tile_cols(3, 0), col_tile_cols(4, 0),
-         col_tile_cols(5, 0), col_tile_cols(6, 0), col_tile_cols(7, 0), col_tile_cols(8, 0), col_tile_cols(9, 0),
-         col_tile_cols(10, 0), col_tile_cols(11, 0), col_tile_cols(12, 0)},
-        {col_tile_cols(0, 1), col_tile_cols(1, 1), col_tile_cols(2, 1), col_tile_cols(3, 1), col_tile_cols(4, 1),
-         col_tile_cols(5, 1), col_tile_cols(6, 1), col_tile_cols(7, 1), col_tile_cols(8, 1), col_tile_cols(9, 1),
-         col_tile_cols(10, 1), col_tile_cols(11, 1), col_tile_cols(12, 1)},
-        {col_tile_cols(0, 2), col_tile_cols(1, 2), col_tile_cols(2, 2), col_tile_cols(3, 2), col_tile_cols(4, 2),
-         col_tile_cols(5, 2), col_tile_cols(6, 2), col_tile_cols(7, 2), col_tile_cols(8, 2), col_tile_cols(9, 2),
-         col_tile_cols(10, 2), col_tile_cols(11, 2), col_tile_cols(12, 2)}};
-    return t[kind][logl];
-}
 // Dynamic shared memory of a column CTA: the tile and its twiddles.
 __host__ __device__ constexpr int col_smem_bytes(int logl, int kind) {
     return col_tile_words(logl, kind) * 4 + (col_tw_smem(logl, kind) ? col_tw_entries(logl) * 8 : 0);
 }
 
-// Persistent pass A (k_col_fwd_pipe) for the two-level column plans, up to
-// 128 registers a thread (1024 threads at 64 registers spill): 2^10-row
-// columns in 16-column tiles (the layout of kind 2), two 256-thread CTAs per
-// SM, whose barriers and phases then overlap (measured 8 % faster than one
-// 512-thread CTA on 32-column tiles); 2^9-row columns in 32-column tiles,
-// one 512-thread CTA per SM (two per SM measured slower).  Shared memory:
-// the tile, a stage of its first n1/2 rows and the level-0 twiddles.
+// Shared-memory layouts of staged column passes for 2^9- and 2^10-row columns
+// (a tile, a stage of its first n1/2 rows and the level-0 twiddles); the
+// passes run from registers now (col_direct.cuh), the layouts are what
+// tests/index_maps_check.cu checks the tile maps with.
 __host__ __device__ constexpr bool col_pipe_ok(int logl) { return logl == 9 || logl == 10; }
 __host__ __device__ constexpr int col_pipe_kind(int logl) { return logl == 10 ? 2 : 0; }  // tile layout (col_tile_cols)
 __host__ __device__ constexpr int col_pipe_warps(int logl) { return logl == 10 ? 8 : 16; }
@@ -120,18 +99,12 @@ __host__ __device__ constexpr int col_pipe_smem_bytes(int logl) {
            (1 << logl) * 8;
 }
 
-// Persistent pass C (k_col_inv_pipe) for the same column lengths: one
-// 512-thread CTA per SM holding the tile, a stage for the whole next tile
-// and the level-0 twiddles (two 256-thread CTAs per SM with a half-tile
-// stage measured 9 % slower: the unstaged half's load is exposed).
+// The same with a stage for a whole tile, inverse and natural-order layouts.
 __host__ __device__ constexpr int col_inv_pipe_warps(int logl) { return 16; }
 __host__ __device__ constexpr int col_inv_pipe_smem_bytes(int logl) {
     return 2 * col_tile_words(logl, 1) * 4 + (1 << logl) * 8;
 }
 
-// Persistent pass A of a natural-order transform (k_col_fwd_pipe1): 2^10-row
-// columns, one 512-thread CTA per SM holding the tile, a stage for the whole
-// next tile and the level-0 twiddles.
 __host__ __device__ constexpr int col_pipe1_smem_bytes(int logl) {
     return 2 * col_tile_words(logl, 2) * 4 + (1 << logl) * 8;
 }
@@ -157,9 +130,8 @@ __host__ __device__ constexpr int row_threads(int logl) { return logl == 14 ? 10
 // Threads of the split row kernels (one operand row per CTA): one per
 // 32-word row of the last level.
 __host__ __device__ constexpr int rowsplit_threads(int logl) { return logl >= 10 ? (1 << (logl - 5)) : 32; }
-// Natural-order row transforms (k_row_ntt): one thread per 32-word group of
-// the last level (at least a warp), one row of shared memory per CTA, 1024
-// threads per SM.
+// Shape of one-row CTAs with a thread per 32-word group, 1024 threads per SM
+// (the maps check bounds the row tables' shared memory with it).
 __host__ __device__ constexpr int ntt_row_threads(int logl) { return logl >= 10 ? (1 << (logl - 5)) : 32; }
 __host__ __device__ constexpr int ntt_row_ctas(int logl) { return 1024 / ntt_row_threads(logl) < 32 ? 1024 / ntt_row_threads(logl) : 32; }
 

@@ -74,7 +74,8 @@ struct SmallLevel {
     }();
 };
 
-// Position in a row after the row plan's DIF levels -> frequency index.
+// Position in a row after the row plan's DIF levels -> frequency index (the
+// order of a product's row spectra).
 template <int L2>
 __host__ __device__ __forceinline__ u32 row_pos_to_freq(u32 P) {
     constexpr LevelPlan PL = row_plan(L2);

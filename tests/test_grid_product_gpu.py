@@ -43,3 +43,39 @@ def test_cyclic_convolution_of_full_grids(cm, p, em, en):
     sign = lambda v: int((v[::2].astype(np.int64).sum() - v[1::2].astype(np.int64).sum()) % p)
     assert sign(got) == sign(f) * sign(g) % p
     assert sign(got.T) == sign(f.T) * sign(g.T) % p
+
+
+_NO_ROOM = """
+import sys, numpy as np, torch
+import cumodp_b200 as cm
+from cumodp_b200.workloads import SplitMix64
+p, em, en = 469762049, int(sys.argv[1]), int(sys.argv[2])
+r = SplitMix64(64 * em + en)
+def product(em, en, fail):
+    f, g = (r.residues(1 << (em + en), p) for _ in range(2))
+    out = []
+    for n in fail:
+        F, G = (torch.from_numpy(v.view(np.int32).copy()).cuda() for v in (f, g))
+        cm.inject_alloc_failures(n)
+        cm.bivariate_mul_dev(em, en, F.data_ptr(), G.data_ptr(), p)
+        cm.inject_alloc_failures(0)
+        out.append(F.cpu().numpy())
+    return out
+product(1, 10, [0])
+a, b = product(em, en, [1, 0])  # the first allocation of the larger grid is its workspace
+assert np.array_equal(a, b)
+print("same")
+"""
+
+
+@pytest.mark.parametrize("em,en", [(5, 8), (12, 6)])
+def test_grid_without_room_for_its_workspace(em, en):
+    """The workspace of two grids cannot be had: the paths with less workspace give the same product (in a
+    process of its own, where no earlier call has left a larger workspace)."""
+    import pathlib
+    import subprocess
+    import sys
+    root = pathlib.Path(__file__).resolve().parents[1]
+    r = subprocess.run([sys.executable, "-c", _NO_ROOM, str(em), str(en)], cwd=root, capture_output=True,
+                       text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.strip().endswith("same"), r.stdout + r.stderr
