@@ -247,7 +247,7 @@ bool tune_single_cta(const PrimeCtx& pc, int logn, int njobs, int dev, cudaStrea
     if (small_args(pc, canonical_root(pc, logn), logn, dev, &A) != OK) return rule;
     A.jobs = T.djs;
     A.njobs = jobs;
-    ensure_kernel_attrs();
+    if (ensure_kernel_attrs(dev) != OK) return rule;
     const float small_ms = T.time([&] { launch_small(logn, A, jobs, st); }, st);
     const bool single = small_ms <= large_ms;
     tune_store(key, single ? 1 : 0);
@@ -524,7 +524,7 @@ int batch_mul_dev(int count, const sfixn* df, const int64_t* f_off, const u32* F
         if (ce != cudaSuccess) return cuda_err(ce);
     }
     if (!P->exec) {
-        ensure_kernel_attrs();
+        if ((err = ensure_kernel_attrs(dev)) != OK) return err;
         if ((err = prepare_capture(*P, *pc)) != OK) return err;
         cudaStream_t cap;
         cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking);
@@ -573,7 +573,7 @@ int direct_batch(int count, const u32* const* a, const long long* la, const u32*
     const PrimeCtx* pc = prime_ctx(p, &err);
     if (!pc) return err;
     const int dev = current_device();
-    ensure_kernel_attrs();
+    if ((err = ensure_kernel_attrs(dev)) != OK) return err;
     std::map<int, std::vector<int>> cls;
     for (int i = 0; i < count; ++i) {
         const int logn = product_logn(la[i], lb[i]);

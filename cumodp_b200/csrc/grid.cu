@@ -16,14 +16,14 @@ constexpr size_t grid_smem() {
 }
 
 template <int E, int L2>
-void launch_rows_t(const GridArgs& a, long long words, cudaStream_t st) {
+int launch_rows_t(const GridArgs& a, long long words, int dev, cudaStream_t st) {
     constexpr int LT = grid_log(E, L2);
-    static const bool attr = [] {
-        cudaFuncSetAttribute(k_grid_fwd_g<E, L2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)grid_smem<E, L2>());
-        cudaFuncSetAttribute(k_grid_mul_f<E, L2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)grid_smem<E, L2>());
-        return true;
-    }();
-    (void)attr;
+    static DeviceOnce once;
+    const int err = once(dev, [] {
+        const cudaError_t e = allow_smem(k_grid_fwd_g<E, L2>, grid_smem<E, L2>());
+        return e == cudaSuccess ? allow_smem(k_grid_mul_f<E, L2>, grid_smem<E, L2>()) : e;
+    });
+    if (err != OK) return err;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(words >> LT));
     cfg.blockDim = dim3(grid_threads(LT));
@@ -41,9 +41,10 @@ void launch_rows_t(const GridArgs& a, long long words, cudaStream_t st) {
     tr = pass_timing_begin(st, &e0);
     cudaLaunchKernelEx(&cfg, k_grid_mul_f<E, L2>, a);
     if (tr) pass_timing_end(st, "grid_mul_f", e0);
+    return OK;
 }
 
-typedef void (*RowsFn)(const GridArgs&, long long, cudaStream_t);
+typedef int (*RowsFn)(const GridArgs&, long long, int, cudaStream_t);
 const RowsFn kRows[3][kMaxRowLog + 1] = {
     {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, launch_rows_t<0, 6>, launch_rows_t<0, 7>, launch_rows_t<0, 8>,
      launch_rows_t<0, 9>, launch_rows_t<0, 10>, launch_rows_t<0, 11>, launch_rows_t<0, 12>, launch_rows_t<0, 13>,
@@ -73,7 +74,7 @@ int grid_mul_dev(u32* F, u32* G, int em, int en, u32 p, cudaStream_t st) {
     if (!pc) return err;
     const int dev = current_device(), l2 = E + en;
     const long long words = 1ll << (em + en);
-    ensure_kernel_attrs();
+    if ((err = ensure_kernel_attrs(dev)) != OK) return err;
     u32* ws = (u32*)workspace(dev, kWsBiv, (size_t)2 * words * sizeof(u32), &err);
     if (!ws) return err;
     const u32 wm = canonical_root(*pc, em), wn = canonical_root(*pc, en), wc = canonical_root(*pc, l1);
@@ -100,7 +101,7 @@ int grid_mul_dev(u32* F, u32* G, int em, int en, u32 p, cudaStream_t st) {
     if (E > 0 && !(A.lead = grid_lead_tables(dev, p, wm, em, en, l1, scale, &err))) return err;
     C.job0 = LargeJob{F, G, F, (int)words, (int)words, (int)words, 0, A.wa, A.wb};
     launch_col_fwd(C, 1, st);
-    kRows[E][en](A, words, st);
+    if ((err = kRows[E][en](A, words, dev, st)) != OK) return err;
     launch_col_inv(C, 1, st);
     return cuda_err(cudaGetLastError());
 }

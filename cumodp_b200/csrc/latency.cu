@@ -204,17 +204,16 @@ int latency_mul_i64(const u32* primes, int np, int dev, const long long* a, int 
 namespace {
 
 template <int LOGL>
-void launch_level_t(const LevelArgs& a, int sms, cudaStream_t st) {
+int launch_level_t(const LevelArgs& a, int dev, cudaStream_t st) {
     constexpr size_t smem = lat_smem(LOGL, 1);
-    static const bool attr = [] {
-        cudaFuncSetAttribute(k_monic_level<LOGL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        return true;
-    }();
-    (void)attr;
-    const int grid = std::min(a.npairs, sms * level_ctas(LOGL));
+    static DeviceOnce once;
+    const int err = once(dev, [] { return allow_smem(k_monic_level<LOGL>, smem); });
+    if (err != OK) return err;
+    const int grid = std::min(a.npairs, sm_count(dev) * level_ctas(LOGL));
     k_monic_level<LOGL><<<grid, level_threads(LOGL), smem, st>>>(a);
+    return cuda_err(cudaGetLastError());
 }
-typedef void (*LevelFn)(const LevelArgs&, int, cudaStream_t);
+typedef int (*LevelFn)(const LevelArgs&, int, cudaStream_t);
 const LevelFn kLevel[] = {launch_level_t<5>, launch_level_t<6>,  launch_level_t<7>,  launch_level_t<8>,
                           launch_level_t<9>, launch_level_t<10>, launch_level_t<11>, launch_level_t<12>};
 
@@ -241,9 +240,9 @@ int monic_level_dev(const PrimeCtx& pc, int l, int npairs, const u32* in, u32* o
     a.npairs = npairs;
     cudaEvent_t e0;
     const bool tr = pass_timing_begin(st, &e0);
-    kLevel[logn - kMinLog](a, sm_count(dev), st);
+    err = kLevel[logn - kMinLog](a, dev, st);
     if (tr) pass_timing_end(st, "monic_level", e0);
-    return cuda_err(cudaGetLastError());
+    return err;
 }
 
 }  // namespace cmb

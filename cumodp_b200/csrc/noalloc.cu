@@ -168,7 +168,7 @@ int mul_dev_noalloc(const u32* a, long long la, const u32* b, long long lb, u32*
             return cuda_err(ce);
         }
     }
-    ensure_kernel_attrs();
+    if ((err = ensure_kernel_attrs(dev)) != OK) return err;
     const long long n = 1ll << logn;
     const u32 root = canonical_root(*pc, logn);
     const bool large = logn > kMaxSmallLog;

@@ -93,16 +93,15 @@ namespace {
 // (root: the transform's own, scale applied to every output): src row s to
 // dst row s, or to row k1(s) when the rows are slots of a column pass of 2^l1.
 template <int L2, bool SLOT>
-void launch_row_nat_t(const RowNatArgs& a, int jobs, cudaStream_t st) {
-    static const bool attr = [] {
-        cudaFuncSetAttribute(k_row_nat<L2, SLOT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)nat_smem(L2));
-        return true;
-    }();
-    (void)attr;
+int launch_row_nat_t(const RowNatArgs& a, int jobs, int dev, cudaStream_t st) {
+    static DeviceOnce once;
+    const int err = once(dev, [] { return allow_smem(k_row_nat<L2, SLOT>, nat_smem(L2)); });
+    if (err != OK) return err;
     const u32 grid = (u32)(((u64)a.rows + nat_rows(L2) - 1) / nat_rows(L2));
     k_row_nat<L2, SLOT><<<dim3(grid, jobs), nat_threads(L2), nat_smem(L2), st>>>(a);
+    return cuda_err(cudaGetLastError());
 }
-typedef void (*RowNatFn)(const RowNatArgs&, int, cudaStream_t);
+typedef int (*RowNatFn)(const RowNatArgs&, int, int, cudaStream_t);
 const RowNatFn kRowNat[15] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
                               launch_row_nat_t<6, false>, launch_row_nat_t<7, false>, launch_row_nat_t<8, false>,
                               launch_row_nat_t<9, false>, launch_row_nat_t<10, false>, launch_row_nat_t<11, false>,
@@ -125,14 +124,14 @@ int row_nat(const PrimeCtx& pc, const u32* src, u32* dst, long long rows, int k,
     if (l1) A.colpl = col_plan(l1);
     cudaEvent_t e0;
     const bool tr = pass_timing_begin(st, &e0);
-    for (long long r0 = 0; r0 < rows; r0 += 1ll << 30) {  // one launch when l1 > 0
+    for (long long r0 = 0; r0 < rows && err == OK; r0 += 1ll << 30) {  // one launch when l1 > 0
         A.src = src + (r0 << k);
         A.dst = dst + (r0 << k);
         A.rows = (u32)std::min<long long>(1ll << 30, rows - r0);
-        kRowNat[k](A, 1, st);
+        err = kRowNat[k](A, 1, dev, st);
     }
     if (tr) pass_timing_end(st, "ntt_row", e0);
-    return cuda_err(cudaGetLastError());
+    return err;
 }
 
 // The rows of four-step transforms of 2^(l1 + l2) words with root `root`, and
@@ -157,8 +156,9 @@ int rows_and_transpose(const PrimeCtx& pc, const u32* w1, u32* w2, u32* out, int
     A.job_stride = 1ll << (l1 + l2);
     cudaEvent_t e0;
     bool tr = pass_timing_begin(st, &e0);
-    kRowSlot[l2](A, jobs, st);
+    err = kRowSlot[l2](A, jobs, dev, st);
     if (tr) pass_timing_end(st, "ntt_row", e0);
+    if (err != OK) return err;
     tr = pass_timing_begin(st, &e0);
     if (l1 >= 6)
         k_transpose64<<<dim3((1 << l2) / 64, (1 << l1) / 64, jobs), 256, 0, st>>>(w2, out, 1 << l1, 1 << l2);
@@ -170,15 +170,13 @@ int rows_and_transpose(const PrimeCtx& pc, const u32* w1, u32* w2, u32* out, int
 
 // Forward-column launchers shared with the product path (single operand).
 template <int L1>
-void launch_colfwd1_t(const LargeArgs& a, int tiles, cudaStream_t st) {
-    const size_t smem = col_smem_bytes(L1, 2);
-    static bool attr = false;
-    if (!attr) {
-        cudaFuncSetAttribute(k_col_fwd<L1, col_warps(L1, 2), 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem);
-        attr = true;
-    }
+int launch_colfwd1_t(const LargeArgs& a, int tiles, int dev, cudaStream_t st) {
+    constexpr size_t smem = col_smem_bytes(L1, 2);
+    static DeviceOnce once;
+    const int err = once(dev, [] { return allow_smem(k_col_fwd<L1, col_warps(L1, 2), 2>, smem); });
+    if (err != OK) return err;
     k_col_fwd<L1, col_warps(L1, 2), 2><<<dim3(tiles, 1, a.njobs), col_warps(L1, 2) * 32, smem, st>>>(a);
+    return OK;
 }
 // w is a primitive 2^k-th root of unity mod p.
 bool root_has_order(u32 w, int k, u32 p) {
@@ -207,8 +205,9 @@ int column_pass(const PrimeCtx& pc, u32 root_c, int l1, int l2, const u32* src, 
     A.job0 = LargeJob{src, nullptr, nullptr, (int)std::min<long long>(len, 1ll << 30), 0, 0, 0, dst, nullptr};
     A.jobs = djobs;  // a device job table (a list of transforms), or nullptr: job0
     A.njobs = njobs;
-    if (!launch_col_fwd1(A, njobs, st)) launch_colfwd1_t<kMaxColLog>(A, (1 << l2) / col_tile_cols(kMaxColLog, 2), st);
-    return OK;
+    if ((err = ensure_kernel_attrs(dev)) != OK) return err;
+    if (launch_col_fwd1(A, njobs, st)) return OK;
+    return launch_colfwd1_t<kMaxColLog>(A, (1 << l2) / col_tile_cols(kMaxColLog, 2), dev, st);
 }
 
 // First radix-2 (decimation-in-frequency) step of a transform of n = 2h

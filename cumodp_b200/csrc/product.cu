@@ -13,15 +13,16 @@ namespace cmb {
 
 namespace {
 
+// allow_smem unless an earlier one failed.
+template <class K>
+void allow_more(cudaError_t* e, K* kernel, size_t bytes) {
+    if (*e == cudaSuccess) *e = allow_smem(kernel, bytes);
+}
+
 template <int LOGL>
 void launch_small_t(const SmallArgs& a, int nctas, cudaStream_t st) {
     constexpr int L = 1 << LOGL;
     const size_t smem = (size_t)small_ppc(LOGL) * 2 * L * sizeof(u32);
-    static bool attr = false;
-    if (!attr) {
-        cudaFuncSetAttribute(k_small_product<LOGL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        attr = true;
-    }
     k_small_product<LOGL><<<nctas, small_threads(LOGL), smem, st>>>(a);
 }
 
@@ -54,11 +55,6 @@ void launch_pdl(K kernel, dim3 grid, int threads, size_t smem, cudaStream_t st, 
 template <int L1>
 void launch_col_fwd_t(const LargeArgs& a, dim3 grid, cudaStream_t st) {
     const size_t smem = col_smem_bytes(L1, false);
-    static bool attr = false;
-    if (!attr) {
-        cudaFuncSetAttribute(k_col_fwd<L1, col_warps(L1, false)>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        attr = true;
-    }
     k_col_fwd<L1, col_warps(L1, false)><<<grid, col_warps(L1, false) * 32, smem, st>>>(a);
 }
 }  // namespace
@@ -79,21 +75,11 @@ namespace {
 template <int L1>
 void launch_col_inv_t(const LargeArgs& a, dim3 grid, cudaStream_t st) {
     const size_t smem = col_smem_bytes(L1, true);
-    static bool attr = false;
-    if (!attr) {
-        cudaFuncSetAttribute(k_col_inv<L1, col_warps(L1, true)>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        attr = true;
-    }
     launch_pdl(k_col_inv<L1, col_warps(L1, true)>, grid, col_warps(L1, true) * 32, smem, st, a);
 }
 template <int L2>
 void launch_row_t(const LargeArgs& a, dim3 grid, cudaStream_t st) {
     const size_t smem = (size_t)2 * (1 << L2) * sizeof(u32);
-    static bool attr = false;
-    if (!attr) {
-        cudaFuncSetAttribute(k_row_fused<L2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        attr = true;
-    }
     k_row_fused<L2><<<grid, row_threads(L2), smem, st>>>(a);
 }
 
@@ -185,9 +171,9 @@ void launch_cold_inv_t(const LargeArgs& a, int njobs, cudaStream_t st) {
                st, a);
 }
 template <int L1>
-void attr_cold() {
-    cudaFuncSetAttribute(k_cold_fwd<L1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cold_smem(L1));
-    cudaFuncSetAttribute(k_cold_inv<L1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cold_smem(L1));
+void attr_cold(cudaError_t* e) {
+    allow_more(e, k_cold_fwd<L1>, cold_smem(L1));
+    allow_more(e, k_cold_inv<L1>, cold_smem(L1));
 }
 typedef void (*ColdFwdFn)(const LargeArgs&, int, int, cudaStream_t);
 typedef void (*ColdInvFn)(const LargeArgs&, int, cudaStream_t);
@@ -205,28 +191,22 @@ const PassFn kRow[15] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
                          launch_row_t<14>};
 
 template <int LOGL>
-void attr_small() {
-    cudaFuncSetAttribute(k_small_product<LOGL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)((size_t)small_ppc(LOGL) * 2 * (1 << LOGL) * sizeof(u32)));
+void attr_small(cudaError_t* e) {
+    allow_more(e, k_small_product<LOGL>, (size_t)small_ppc(LOGL) * 2 * (1 << LOGL) * sizeof(u32));
 }
 template <int L1>
-void attr_col() {
-    cudaFuncSetAttribute(k_col_fwd<L1, col_warps(L1, false)>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         col_smem_bytes(L1, false));
-    cudaFuncSetAttribute(k_col_inv<L1, col_warps(L1, true)>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         col_smem_bytes(L1, true));
+void attr_col(cudaError_t* e) {
+    allow_more(e, k_col_fwd<L1, col_warps(L1, false)>, col_smem_bytes(L1, false));
+    allow_more(e, k_col_inv<L1, col_warps(L1, true)>, col_smem_bytes(L1, true));
 }
 template <int L2>
-void attr_row() {
-    cudaFuncSetAttribute(k_row_fused<L2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         2 * (1 << L2) * (int)sizeof(u32));
+void attr_row(cudaError_t* e) {
+    allow_more(e, k_row_fused<L2>, (size_t)2 * (1 << L2) * sizeof(u32));
 }
-
 template <int L2>
-void attr_rowsplit() {
-    const int smem = (int)rowsplit_smem<L2>();
-    cudaFuncSetAttribute(k_row_fwd_g<L2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    cudaFuncSetAttribute(k_row_mul_f<L2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+void attr_rowsplit(cudaError_t* e) {
+    allow_more(e, k_row_fwd_g<L2>, rowsplit_smem<L2>());
+    allow_more(e, k_row_mul_f<L2>, rowsplit_smem<L2>());
 }
 
 const PassFn kRowG[15] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
@@ -246,17 +226,19 @@ int ceil_log2(long long s) {
 
 }  // namespace
 
-void ensure_kernel_attrs() {
-    static std::once_flag once;
-    std::call_once(once, [] {
-        attr_small<5>(); attr_small<6>(); attr_small<7>(); attr_small<8>(); attr_small<9>();
-        attr_small<10>(); attr_small<11>(); attr_small<12>(); attr_small<13>(); attr_small<14>();
-        attr_col<11>();
-        attr_cold<6>(); attr_cold<7>(); attr_cold<8>(); attr_cold<9>(); attr_cold<10>();
-        attr_row<6>(); attr_row<7>(); attr_row<8>(); attr_row<9>(); attr_row<10>();
-        attr_row<11>(); attr_row<12>(); attr_row<13>(); attr_row<14>();
-        attr_rowsplit<6>(); attr_rowsplit<7>(); attr_rowsplit<8>(); attr_rowsplit<9>(); attr_rowsplit<10>();
-        attr_rowsplit<11>(); attr_rowsplit<12>(); attr_rowsplit<13>(); attr_rowsplit<14>();
+int ensure_kernel_attrs(int dev) {
+    static DeviceOnce once;
+    return once(dev, [] {
+        cudaError_t e = cudaSuccess;
+        attr_small<5>(&e); attr_small<6>(&e); attr_small<7>(&e); attr_small<8>(&e); attr_small<9>(&e);
+        attr_small<10>(&e); attr_small<11>(&e); attr_small<12>(&e); attr_small<13>(&e); attr_small<14>(&e);
+        attr_col<11>(&e);
+        attr_cold<6>(&e); attr_cold<7>(&e); attr_cold<8>(&e); attr_cold<9>(&e); attr_cold<10>(&e);
+        attr_row<6>(&e); attr_row<7>(&e); attr_row<8>(&e); attr_row<9>(&e); attr_row<10>(&e);
+        attr_row<11>(&e); attr_row<12>(&e); attr_row<13>(&e); attr_row<14>(&e);
+        attr_rowsplit<6>(&e); attr_rowsplit<7>(&e); attr_rowsplit<8>(&e); attr_rowsplit<9>(&e); attr_rowsplit<10>(&e);
+        attr_rowsplit<11>(&e); attr_rowsplit<12>(&e); attr_rowsplit<13>(&e); attr_rowsplit<14>(&e);
+        return e;
     });
 }
 
@@ -359,7 +341,6 @@ void launch_col_fwd(const LargeArgs& a, int njobs, cudaStream_t st) {
 
 bool launch_col_fwd1(const LargeArgs& a, int njobs, cudaStream_t st) {
     if (a.l1 > kMaxDirectColLog) return false;
-    ensure_kernel_attrs();
     kColdFwd[a.l1](a, 1, njobs, st);
     return true;
 }
@@ -462,7 +443,7 @@ int mul_dev_len(const u32* a, long long la, const u32* b, long long lb, u32* h, 
     int err = OK;
     const long long n = 1ll << logn;
     const int dev = current_device();
-    ensure_kernel_attrs();
+    if ((err = ensure_kernel_attrs(dev)) != OK) return err;
     if (lh > n) {  // coefficients beyond the transform length are zero
         cudaError_t e = cudaMemsetAsync(h + n, 0, (size_t)(lh - n) * sizeof(u32), st);
         if (e != cudaSuccess) return cuda_err(e);

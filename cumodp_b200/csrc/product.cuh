@@ -66,9 +66,9 @@ int latency_mul_i64(const u32* primes, int np, int dev, const long long* a, int 
 constexpr int kMaxLevelLog = 12;
 int monic_level_dev(const PrimeCtx& pc, int l, int npairs, const u32* in, u32* out, cudaStream_t st);
 
-// Sets the shared-memory limits of every product kernel once (must run
-// before any launch is captured into a graph).
-void ensure_kernel_attrs();
+// Sets the shared-memory limits of every product kernel on the current device
+// dev, once (must run before the first launch there).
+int ensure_kernel_attrs(int dev);
 
 // Batched products on caller-owned buffers, direct launches (batch.cu).
 size_t direct_ws_words(int count, const long long* la, const long long* lb);

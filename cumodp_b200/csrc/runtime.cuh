@@ -3,6 +3,7 @@
 #pragma once
 #include <nvtx3/nvToolsExt.h>
 #include <cuda_runtime.h>
+#include <atomic>
 #include <cstddef>
 #include <cstdint>
 #include <map>
@@ -143,5 +144,34 @@ std::string pass_timing_report(bool reset);
 
 // Copies the last CUDA error (if any) into a library code.
 int cuda_err(cudaError_t e);
+
+// Set-up that belongs to a device, done once on each: function attributes (the
+// dynamic shared-memory limit above 48 KiB) are the current device's alone.
+// `set` runs on the current device `dev` and may run again (two threads at
+// once; after a failure, which is returned and not remembered).
+class DeviceOnce {
+public:
+    template <class F>
+    int operator()(int dev, F set) {
+        const u64 bit = dev >= 0 && dev < 64 ? 1ull << dev : 0;
+        if (done_.load(std::memory_order_acquire) & bit) return OK;
+        const cudaError_t e = set();
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            return cuda_err(e);
+        }
+        done_.fetch_or(bit, std::memory_order_release);
+        return OK;
+    }
+
+private:
+    std::atomic<u64> done_{0};
+};
+
+// Raises a kernel's dynamic shared-memory limit on the current device.
+template <class K>
+cudaError_t allow_smem(K* kernel, size_t bytes) {
+    return cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
 
 }  // namespace cmb

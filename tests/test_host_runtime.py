@@ -1,0 +1,109 @@
+"""The library's host side on a stand-in CUDA runtime, without a GPU.
+
+tests/fake_cudart.cpp takes the runtime's place: kernels do nothing, but
+function attributes belong to a device, launches over a kernel's shared-memory
+limit are refused, and every launch, copy, event record and wait is logged with
+its stream.  Each case runs in a process of its own.
+"""
+import ast
+import os
+import shutil
+import subprocess
+import sys
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CUDA_INC = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")
+
+PRELUDE = r"""
+import ctypes, sys
+fake = ctypes.CDLL(sys.argv[1], mode=ctypes.RTLD_GLOBAL)
+sys.path.insert(0, sys.argv[2])
+import numpy as np
+import cumodp_b200 as cm
+fake.fake_log.restype = ctypes.c_char_p
+L = cm.lib()
+P = 469762049
+
+def log():
+    return [fake.fake_log(i).decode() for i in range(fake.fake_log_size())]
+
+def root(k):
+    return pow(3, (P - 1) >> k, P)  # 3 generates the group
+
+mem = np.zeros(1 << 28, np.int32)  # pages are there once touched
+A, B, H = (mem.ctypes.data + (i << 28) for i in range(3))  # 2^26 words each
+
+def product(logn, stream=0):
+    n = 1 << (logn - 1)
+    cm.fftmul_uni_dev(H, 2 * n - 1, A, n - 1, B, n - 1, P, stream)
+
+def batch(shapes, stream=0):
+    d = np.array([n - 1 for n in shapes], np.int32)
+    off = np.concatenate([[0], np.cumsum(d.astype(np.int64) + 1)[:-1]])
+    cm.fftmul_batch_dev(d, off, A, d, off, B, 2 * off, H, P, stream)
+
+def exact(n, bits=34, stream=0):
+    rc = L.cumodp_twoconv_mul_i64_dev(n, A, n, B, H, bits, 0, stream or None)
+    assert rc == 0, rc
+
+def big(n, words, stream=0):
+    ow = L.cumodp_twoconv_big_out_words(n, n, 64 * words)
+    rc = L.cumodp_twoconv_mul_big_dev(n, A, n, B, words + 1, H, ow, 64 * words, stream or None)
+    assert rc == 0, rc
+"""
+
+
+@pytest.fixture(scope="module")
+def fake(tmp_path_factory):
+    if not shutil.which("g++") or not os.path.exists(os.path.join(CUDA_INC, "cuda_runtime_api.h")):
+        pytest.skip("no compiler or CUDA headers")
+    d = tmp_path_factory.mktemp("fake")
+    ver = d / "v.map"
+    ver.write_text("libcudart.so.12 { global: *; };\n")
+    so = str(d / "libcudart.so.12")
+    r = subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-I", CUDA_INC, "-Wl,-soname,libcudart.so.12",
+                        f"-Wl,--version-script={ver}", os.path.join(ROOT, "tests", "fake_cudart.cpp"), "-o", so],
+                       capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr[-2000:]
+
+    def run(code, **env):
+        """What the code's last line prints, as a Python value."""
+        out = subprocess.run([sys.executable, "-c", PRELUDE + code, so, ROOT], capture_output=True, text=True,
+                             timeout=600, env=dict(os.environ, **env))
+        assert out.returncode == 0, out.stderr[-2000:]
+        return ast.literal_eval(out.stdout.strip().splitlines()[-1])
+
+    return run
+
+
+@pytest.mark.parametrize("env", [{}, {"CUMODP_ROW_FUSED": "1"}])
+def test_every_entry_launches_on_a_second_device(fake, env):
+    """Kernels with more than 48 KiB of shared memory run on every device of a process, not only on the first."""
+    bad = fake(r"""
+bad = []
+for dev in (0, 1):
+    cm.select_device(dev)
+    calls = [("product", product, (k,)) for k in range(5, 26)]
+    calls += [("fft", lambda k: cm.fft_uni_dev(A, k, root(k), P, False, 0), (k,)) for k in range(5, 26)]
+    calls += [("list", lambda k: cm.list_fft_dev(A, 3, k, root(k), P, True, 0), (k,)) for k in (6, 13, 14, 15, 20)]
+    calls += [("fft2d", lambda m, n: cm.fft_bivariate_dev(A, m, root(m), n, root(n), P, False, 0), e)
+              for e in ((0, 14), (11, 14), (10, 6), (5, 14))]
+    calls += [("bivariate", lambda m, n: cm.bivariate_mul_dev(m, n, A, B, P, 0), e)
+              for e in ((5, 6), (12, 12), (10, 14), (11, 13), (11, 14), (12, 10), (2, 5))]
+    calls += [("level", lambda l: cm.subproduct_level_dev(l, 3, A, H, P, 0), (l,))
+              for l in (1, 16, 300, 513, 1024, 2000, 2048, 5000)]
+    calls += [("noalloc", lambda k: cm.fftmul_uni_dev_noalloc(H, (1 << k) - 1, A, (1 << (k - 1)) - 1, B,
+                                                             (1 << (k - 1)) - 1, P, 0), (k,)) for k in (8, 13, 14, 17, 20)]
+    calls += [("exact", exact, (n,)) for n in (1000, 8192, 40000, 300000)]
+    calls += [("big", big, e) for e in ((4, 1), (100, 8), (1024, 16))]
+    calls += [("batch", lambda *s: batch(s), e) for e in ((16, 100, 2000), (4096,) * 3, (8192,) * 3, (1 << 17,) * 2)]
+    for name, f, args in calls:
+        try:
+            f(*args)
+        except Exception as e:
+            bad.append((dev, name, args, str(e)))
+print(bad + [l for l in log() if l.startswith("refused")])
+""", CUMODP_AUTOTUNE="0", **env)
+    assert bad == []
