@@ -220,6 +220,8 @@ int tune_row_log(const PrimeCtx& pc, int logn, int njobs, int dev, cudaStream_t 
     // timed at the class's own size (its bucket), up to 2^25 operand words: a split that wins for a few
     // products (many small CTAs) can lose for hundreds
     const int jobs = std::min(key.bucket, std::max(1, (int)((1ll << 25) >> logn)));
+    // a refused launch would count as a slow one
+    if (ensure_kernel_attrs(dev) != OK) return default_row_log(logn);
     TuneBufs T(jobs, 1ll << logn, st);
     if (!T.ok) return default_row_log(logn);
     float ms;
@@ -239,6 +241,7 @@ bool tune_single_cta(const PrimeCtx& pc, int logn, int njobs, int dev, cudaStrea
     if (tune_lookup(key, &v)) return v != 0;
     if (!allow_tuning) return rule;
     const int jobs = key.bucket;  // the class's own size (up to 256 products: 64 MiB at 2^14)
+    if (ensure_kernel_attrs(dev) != OK) return rule;
     TuneBufs T(jobs, 1ll << logn, st);
     if (!T.ok) return rule;
     float large_ms;
@@ -247,7 +250,6 @@ bool tune_single_cta(const PrimeCtx& pc, int logn, int njobs, int dev, cudaStrea
     if (small_args(pc, canonical_root(pc, logn), logn, dev, &A) != OK) return rule;
     A.jobs = T.djs;
     A.njobs = jobs;
-    if (ensure_kernel_attrs(dev) != OK) return rule;
     const float small_ms = T.time([&] { launch_small(logn, A, jobs, st); }, st);
     const bool single = small_ms <= large_ms;
     tune_store(key, single ? 1 : 0);

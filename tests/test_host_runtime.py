@@ -107,3 +107,16 @@ for dev in (0, 1):
 print(bad + [l for l in log() if l.startswith("refused")])
 """, CUMODP_AUTOTUNE="0", **env)
     assert bad == []
+
+
+def test_first_batch_of_a_process_times_every_candidate(fake):
+    """The autotuner's launches are allowed before the first product of a process has run: a refused one
+    counts as a slow one, and the choice is kept (in CUMODP_TUNE_FILE too)."""
+    log = fake("""
+batch((1 << 19,) * 2)       # 2^20: every split
+batch((8192,) * 3)          # 2^14: one CTA per product or three passes
+print([l for l in log() if l.startswith(("refused", "launch"))])
+""", CUMODP_AUTOTUNE="1")
+    assert [x for x in log if x.startswith("refused")] == []
+    assert any("k_small_productILi14" in x for x in log)
+    assert all(any(f"k_row_mul_fILi{l2}E" in x for x in log) for l2 in range(9, 15))
