@@ -74,6 +74,32 @@ __host__ __device__ constexpr size_t lat_smem(int logl, int cluster) {
     return words * sizeof(u32) + (size_t)2 * lat_entries(logl) * sizeof(Tw);
 }
 
+// Exponent e of entry t of latency_tables' array: the entry is w^e for the
+// product's primitive 2^logn-th root w.  The block's levels (2^logl words),
+// forward then inverse, and for logl < logn the leading level, forward then
+// inverse (an inverse entry's exponent is 2^logn less the forward one's).
+struct LatExponent {
+    LevelPlan pl;
+    int logl, logn, block;  // block: lat_entries(logl)
+    __host__ __device__ u32 operator()(u32 t) const {
+        const u32 n = 1u << logn;
+        u32 e, q = t < 2u * block ? t % block : (t - 2u * block) % n;
+        const bool inv = t < 2u * block ? t >= (u32)block : t - 2u * block >= n;
+        if (t < 2u * block) {
+            int i = 0, lb = logl;
+            while (q >= 1u << lb) {
+                q -= 1u << lb;
+                lb -= pl.logr[i++];
+            }
+            const int lt = lb - pl.logr[i];  // 2^lt tasks a block
+            e = ((q & ((1u << lt) - 1)) * rev_bits(q >> lt, pl.logr[i])) << (logn - lb);
+        } else {
+            e = (q & ((1u << logl) - 1)) * rev_bits(q >> logl, logn - logl);
+        }
+        return inv ? (n - e) & (n - 1) : e;
+    }
+};
+
 struct LatPrime {
     PrimeK pk;
     Tw scale;        // 2^32 / n (undoes Montgomery's 2^-32 and the inverse's n)

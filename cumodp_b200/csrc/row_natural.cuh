@@ -77,6 +77,15 @@ struct RowNatArgs {
 // in; the second is the task's own and commutes with the DFT.  Per slot: W^(TB
 // m) for m < R0, then W^o for every task.
 __host__ __device__ constexpr int nat_slot_entries(int logl) { return (1 << nat_plan(logl).logr[0]) + nat_row_threads(logl); }
+// Exponent of entry t of nat_slot_tables' array to the base w.
+struct SlotExponent {
+    LevelPlan colpl;
+    int l1, r0, tb;  // columns of 2^l1; level 0's radix and tasks
+    __host__ __device__ u32 operator()(u32 t) const {
+        const u32 s = t / (u32)(r0 + tb), i = t % (u32)(r0 + tb);
+        return col_slot_to_k1(s, colpl, l1) * (i < (u32)r0 ? tb * i : i - r0);
+    }
+};
 
 #ifdef __CUDACC__
 

@@ -242,29 +242,52 @@ cudaError_t dev_malloc_async(void** p, size_t bytes, cudaStream_t st) {
     return cudaMallocAsync(p, bytes, st);
 }
 
+// The stream tables are made on, per device.
+static cudaStream_t table_stream() {
+    static std::mutex m;
+    static std::map<int, cudaStream_t> streams;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    std::lock_guard<std::mutex> g(m);
+    auto it = streams.find(dev);
+    if (it != streams.end()) return it->second;
+    cudaStream_t s;
+    cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
+    return streams[dev] = s;
+}
+
 // Host-to-device upload of a cached table that has landed when it returns.
 // cudaMemcpy from pageable memory may return once the words are staged,
 // before the DMA lands, and the kernels that read the table run on
 // non-blocking streams, which do not wait for it.
 static cudaError_t upload_now(void* d, const void* h, size_t bytes) {
-    static std::mutex m;
-    static std::map<int, cudaStream_t> streams;
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaStream_t s;
-    {
-        std::lock_guard<std::mutex> g(m);
-        auto it = streams.find(dev);
-        if (it == streams.end()) {
-            cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
-            streams[dev] = s;
-        } else {
-            s = it->second;
-        }
-    }
+    const cudaStream_t s = table_stream();
     cudaError_t e = cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     return e;
+}
+
+// Entry t is w^ex(t), computed from sq[i] = w^(2^i) (Montgomery form).  For the
+// tables of 10^5 entries and more, where the host's two 64-bit divisions an
+// entry and the upload are milliseconds.  Measured, host -> here: a prime's
+// first product of 2^16 points 2.48 -> 0.38 ms (most of it the allocation), of
+// 2^14 340 -> 39 us; a root's first transform of 2^24 5.5 -> 0.73 ms.
+struct PowerArgs {
+    Tw* out;
+    u32 count, p, pinv_neg, one_m;
+    double r32p;
+    u32 sq[32];
+};
+template <class E>
+__global__ void __launch_bounds__(256) k_power_table(const __grid_constant__ PowerArgs A, const __grid_constant__ E ex) {
+    for (u32 t = blockIdx.x * blockDim.x + threadIdx.x; t < A.count; t += gridDim.x * blockDim.x) {
+        u32 v = A.one_m;
+#pragma unroll 1
+        for (u32 e = ex(t), i = 0; e; e >>= 1, ++i)
+            if (e & 1) v = mul_mont(v, A.sq[i], A.p, A.pinv_neg);
+        v = red1(mul_mont(v, 1u, A.p, A.pinv_neg), A.p);
+        A.out[t] = Tw{v, shoup_quot_dev(v, A.p, A.r32p)};
+    }
 }
 
 namespace {
@@ -288,17 +311,40 @@ const Tw* keep_table(Caches& C, const std::tuple<int, u32, u32, int, int>& key, 
     return d;
 }
 
-// One level's entries in the layout [slot j][task o < tasks]: w^(o bitrev(j)),
-// row by row with one product per entry.
-void push_slot_major(std::vector<Tw>& t, u32 w, int logr, int tasks, u32 p) {
-    for (int j = 0; j < 1 << logr; ++j) {
-        const u32 step = powmod_exact(w, bitrev((u32)j, logr), p);
-        u32 v = 1;
-        for (int o = 0; o < tasks; ++o) {
-            t.push_back(tw_of(v, p));
-            v = mulmod_exact(v, step, p);
-        }
+// A table of `count` powers of w, a primitive 2^logn-th root, made on the
+// device and kept under key (C.m held).
+template <class E>
+const Tw* build_powers(Caches& C, const std::tuple<int, u32, u32, int, int>& key, u32 p, u32 w, int logn, size_t count,
+                       const E& ex, int* err) {
+    PowerArgs A;
+    A.count = (u32)count;
+    A.p = p;
+    u32 inv = 1;  // p^-1 mod 2^32 by Newton iteration
+    for (int i = 0; i < 5; ++i) inv *= 2 - p * inv;
+    A.pinv_neg = 0u - inv;
+    A.one_m = (u32)((1ull << 32) % p);
+    A.r32p = 4294967296.0 / (double)p;
+    u32 v = w;
+    for (int i = 0; i < 32; ++i) {
+        A.sq[i] = i < logn ? mulmod_exact(v, A.one_m, p) : 0u;
+        v = mulmod_exact(v, v, p);
     }
+    if (dev_malloc((void**)&A.out, count * sizeof(Tw)) != cudaSuccess) {
+        cudaGetLastError();
+        *err = OUT_OF_MEMORY;
+        return nullptr;
+    }
+    const cudaStream_t st = table_stream();
+    k_power_table<<<(unsigned)std::min<size_t>((count + 255) / 256, 148 * 8), 256, 0, st>>>(A, ex);
+    if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess) {
+        cudaGetLastError();
+        cudaFree(A.out);
+        *err = FFT_ERROR;
+        return nullptr;
+    }
+    C.bytes += (long long)(count * sizeof(Tw));
+    C.tables[key] = A.out;
+    return A.out;
 }
 
 }  // namespace
@@ -309,19 +355,8 @@ const Tw* latency_tables(int dev, u32 p, u32 root, int logn, int logl, int* err)
     auto key = std::make_tuple(dev, p, root, logn, 16 + logl);
     auto it = C.tables.find(key);
     if (it != C.tables.end()) return it->second;
-    const LevelPlan pl = lat_plan(logl);
-    std::vector<Tw> t;
-    const u32 rinv = powmod_exact(root, (1ull << logn) - 1, p);
-    for (u32 w : {root, rinv}) {
-        int lb = logl;
-        for (int i = 0; i + 1 < pl.nlev; ++i) {
-            push_slot_major(t, powmod_exact(w, 1ull << (logn - lb), p), pl.logr[i], 1 << (lb - pl.logr[i]), p);
-            lb -= pl.logr[i];
-        }
-    }
-    if (logl < logn)
-        for (u32 w : {root, rinv}) push_slot_major(t, w, logn - logl, 1 << logl, p);
-    return keep_table(C, key, t, err);
+    const LatExponent ex{lat_plan(logl), logl, logn, lat_entries(logl)};
+    return build_powers(C, key, p, root, logn, 2 * ((size_t)ex.block + (logl < logn ? 1u << logn : 0u)), ex, err);
 }
 
 const Tw* grid_lead_tables(int dev, u32 p, u32 wm, int em, int en, int l1, u32 scale, int* err) {
@@ -377,23 +412,8 @@ const Tw* nat_slot_tables(int dev, u32 p, u32 w, int l1, int l2, int* err) {
     auto key = std::make_tuple(dev, p, w, l1 * 64 + l2, 4);
     auto it = C.tables.find(key);
     if (it != C.tables.end()) return it->second;
-    const LevelPlan pl = col_plan(l1);
-    const int r0 = 1 << nat_plan(l2).logr[0], tb = nat_row_threads(l2);
-    std::vector<Tw> t;
-    t.reserve((size_t)nat_slot_entries(l2) << l1);
-    auto powers = [&](u32 b, int count) {
-        u32 v = 1;
-        for (int i = 0; i < count; ++i) {
-            t.push_back(tw_of(v, p));
-            v = mulmod_exact(v, b, p);
-        }
-    };
-    for (u32 s = 0; s < 1u << l1; ++s) {
-        const u32 W = powmod_exact(w, col_slot_to_k1(s, pl, l1), p);
-        powers(powmod_exact(W, tb, p), r0);
-        powers(W, tb);
-    }
-    return keep_table(C, key, t, err);
+    const SlotExponent ex{col_plan(l1), l1, 1 << nat_plan(l2).logr[0], nat_row_threads(l2)};
+    return build_powers(C, key, p, w, l1 + l2, (size_t)nat_slot_entries(l2) << l1, ex, err);
 }
 
 static const Tw* level_tables(int dev, u32 p, u32 root, int logl, int kind, int* err) {

@@ -28,6 +28,7 @@
 
 #include "../cumodp_b200/csrc/large_product.cuh"
 #include "../cumodp_b200/csrc/latency_product.cuh"
+#include "../cumodp_b200/csrc/row_natural.cuh"
 
 using namespace cmb;
 
@@ -370,7 +371,61 @@ void latency_check(int cluster) {
     }
 }
 
+// latency_tables' exponents: entry (o, j) of a level of blocks of B = 2^lb
+// words is (w^(2^(logn - lb)))^(+-o bitrev(j)), where the kernels read it.
+template <int LOGL>
+void latency_exponent_check(int logn) {
+    const LevelPlan pl = lat_plan(LOGL);
+    const u32 n = 1u << logn, ne = lat_entries(LOGL);
+    const LatExponent ex{pl, LOGL, logn, (int)ne};
+    auto both = [&](u32 fwd, u32 inv, u32 e, const char* what) {
+        CHECK(ex(fwd) == e, "latency exponent L=%d %s", LOGL, what);
+        CHECK(ex(inv) < n && (ex(inv) + e) % n == 0, "latency inverse exponent L=%d %s", LOGL, what);
+    };
+    u32 off = 0;
+    int lb = LOGL;
+    for (int lev = 0; lev + 1 < pl.nlev; ++lev) {
+        const int r = pl.logr[lev];
+        const u32 TB = 1u << (lb - r);
+        for (u32 j = 0; j < 1u << r; ++j)
+            for (u32 o = 0; o < TB; ++o)
+                both(off + j * TB + o, ne + off + j * TB + o, (n >> lb) * o * rev_bits(j, r), "level");
+        off += 1u << lb;
+        lb -= r;
+    }
+    if (logn > LOGL)
+        for (u32 j = 0; j < n >> LOGL; ++j)
+            for (u32 o = 0; o < 1u << LOGL; ++o)
+                both(2 * ne + (j << LOGL) + o, 2 * ne + n + (j << LOGL) + o, o * rev_bits(j, logn - LOGL), "lead");
+}
+
+// nat_slot_tables' exponents: slot s's W = w^k1(s): W^(TB m), then W^o.
+template <int L2>
+void slot_exponent_check(int l1) {
+    const int r0 = 1 << nat_plan(L2).logr[0], tb = nat_row_threads(L2);
+    const SlotExponent ex{col_plan(l1), l1, r0, tb};
+    CHECK(r0 + tb == nat_slot_entries(L2) && r0 * tb == 1 << L2, "slot L2=%d entries", L2);
+    for (u32 s = 0; s < 1u << l1; ++s) {
+        const u32 k1 = col_slot_to_k1(s, col_plan(l1), l1), at = s * nat_slot_entries(L2);
+        for (int m = 0; m < r0; ++m) CHECK(ex(at + m) == k1 * tb * m, "slot L2=%d factor", L2);
+        for (int o = 0; o < tb; ++o) CHECK(ex(at + r0 + o) == k1 * o, "slot L2=%d task", L2);
+        CHECK((long long)k1 * tb * (r0 - 1) < 1ll << (l1 + L2), "slot L2=%d exponent range", L2);
+    }
+}
+
 int main() {
+    latency_exponent_check<5>(5);
+    latency_exponent_check<9>(9);
+    latency_exponent_check<11>(11);
+    latency_exponent_check<12>(12);
+    latency_exponent_check<8>(12);
+    latency_exponent_check<10>(14);
+    latency_exponent_check<12>(16);
+    slot_exponent_check<10>(5);
+    slot_exponent_check<12>(5);
+    slot_exponent_check<13>(5);
+    slot_exponent_check<14>(10);
+    slot_exponent_check<14>(11);
     latency_check<5>(1);
     latency_check<6>(1);
     latency_check<7>(1);

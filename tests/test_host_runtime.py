@@ -44,8 +44,8 @@ def batch(shapes, stream=0):
     off = np.concatenate([[0], np.cumsum(d.astype(np.int64) + 1)[:-1]])
     cm.fftmul_batch_dev(d, off, A, d, off, B, 2 * off, H, P, stream)
 
-def exact(n, bits=34, stream=0):
-    rc = L.cumodp_twoconv_mul_i64_dev(n, A, n, B, H, bits, 0, stream or None)
+def exact(n, method=0, stream=0):
+    rc = L.cumodp_twoconv_mul_i64_dev(n, A, n, B, H, 34, method, stream or None)
     assert rc == 0, rc
 
 def big(n, words, stream=0):
@@ -120,3 +120,18 @@ print([l for l in log() if l.startswith(("refused", "launch"))])
     assert [x for x in log if x.startswith("refused")] == []
     assert any("k_small_productILi14" in x for x in log)
     assert all(any(f"k_row_mul_fILi{l2}E" in x for x in log) for l2 in range(9, 15))
+
+
+def test_large_tables_are_made_on_the_device(fake):
+    """A prime's or a root's first call uploads no table of more than 2^15 words: the tables of the one-launch
+    products and of the four-step rows are 10^5 entries and more, milliseconds on the host."""
+    uploads = fake("""
+for k in (12, 14, 16):
+    product(k)
+for k in (15, 20, 24):
+    cm.fft_uni_dev(A, k, root(k), P, False, 0)
+cm.subproduct_level_dev(2048, 3, A, H, P, 0)
+exact(8192)
+print([int(l.split()[-1]) for l in log() if l.startswith("copy h2d")])
+""")
+    assert uploads and max(uploads) <= 1 << 18
