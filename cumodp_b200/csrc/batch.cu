@@ -282,6 +282,8 @@ struct BatchPlan {
     std::vector<unsigned char> hjobs;  // host copy of what djobs holds
     u32* ws = nullptr;
     size_t ws_words = 0;
+    StreamOrder order;  // one call's job table must not replace another's under its kernels
+    std::unique_ptr<BatchPlan> retired;  // the first stream's plan, when another stream came with other operands
     cudaGraphExec_t exec = nullptr;
     std::vector<cudaStream_t> side;
     cudaEvent_t fork = nullptr;
@@ -501,6 +503,14 @@ int batch_mul_dev(int count, const sfixn* df, const int64_t* f_off, const u32* F
     PlanCache& PC = plan_cache();
     std::lock_guard<std::mutex> g(PC.m);
     const size_t key = shape_hash(p, dev, la, lb);
+    auto new_plan = [&] {
+        std::unique_ptr<BatchPlan> np(new BatchPlan());
+        np->p = p;
+        np->dev = dev;
+        np->la = la;
+        np->lb = lb;
+        return np;
+    };
     auto it = PC.plans.find(key);
     BatchPlan* P = nullptr;
     if (it != PC.plans.end() && it->second->p == p && it->second->dev == dev && it->second->la == la &&
@@ -508,17 +518,38 @@ int batch_mul_dev(int count, const sfixn* df, const int64_t* f_off, const u32* F
         P = it->second.get();
     } else {
         if (PC.plans.size() >= 64) PC.plans.clear();  // bounded cache of batch shapes
-        std::unique_ptr<BatchPlan> np(new BatchPlan());
-        np->p = p;
-        np->dev = dev;
-        np->la = la;
-        np->lb = lb;
+        std::unique_ptr<BatchPlan> np = new_plan();
         if ((err = build_plan(*np, *pc, st)) != OK) return err;
         P = np.get();
         PC.plans[key] = std::move(np);
     }
     std::vector<unsigned char> hj;
     fill_jobs(*P, F, f_off, G, g_off, H, h_off, hj);
+    // launches of one graph follow one another whatever their streams; only a
+    // new job table has to wait for them
+    bool replace = false;
+    if ((err = P->order.enter(st, hj != P->hjobs ? &replace : nullptr)) != OK) return err;
+    if (replace) {
+        std::unique_ptr<BatchPlan> np = new_plan();
+        if ((err = build_plan(*np, *pc, st)) == OK) {
+            std::unique_ptr<BatchPlan>& slot = PC.plans[key];
+            np->retired = std::move(slot);
+            slot = std::move(np);
+            P = slot.get();
+            fill_jobs(*P, F, f_off, G, g_off, H, h_off, hj);
+            P->order.fresh();
+            if ((err = P->order.enter(st, nullptr)) != OK) return err;
+        } else if ((err = cuda_err(cudaDeviceSynchronize())) != OK) {
+            return err;
+        } else {
+            P->order.fresh();
+        }
+    }
+    struct Leave {
+        StreamOrder& order;
+        cudaStream_t st;
+        ~Leave() { order.leave(st); }
+    } leave{P->order, st};
     if (hj != P->hjobs) {
         P->hjobs.swap(hj);
         // pageable source: the call returns once the bytes are staged
@@ -722,7 +753,8 @@ int pipelined_host_batch(int count, const sfixn* df, const int64_t* f_off, const
     }
     const size_t slot_words = (size_t)(maxa + maxb + maxh);
     int err = OK;
-    u32* d = (u32*)workspace(dev, kWsBatch, kSlots * slot_words * sizeof(u32), &err);
+    const Workspace d_space(dev, kWsBatch, kSlots * slot_words * sizeof(u32), st, &err);
+    u32* d = d_space.get();
     if (!d) return err;
     struct Streams {
         cudaStream_t in, out;
@@ -840,7 +872,8 @@ cumodp_err cumodp_fftmul_batch(int count, const sfixn* df, const int64_t* f_off,
         return (cumodp_err)err;
     }
     int err = OK;
-    u32* d = (u32*)workspace(dev, kWsBatch, (nf + ng + nh) * sizeof(u32), &err);
+    const Workspace d_space(dev, kWsBatch, (nf + ng + nh) * sizeof(u32), st, &err);
+    u32* d = d_space.get();
     if (!d) return (cumodp_err)err;
     u32 *dF = d, *dG = d + nf, *dH = d + nf + ng;
     cudaError_t ce = cudaMemcpyAsync(dF, F, nf * 4, cudaMemcpyHostToDevice, st);

@@ -32,6 +32,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <optional>
 #include <vector>
 
 #include "../../include/cumodp.h"
@@ -428,7 +429,9 @@ int bigconv_mul_dev(const unsigned long long* a, long long na, const unsigned lo
     // scratch: split operands and products, prime by prime
     const BigSizes z = big_sizes(pl, na, nb);
     const int dev = current_device();
-    u32* w32 = bufs ? bufs->eval : (u32*)workspace(dev, kWsBig, z.words * 4, &err);
+    std::optional<Workspace> space;
+    if (!bufs) space.emplace(dev, kWsBig, z.words * 4, st, &err);
+    u32* w32 = bufs ? bufs->eval : space->get();
     if (!w32) return err;
     u32 *ap[kBigMaxPrimes], *bp[kBigMaxPrimes], *cp[kBigMaxPrimes];
     for (int k = 0; k < r; ++k) {
@@ -727,7 +730,8 @@ cumodp_err cumodp_twoconv_mul_big(long long na, const uint64_t* a, long long nb,
     const long long lc = na + nb - 1;
     int err = OK;
     const size_t in_bytes = (size_t)(na + nb) * in_words * 8, out_bytes = (size_t)lc * out_words * 8;
-    char* d = (char*)workspace(dev, kWsStage, in_bytes + out_bytes, &err);
+    const Workspace d_space(dev, kWsStage, in_bytes + out_bytes, st, &err);
+    char* d = d_space.get<char>();
     if (!d) return (cumodp_err)err;
     unsigned long long* da = (unsigned long long*)d;
     unsigned long long* db = da + (size_t)na * in_words;

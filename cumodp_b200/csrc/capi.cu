@@ -129,7 +129,8 @@ cumodp_err cumodp_fftmul_uni(sfixn dh, sfixn* H, sfixn df, const sfixn* F, sfixn
         }
         return to_err(err);
     }
-    u32* d = (u32*)workspace(dev, kWsStage, (la + lb + lh) * sizeof(u32), &err);
+    const Workspace d_space(dev, kWsStage, (la + lb + lh) * sizeof(u32), st, &err);
+    u32* d = d_space.get();
     if (!d) return to_err(err);
     u32 *dA = d, *dB = d + la, *dH = d + la + lb;
     cudaError_t ce = cudaMemcpyAsync(dA, F, la * 4, cudaMemcpyHostToDevice, st);

@@ -75,7 +75,8 @@ int grid_mul_dev(u32* F, u32* G, int em, int en, u32 p, cudaStream_t st) {
     const int dev = current_device(), l2 = E + en;
     const long long words = 1ll << (em + en);
     if ((err = ensure_kernel_attrs(dev)) != OK) return err;
-    u32* ws = (u32*)workspace(dev, kWsBiv, (size_t)2 * words * sizeof(u32), &err);
+    const Workspace ws_space(dev, kWsBiv, (size_t)2 * words * sizeof(u32), st, &err);
+    u32* ws = ws_space.get();
     if (!ws) return err;
     const u32 wm = canonical_root(*pc, em), wn = canonical_root(*pc, en), wc = canonical_root(*pc, l1);
     const u32 ninv = powmod_exact((u32)(words % p), p - 2, p), scale = mulmod_exact(ninv, pc->info.r1, p);

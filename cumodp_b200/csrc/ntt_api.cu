@@ -283,7 +283,8 @@ int ntt_split_dev(const PrimeCtx& pc, const u32* x_in, u32* x_out, int k, u32 ro
     const int dev = current_device();
     const u32* seeds = seed_tables(dev, p, root, k, &err);
     if (!seeds) return err ? err : OUT_OF_MEMORY;
-    u32* S = (u32*)workspace(dev, kWsSplitNtt + (k - kMaxLog - 1), (size_t)n * sizeof(u32), &err);
+    const Workspace S_space(dev, kWsSplitNtt + (k - kMaxLog - 1), (size_t)n * sizeof(u32), st, &err);
+    u32* S = S_space.get();
     if (!S) return err;
     const int grid = 4 * sm_count(dev);
     k_split_dif<<<grid, 256, 0, st>>>(x_in, x_out, h, seeds, (int)std::min<long long>(n, 4096), pc.pk,
@@ -318,7 +319,8 @@ int ntt_natural_dev(const u32* x_in, u32* x_out, int k, u32 w, u32 p, bool inver
     if (k <= kMaxSmallLog) return row_nat(*pc, x_in, x_out, 1, k, root, sc, 0, dev, st);
     const int l1 = std::max(5, k - kMaxRowLog), l2 = k - l1;
     const long long n = 1ll << k;
-    u32* ws = (u32*)workspace(dev, kWsNtt, (size_t)2 * n * sizeof(u32), &err);
+    const Workspace ws_space(dev, kWsNtt, (size_t)2 * n * sizeof(u32), st, &err);
+    u32* ws = ws_space.get();
     if (!ws) return err;
     u32 *w1 = ws, *w2 = ws + n;
     const u32 root_c = powmod_exact(root, 1ull << l2, p);
@@ -343,9 +345,11 @@ int list_ntt_four_step(const PrimeCtx& pc, u32* x, long long m, int k, u32 root,
     const int l1 = std::max(5, k - kMaxRowLog), l2 = k - l1;
     const long long n = 1ll << k;
     const long long cm = std::min<long long>(m, std::max<long long>(1, std::min<long long>(65535, (1ll << 26) >> k)));
-    u32* ws = (u32*)workspace(dev, kWsNtt, (size_t)2 * cm * n * sizeof(u32), &err);
+    const Workspace ws_space(dev, kWsNtt, (size_t)2 * cm * n * sizeof(u32), st, &err);
+    u32* ws = ws_space.get();
     if (!ws) return err;
-    LargeJob* dj = (LargeJob*)workspace(dev, kWsListJobs, (size_t)cm * sizeof(LargeJob), &err);
+    const Workspace dj_space(dev, kWsListJobs, (size_t)cm * sizeof(LargeJob), st, &err);
+    LargeJob* dj = dj_space.get<LargeJob>();
     if (!dj) return err;
     u32 *w1 = ws, *w2 = ws + cm * n;
     const u32 root_c = powmod_exact(root, 1ull << l2, p);
@@ -427,7 +431,8 @@ int bivariate_general(u32* x, int em, u32 wm, int en, u32 wn, u32 p, bool invers
     const long long rows = 1ll << em, cols = 1ll << en;
     if ((err = list_ntt_dev(x, rows, en, wn, p, inverse, st)) != OK) return err;
     if (em == 0) return OK;
-    u32* t = (u32*)workspace(current_device(), kWsBivT, (size_t)(rows * cols) * sizeof(u32), &err);
+    const Workspace t_space(current_device(), kWsBivT, (size_t)(rows * cols) * sizeof(u32), st, &err);
+    u32* t = t_space.get();
     if (!t) return err;
     transpose_long(x, t, rows, cols, st);
     if ((err = list_ntt_dev(t, cols, em, wm, p, inverse, st)) != OK) return err;
@@ -453,7 +458,8 @@ int bivariate_dev(u32* x, int em, u32 wm, int en, u32 wn, u32 p, bool inverse, c
     const u32 sc = inverse ? inv_of((u32)((1ull << (em + en)) % p), p) : 1u;
     const long long total = 1ll << (em + en);
     if (em == 0) return row_nat(*pc, x, x, 1, en, rn, sc, 0, dev, st);
-    u32* w1 = (u32*)workspace(dev, kWsNtt, (size_t)total * sizeof(u32), &err);
+    const Workspace w1_space(dev, kWsNtt, (size_t)total * sizeof(u32), st, &err);
+    u32* w1 = w1_space.get();
     if (!w1) return err;
     if ((err = column_pass(*pc, rm, em, en, x, total, w1, dev, st)) != OK) return err;
     return row_nat(*pc, w1, x, 1ll << em, en, rn, sc, em, dev, st);
@@ -500,7 +506,8 @@ int cyclic_mul_compose(u32* f, const u32* g, int e, u32 p, cudaStream_t st) {
     if (!pc) return err;
     const long long n = 1ll << e;
     const u32 w = canonical_root(*pc, e);
-    u32* gt = (u32*)workspace(current_device(), kWsCyclic, (size_t)n * sizeof(u32), &err);
+    const Workspace gt_space(current_device(), kWsCyclic, (size_t)n * sizeof(u32), st, &err);
+    u32* gt = gt_space.get();
     if (!gt) return err;
     if ((err = ntt_natural_dev(g, gt, e, w, p, false, st)) != OK) return err;
     if ((err = ntt_natural_dev(f, f, e, w, p, false, st)) != OK) return err;
@@ -543,7 +550,8 @@ int bivariate_mul_dev(u32* F, u32* G, int em, int en, u32 p, cudaStream_t st) {
     }
     const int dev = current_device();
     const long long tpad = (total + 3) & ~3ll;  // 16-byte aligned halves
-    u32* ws = (u32*)workspace(dev, kWsBiv, (size_t)2 * tpad * sizeof(u32), &err);
+    const Workspace ws_space(dev, kWsBiv, (size_t)2 * tpad * sizeof(u32), st, &err);
+    u32* ws = ws_space.get();
     if (!ws) return err;
     u32 *W1 = ws, *W2 = ws + tpad;
     u32* src[2] = {F, G};
@@ -572,7 +580,8 @@ int bivariate_product_dev(const u32* F, int nxf, int nyf, const u32* G, int nxg,
     if (ex + ey > 30) return FFT_SIZE_TOO_LARGE;
     const long long total = 1ll << (ex + ey);
     const long long tpad = (total + 3) & ~3ll;  // 16-byte aligned halves
-    u32* ws = (u32*)workspace(current_device(), kWsBivHost, (size_t)2 * tpad * sizeof(u32), &err);
+    const Workspace ws_space(current_device(), kWsBivHost, (size_t)2 * tpad * sizeof(u32), st, &err);
+    u32* ws = ws_space.get();
     if (!ws) return err;
     u32 *F2 = ws, *G2 = ws + tpad;
     k_expand2<<<grid_for(total), 256, 0, st>>>(F, nxf, nyf, F2, ex, ey, p);
@@ -599,7 +608,8 @@ cumodp_err host_ntt(sfixn* X, sfixn n, sfixn k, sfixn w, sfixn p, bool inverse) 
     const int dev = current_device();
     cudaStream_t st = lib_stream(dev);
     int err = OK;
-    u32* d = (u32*)workspace(dev, kWsStage, (size_t)n * sizeof(u32), &err);
+    const Workspace d_space(dev, kWsStage, (size_t)n * sizeof(u32), st, &err);
+    u32* d = d_space.get();
     if (!d) return (cumodp_err)err;
     cudaError_t ce = cudaMemcpyAsync(d, X, (size_t)n * 4, cudaMemcpyHostToDevice, st);
     if (ce != cudaSuccess) return (cumodp_err)cuda_err(ce);
@@ -625,7 +635,8 @@ cumodp_err host_bivariate(sfixn* X, sfixn em, sfixn wm, sfixn en, sfixn wn, sfix
     cudaStream_t st = lib_stream(dev);
     const size_t total = (size_t)1 << (em + en);
     int err = OK;
-    u32* d = (u32*)workspace(dev, kWsStage, total * sizeof(u32), &err);
+    const Workspace d_space(dev, kWsStage, total * sizeof(u32), st, &err);
+    u32* d = d_space.get();
     if (!d) return (cumodp_err)err;
     cudaError_t ce = cudaMemcpyAsync(d, X, total * 4, cudaMemcpyHostToDevice, st);
     if (ce != cudaSuccess) return (cumodp_err)cuda_err(ce);
@@ -715,7 +726,8 @@ cumodp_err cumodp_bivariate_mul(sfixn nxf, sfixn nyf, const sfixn* F, sfixn nxg,
     const int dev = current_device();
     cudaStream_t st = lib_stream(dev);
     int err = OK;
-    u32* d = (u32*)workspace(dev, kWsStage, (size_t)(nf + ng + nh) * sizeof(u32), &err);
+    const Workspace d_space(dev, kWsStage, (size_t)(nf + ng + nh) * sizeof(u32), st, &err);
+    u32* d = d_space.get();
     if (!d) return (cumodp_err)err;
     cudaError_t ce = cudaMemcpyAsync(d, F, nf * 4, cudaMemcpyHostToDevice, st);
     if (ce == cudaSuccess) ce = cudaMemcpyAsync(d + nf, G, ng * 4, cudaMemcpyHostToDevice, st);

@@ -5,6 +5,7 @@
 #include <algorithm>
 #include <map>
 #include <mutex>
+#include <optional>
 #include <tuple>
 #include <cstdlib>
 #include <cstring>
@@ -402,8 +403,10 @@ int mul_split_dev(const u32* a, long long la, const u32* b, long long lb, u32* h
     const int dev = current_device();
     int err = OK;
     auto overlaps = [&](const u32* x, long long lx) { return x < h + lh && h < x + lx; };
+    std::optional<Workspace> copy;
     if (overlaps(a, la) || overlaps(b, lb)) {
-        u32* in = (u32*)workspace(dev, kWsSplitIn, (size_t)(la + lb) * sizeof(u32), &err);
+        copy.emplace(dev, kWsSplitIn, (size_t)(la + lb) * sizeof(u32), st, &err);
+        u32* in = copy->get();
         if (!in) return err;
         cudaError_t e = cudaMemcpyAsync(in, a, (size_t)la * sizeof(u32), cudaMemcpyDeviceToDevice, st);
         if (e == cudaSuccess)
@@ -412,7 +415,8 @@ int mul_split_dev(const u32* a, long long la, const u32* b, long long lb, u32* h
         a = in;
         b = in + la;
     }
-    u32* t = (u32*)workspace(dev, kWsSplitProd, (size_t)(2 * C) * sizeof(u32), &err);
+    const Workspace t_space(dev, kWsSplitProd, (size_t)(2 * C) * sizeof(u32), st, &err);
+    u32* t = t_space.get();
     if (!t) return err;
     cudaError_t e = cudaMemsetAsync(h, 0, (size_t)lh * sizeof(u32), st);
     if (e != cudaSuccess) return cuda_err(e);
@@ -465,7 +469,8 @@ int mul_dev_len(const u32* a, long long la, const u32* b, long long lb, u32* h, 
         const int l2 = default_row_log(logn);
         LargeArgs A;
         if ((err = large_args(pc, root, logn, l2, dev, &A)) != OK) return err;
-        u32* ws = (u32*)workspace(dev, kWsSingle, (size_t)2 * n * sizeof(u32), &err);
+        const Workspace ws_space(dev, kWsSingle, (size_t)2 * n * sizeof(u32), st, &err);
+        u32* ws = ws_space.get();
         if (!ws) return err;
         A.job0 = LargeJob{a, b, h, (int)la, (int)lb, (int)lh, 0, ws, ws + n};
         A.njobs = 1;

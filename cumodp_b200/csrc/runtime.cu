@@ -12,6 +12,7 @@
 #include "latency_product.cuh"
 #include "row_natural.cuh"
 
+#include <algorithm>
 #include <atomic>
 #include <cstdio>
 #include <map>
@@ -56,9 +57,16 @@ struct Caches {
     std::map<u32, PrimeCtx*> primes;
     std::map<std::tuple<int, u32, u32, int, int>, Tw*> tables;  // dev, p, root, logl, kind
     std::map<std::tuple<int, u32, u32, int>, u32*> seeds;
-    std::map<std::pair<int, int>, std::pair<void*, size_t>> ws;
+    struct Slot {
+        void *p = nullptr, *retired = nullptr;  // retired: the copy the first stream's calls may still use
+        size_t bytes = 0, retired_bytes = 0;
+        StreamOrder order;
+    };
+    std::map<std::pair<int, int>, Slot> ws;
     std::map<int, std::pair<void*, size_t>> pinned;
     std::map<int, cudaStream_t> streams;
+    std::mutex own_m;
+    std::vector<cudaStream_t> own;  // streams that live as long as the process
 };
 
 Caches& caches() {
@@ -492,27 +500,122 @@ const u32* seed_tables(int dev, u32 p, u32 root, int logn, int* err) {
     return d;
 }
 
-void* workspace(int dev, int slot, size_t bytes, int* err) {
+namespace {
+
+bool own_stream(cudaStream_t st) {
+    Caches& C = caches();
+    std::lock_guard<std::mutex> g(C.own_m);
+    return std::find(C.own.begin(), C.own.end(), st) != C.own.end();
+}
+void keep_stream(cudaStream_t st) {
+    Caches& C = caches();
+    std::lock_guard<std::mutex> g(C.own_m);
+    C.own.push_back(st);
+}
+
+}  // namespace
+
+int StreamOrder::mark(cudaStream_t st) {
+    cudaError_t e = cudaSuccess;
+    if (!ev_) e = cudaEventCreateWithFlags(&ev_, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventRecord(ev_, st);
+    if (e != cudaSuccess) {  // nothing to wait for later: wait now
+        cudaGetLastError();
+        e = cudaStreamSynchronize(st);
+        used_ = e != cudaSuccess;
+        return cuda_err(e);
+    }
+    marked_ = true;
+    return OK;
+}
+
+int StreamOrder::enter(cudaStream_t st, bool* replace) {
+    if (replace) *replace = false;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    // (the legacy stream answers with an error while a blocking stream is captured)
+    skip_ = cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone;
+    if (skip_) {
+        cudaGetLastError();
+        return OK;
+    }
+    cudaError_t e = cudaStreamGetId(st, &id_);
+    if (e == cudaSuccess && replace && used_ && id_ != last_) {
+        if (!marked_ && own_stream(last_stream_)) {
+            const int err = mark(last_stream_);
+            if (err != OK) return err;
+        }
+        if (used_ && marked_) e = cudaStreamWaitEvent(st, ev_, 0);
+        else *replace = used_;
+    }
+    if (e != cudaSuccess) cudaGetLastError();
+    return cuda_err(e);
+}
+
+void StreamOrder::fresh() {
+    used_ = marked_ = false;
+    shared_ = true;
+}
+
+void StreamOrder::leave(cudaStream_t st) {
+    if (skip_) return;
+    used_ = true;
+    marked_ = false;
+    last_ = id_;
+    last_stream_ = st;
+    if (shared_ && !own_stream(st)) mark(st);
+}
+
+StreamOrder::~StreamOrder() {
+    if (ev_) cudaEventDestroy(ev_);
+}
+
+Workspace::Workspace(int dev, int slot, size_t bytes, cudaStream_t st, int* err) : st_(st) {
     Caches& C = caches();
     std::lock_guard<std::mutex> g(C.m);
     auto& e = C.ws[std::make_pair(dev, slot)];
-    if (e.second >= bytes && e.first) return e.first;
-    if (e.first) {
-        cudaFree(e.first);
-        C.bytes -= (long long)e.second;
+    if (e.bytes < bytes || !e.p) {
+        // (cudaFree waits for the device: nothing queued uses the buffer any more)
+        if (e.p) cudaFree(e.p);
+        if (e.retired) cudaFree(e.retired);
+        C.bytes -= (long long)(e.bytes + e.retired_bytes);
+        e.p = e.retired = nullptr;
+        e.bytes = e.retired_bytes = 0;
+        e.order.idle();
+        const size_t sz = bytes < 4096 ? 4096 : bytes;
+        if (dev_malloc(&e.p, sz) != cudaSuccess) {
+            cudaGetLastError();
+            *err = OUT_OF_MEMORY;
+            e.p = nullptr;
+            return;
+        }
+        e.bytes = sz;
+        C.bytes += (long long)sz;
     }
-    e.first = nullptr;
-    e.second = 0;
-    size_t sz = bytes < 4096 ? 4096 : bytes;
-    if (dev_malloc(&e.first, sz) != cudaSuccess) {
-        cudaGetLastError();
-        *err = OUT_OF_MEMORY;
-        e.first = nullptr;
-        return nullptr;
+    bool replace = false;
+    int oe = e.order.enter(st, &replace);
+    if (oe == OK && replace) {
+        void* n = nullptr;
+        if (dev_malloc(&n, e.bytes) == cudaSuccess) {
+            e.retired = e.p;  // once in a slot's life between two growths: calls are marked from here on
+            e.retired_bytes = e.bytes;
+            C.bytes += (long long)e.bytes;
+            e.p = n;
+        } else {
+            cudaGetLastError();
+            oe = cuda_err(cudaDeviceSynchronize());
+        }
+        if (oe == OK) e.order.fresh();
     }
-    e.second = sz;
-    C.bytes += (long long)sz;
-    return e.first;
+    if (oe != OK) {
+        *err = oe;
+        return;
+    }
+    p_ = e.p;
+    order_ = &e.order;
+}
+
+Workspace::~Workspace() {
+    if (order_) order_->leave(st_);
 }
 
 void* pinned_workspace(int slot, size_t bytes, int* err) {
@@ -542,6 +645,7 @@ cudaStream_t lib_stream(int dev) {
     cudaStream_t s;
     cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
     C.streams[dev] = s;
+    keep_stream(s);
     return s;
 }
 
@@ -562,6 +666,7 @@ static AuxSet& aux_set(int dev) {
     AuxSet* a = new AuxSet();
     for (int i = 0; i < kAuxStreams; ++i) {
         cudaStreamCreateWithFlags(&a->s[i], cudaStreamNonBlocking);
+        keep_stream(a->s[i]);
         cudaEventCreateWithFlags(&a->join[i], cudaEventDisableTiming);
     }
     cudaEventCreateWithFlags(&a->fork, cudaEventDisableTiming);

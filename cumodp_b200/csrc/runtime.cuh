@@ -83,9 +83,56 @@ int level_tables_into(int kind, u32 p, u32 root, int logl, Tw* out, size_t cap);
 size_t seed_words(int logn);
 int seeds_into(u32 p, u32 root, int logn, u32* out, size_t cap);
 
-// Per-device scratch that grows on demand (never shrinks while the process
-// lives).  Each call site names a slot so concurrent users do not collide.
-void* workspace(int dev, int slot, size_t bytes, int* err);
+// Orders the users of something shared (a scratch buffer, a job table) that
+// come on different streams.  enter() makes st follow the user before, leave()
+// marks where this one's work on st ends.  A stream needs no wait for itself
+// (streams are told apart by their id, which a destroyed stream's handle does
+// not carry on), and a program with one stream pays nothing: an event after
+// every call cost the calls of 17-40 us on one stream 0.5-1.5 us each.  So the
+// first user's calls are not marked, and when another stream comes they cannot
+// be waited for any more (their stream may be gone): enter() then sets
+// *replace, the caller gives st another copy of the thing (or waits for the
+// device) and says fresh(); from then on every call is marked.  Marks on the
+// library's own streams are made when they are needed.
+// Work being captured into a graph is left alone (it runs when the graph is
+// launched, which is the caller's to order).  The caller holds lib_mutex from
+// enter() to leave(); the device of st is current.
+class StreamOrder {
+public:
+    int enter(cudaStream_t st, bool* replace);  // replace null: nothing to wait for
+    void fresh();                               // a new copy, or an idle device: in use by several streams
+    void idle() { used_ = false; }              // nothing queued uses it any more
+    void leave(cudaStream_t st);
+    ~StreamOrder();
+
+private:
+    int mark(cudaStream_t st);
+    cudaEvent_t ev_ = nullptr;
+    bool used_ = false, marked_ = false, shared_ = false, skip_ = false;
+    unsigned long long last_ = 0, id_ = 0;  // stream ids of the last user and of the present one
+    cudaStream_t last_stream_ = nullptr;    // looked at only when it is the library's
+};
+
+// Per-device scratch of one call on stream st: each slot is one buffer that
+// grows on demand (and never shrinks while the process lives).  Each call site
+// names a slot, so nested users do not collide, and calls on different streams
+// are ordered (StreamOrder) for as long as the object lives: it is declared
+// before the first work on the buffer is queued and goes out of scope when all
+// of it is on st.  get() is null, and *err set, when it cannot be had.
+class Workspace {
+public:
+    Workspace(int dev, int slot, size_t bytes, cudaStream_t st, int* err);
+    ~Workspace();
+    Workspace(const Workspace&) = delete;
+    Workspace& operator=(const Workspace&) = delete;
+    template <class T = u32>
+    T* get() const { return (T*)p_; }
+
+private:
+    void* p_ = nullptr;
+    StreamOrder* order_ = nullptr;
+    cudaStream_t st_;
+};
 
 // Pinned host staging that grows on demand (shared by every device; the
 // caller holds lib_mutex and keeps no copy from it in flight past its call).

@@ -33,6 +33,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <optional>
 
 #include "../../include/cumodp.h"
 #include "exact.cuh"
@@ -419,7 +420,9 @@ int twoconv_mul_dev(const long long* a, long long la, const long long* b, long l
     const int dev = current_device();
     // workspace: evaluations of a and b, and the products, per prime and point
     const size_t words = (size_t)np * npts * (la + lb + lc);
-    u32* ws = bufs ? bufs->eval : (u32*)workspace(dev, kWsTwoConv, words * sizeof(u32), &err);
+    std::optional<Workspace> space;
+    if (!bufs) space.emplace(dev, kWsTwoConv, words * sizeof(u32), st, &err);
+    u32* ws = bufs ? bufs->eval : space->get();
     if (!ws) return err;
     u32* ea = ws;
     u32* eb = ea + (size_t)np * npts * la;
@@ -593,7 +596,8 @@ cumodp_err cumodp_twoconv_mul_i64(long long na, const int64_t* a, long long nb, 
     const long long lc = na + nb - 1;
     const size_t in_bytes = (size_t)(na + nb) * 8, out_bytes = (size_t)lc * 16;
     int err = OK;
-    long long* d = (long long*)workspace(dev, kWsStage, in_bytes + out_bytes, &err);
+    const Workspace d_space(dev, kWsStage, in_bytes + out_bytes, st, &err);
+    long long* d = d_space.get<long long>();
     if (!d) return (cumodp_err)err;
     // the operands and the result pass through pinned staging: one copy each way
     char* hs = (char*)pinned_workspace(kPinTwoConv, std::max(in_bytes, out_bytes), &err);

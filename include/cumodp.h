@@ -11,6 +11,13 @@
  * odd "Fourier" prime p = c * 2^e + 1 below 2^30.  Unless noted, pointers
  * are HOST pointers and results are complete when the call returns.  All
  * entry points are thread-safe (calls are serialised per process).
+ *
+ * Entry points with a `stream` argument may be called on several streams: the
+ * library's scratch is shared, and a call that uses it waits, on its own
+ * stream, for the call before it on another one (cumodp_fftmul_uni_dev_noalloc
+ * excepted, see there).  Calls captured into a CUDA graph take no part in that
+ * order: launches of the graph must be ordered by the caller against each
+ * other and against calls on other streams.
  */
 #ifndef CUMODP_B200_H
 #define CUMODP_B200_H

@@ -122,7 +122,11 @@ cudaError_t cudaGetLastError(void) { L; const cudaError_t e = g_last; g_last = c
 cudaError_t cudaDeviceSynchronize(void) { L; log_op("devicesync dev %d", g_dev); return cudaSuccess; }
 
 // ---- memory ----
-cudaError_t cudaMalloc(void** p, size_t n) { return (*p = malloc(n)) ? cudaSuccess : ret(cudaErrorMemoryAllocation); }
+cudaError_t cudaMalloc(void** p, size_t n) {
+    L;
+    log_op("malloc bytes %zu", n);
+    return (*p = malloc(n)) ? cudaSuccess : ret(cudaErrorMemoryAllocation);
+}
 cudaError_t cudaMallocAsync(void** p, size_t n, cudaStream_t) { return cudaMalloc(p, n); }
 cudaError_t cudaFree(void* p) { free(p); return cudaSuccess; }
 cudaError_t cudaFreeAsync(void* p, cudaStream_t) { free(p); return cudaSuccess; }

@@ -135,3 +135,138 @@ exact(8192)
 print([int(l.split()[-1]) for l in log() if l.startswith("copy h2d")])
 """)
     assert uploads and max(uploads) <= 1 << 18
+
+
+STREAMS = r"""
+def new_stream():
+    s = ctypes.c_void_p()
+    fake.cudaStreamCreateWithFlags(ctypes.byref(s), 1)
+    return s.value
+
+def fft(k, s):
+    cm.fft_uni_dev(A, k, root(k), P, False, s)
+
+calls = {
+    "product": lambda s: product(18, s),
+    "split_product": lambda s: cm.fftmul_uni_dev(A, 1 << 25, A, (1 << 24), B, 1 << 24, P, s),
+    "cyclic": lambda s: L.cumodp_cyclic_mul_dev(4, ctypes.c_void_p(A), ctypes.c_void_p(B), P, ctypes.c_void_p(s)),
+    "fft": lambda s: fft(18, s),
+    "long_fft": lambda s: fft(26, s),
+    "list": lambda s: cm.list_fft_dev(A, 3, 16, root(16), P, False, s),
+    "fft2d": lambda s: cm.fft_bivariate_dev(A, 6, root(6), 8, root(8), P, False, s),
+    "fft2d_long": lambda s: cm.fft_bivariate_dev(A, 12, root(12), 8, root(8), P, False, s),
+    "bivariate": lambda s: cm.bivariate_mul_dev(8, 8, A, B, P, s),
+    "bivariate_long": lambda s: cm.bivariate_mul_dev(3, 15, A, B, P, s),
+    "exact": lambda s: exact(5000, 0, s),
+    "exact_limbs": lambda s: exact(5000, 1, s),
+    "exact_long": lambda s: exact(300000, 0, s),
+    "big": lambda s: big(64, 8, s),
+    "big_long": lambda s: big(1024, 16, s),
+    "batch": lambda s: batch((1 << 16,) * 2, s),
+    "level": lambda s: cm.subproduct_level_dev(4096, 2, A, H, P, s),
+}
+"""
+
+
+NAMES = ["product", "split_product", "cyclic", "fft", "long_fft", "list", "fft2d", "fft2d_long", "bivariate",
+         "bivariate_long", "exact", "exact_limbs", "exact_long", "big", "big_long", "batch", "level"]
+# these work on the caller's arrays alone
+OWN = {"level": "k_monic_level_fixup", "fft2d_long": "k_row_natILi8E"}
+
+
+def _works(line):
+    return line.startswith(("launch", "graph", "copy", "memset"))
+
+
+def _field(line, what):
+    return line.split(what + " ")[1].split()[0]
+
+
+def _marks(part, s):
+    """Events recorded on stream s after the part's last operation there."""
+    last = max(i for i, x in enumerate(part) if _works(x) and _field(x, "stream") == s)
+    return {_field(x, "event") for x in part[last:] if x.startswith("record") and _field(x, "stream") == s}
+
+
+def _waits(part, s):
+    """Events stream s waits for before any operation of the part."""
+    begin = min(i for i, x in enumerate(part) if _works(x))
+    return {_field(x, "event") for x in part[:begin] if x.startswith("wait") and _field(x, "stream") == s}
+
+
+@pytest.mark.parametrize("name", NAMES)
+def test_calls_on_two_streams_are_ordered_by_their_scratch(fake, name):
+    """A call that uses the library's scratch (or a batch shape's job table) on another stream than the call before
+    it gets scratch of its own the first time; from then on its stream waits for an event recorded after that call's
+    last operation.  A stream does not wait for itself, and one stream alone is not marked."""
+    s1, s2, logs = fake(STREAMS + f"""
+f, name = calls[{name!r}], {name!r}
+s1, s2 = new_stream(), new_stream()
+logs = []
+f(s1)  # tables
+for s in (s1, s2, s1, s2, s2):
+    if name in ("batch", "level"):
+        A, B, H = B, H, A  # other operands: the job table is rewritten
+    fake.fake_set(b"clear", 0)
+    f(s)
+    logs.append(log())
+print([hex(s1), hex(s2), logs])
+""")
+    alone, first, third, fourth, fifth = ([x for x in part if OWN.get(name, "(none)") not in x] for part in logs)
+    if not any("graph" in x for x in alone):  # (side streams fork and join by events)
+        assert not any(x.startswith(("record", "wait")) for x in alone), alone
+    begin = min(i for i, x in enumerate(first) if _works(x))
+    assert any(x.startswith("malloc") for x in first[:begin]), first
+    assert not any(x.startswith("devicesync") for part in logs for x in part)
+    assert _marks(first, s2) & _waits(third, s1), (first, third)
+    assert _marks(third, s1) & _waits(fourth, s2), (third, fourth)
+    assert not _marks(fourth, s2) & _waits(fifth, s2), (fourth, fifth)
+    assert not any(x.startswith("malloc") for part in (third, fourth, fifth) for x in part)
+
+
+@pytest.mark.parametrize("name", ["fft", "bivariate", "exact", "batch"])
+def test_a_second_stream_without_memory_waits_for_the_device(fake, name):
+    """Where the second stream's copy of the scratch cannot be had, the call waits for the device and shares it."""
+    lines = fake(STREAMS + f"""
+f = calls[{name!r}]
+s1, s2 = new_stream(), new_stream()
+f(s1)
+A, B, H = B, H, A
+L.cumodp_inject_alloc_failures(1)
+fake.fake_set(b"clear", 0)
+f(s2)
+print(log())
+""")
+    begin = min(i for i, x in enumerate(lines) if _works(x))
+    assert any(x.startswith("devicesync") for x in lines[:begin]), lines
+
+
+def test_host_calls_and_one_stream_share_scratch_by_marks(fake):
+    """The library's own stream outlives every call, so what runs on it is marked when another stream asks."""
+    lib, s1, logs = fake(STREAMS + """
+x = np.ones(1 << 18, np.int32)
+s1 = new_stream()
+cm.fftmul_uni(x, x, P)
+cm.fftmul_uni(x, x, P)
+lib = [l.split("stream ")[1].split()[0] for l in log() if l.startswith("launch")][-1]
+fake.fake_set(b"clear", 0)
+product(19, s1)
+print([lib, hex(s1), log()])
+""")
+    begin = min(i for i, x in enumerate(logs) if _works(x))
+    marked = {_field(x, "event") for x in logs[:begin] if x.startswith("record") and _field(x, "stream") == lib}
+    assert marked & _waits(logs, s1) and not any(x.startswith("malloc") for x in logs)
+
+
+def test_captured_calls_record_and_wait_for_nothing(fake):
+    """Scratch ordering leaves a stream being captured alone: the graph's launches are the caller's to order."""
+    lines = fake(STREAMS + """
+s1, s2 = new_stream(), new_stream()
+for s in (s1, s2, s1, s2):
+    calls["bivariate"](s)
+fake.cudaStreamBeginCapture(ctypes.c_void_p(s1), 0)
+fake.fake_set(b"clear", 0)
+calls["bivariate"](s1)
+print(log())
+""")
+    assert len(lines) == 4 and all(x.startswith("launch") for x in lines)
