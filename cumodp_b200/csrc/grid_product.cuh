@@ -130,8 +130,8 @@ __global__ void __launch_bounds__(grid_threads(grid_log(E, L2)), grid_ctas(grid_
     constexpr int LT = grid_log(E, L2), T = grid_threads(LT), N = 1 << LT;
     extern __shared__ __align__(16) u32 sm[];
     u32* row = A.wb + (size_t)blockIdx.x * N;
-    pdl_trigger();
     pdl_wait();  // the column pass
+    pdl_trigger();  // after it: k_grid_mul_f reads F's columns before its own wait
     grid_forward<E, L2, LT, T>(sm, row, A);
     for (int r = threadIdx.x; r < N / 32; r += T) {
         u32 x[32];
@@ -155,8 +155,8 @@ __global__ void __launch_bounds__(grid_threads(grid_log(E, L2)), grid_ctas(grid_
     u32* row = A.wa + (size_t)blockIdx.x * N;
     const u32* rowG = A.wb + (size_t)blockIdx.x * N;
     pdl_trigger();
-    // F's forward rows depend only on the column passes, complete before G's
-    // row pass started; G's spectrum is read after pdl_wait
+    // F's forward rows depend only on the column passes, which G's row kernel
+    // waits for before it allows this launch; G's spectrum is read after pdl_wait
     grid_forward<E, L2, LT, T>(sm, row, A);
     pdl_wait();
     for (int r = threadIdx.x; r < N / 32; r += T) {

@@ -736,10 +736,11 @@ __global__ void __launch_bounds__(rowsplit_threads(L2), rowsplit_ctas(L2)) k_row
     const u32 k1 = col_slot_to_k1(s, A.colpl, A.l1);
     const u32 p = A.pk.p, p2 = A.pk.p2;
     u32* row = J.wb + (size_t)s * n2;
-    pdl_trigger();
     if constexpr (RowTab<L2>::USE) row_tab_fetch<L2, T>(tab, wp, A, s, k1, false);
     else row_slot_factors<L2>(A, k1, bf, nullptr);
     pdl_wait();  // pass A's columns of G
+    // after the wait: F's row kernel reads pass A's columns of F before its own
+    pdl_trigger();
     if constexpr (RowTab<L2>::USE) {
         row_level0_fwd<L2, T>(sm, row, A, tab);
     } else {
@@ -785,9 +786,9 @@ __global__ void __launch_bounds__(rowsplit_threads(L2), rowsplit_ctas(L2)) k_row
     const u32* rowG = J.wb + (size_t)s * n2;
     RowCtx ctx{A.pk, A.twr, A.twr_inv};
     pdl_trigger();
-    // F's forward row pass depends only on pass A (complete before the
-    // previous kernel, G's row pass, started), so it runs while that kernel
-    // finishes; G's spectrum is read after pdl_wait
+    // F's forward row pass depends only on pass A, which G's row kernel waits
+    // for before it allows this launch, so it runs while that kernel finishes;
+    // G's spectrum is read after pdl_wait
     if constexpr (RowTab<L2>::USE) {
         row_tab_fetch<L2, T>(tab, wp, A, s, k1, false);
         row_level0_fwd<L2, T>(sm, rowF, A, tab);
