@@ -109,15 +109,25 @@ cumodp_err cumodp_fftmul_uni(sfixn dh, sfixn* H, sfixn df, const sfixn* F, sfixn
     cudaStream_t st = lib_stream(dev);
     const size_t la = (size_t)df + 1, lb = (size_t)dg + 1, lh = (size_t)dh + 1;
     int err = OK;
-    if (product_logn((long long)la, (long long)lb) <= kMaxLatencyLog) {
-        // the one-launch kernels read each operand word once and write each
-        // result word once: they do both in pinned host memory (mapped by
-        // unified addressing), so no copy is queued on either side: 1000 x 1000
-        // coefficients 44 -> 27 us a call, 32768 x 32768 83 -> 62 us (longer
-        // products read their operands more than once and keep the copies)
-        const size_t lc = std::min(lh, la + lb - 1);  // words past the product are zero
-        u32* hs = (u32*)pinned_workspace(kPinMul, (la + lb + lc) * sizeof(u32), &err);
-        if (!hs) return to_err(err);
+    // The one-launch kernels read each operand word once and write each result
+    // word once: they do both in pinned host memory (mapped by unified
+    // addressing), so no copy is queued on either side: 1000 x 1000 coefficients
+    // 44 -> 27 us a call, 32768 x 32768 83 -> 62 us.  Every other product reads
+    // its operands more than once and keeps the copies: longer ones, and any
+    // where the kernel cannot run or pinned memory is short.
+    const size_t lc = std::min(lh, la + lb - 1);  // words past the product are zero
+    const int logn = product_logn((long long)la, (long long)lb);
+    u32* hs = nullptr;
+    if (logn <= kMaxLatencyLog) {
+        const PrimeCtx* pc = prime_ctx((u32)p, &err);
+        if (!pc) return to_err(err);
+        if (logn > pc->info.two_adic) return CUMODP_FFT_SIZE_TOO_LARGE;
+        bool one = false;
+        int pinned_err = OK;
+        if ((err = latency_usable(*pc, logn, dev, &one)) != OK) return to_err(err);
+        if (one) hs = (u32*)pinned_workspace(kPinMul, (la + lb + lc) * sizeof(u32), &pinned_err);
+    }
+    if (hs) {
         memcpy(hs, F, la * sizeof(u32));
         memcpy(hs + la, G, lb * sizeof(u32));
         err = mul_dev(hs, (long long)la, hs + la, (long long)lb, hs + la + lb, (long long)lc, (u32)p, st);

@@ -127,6 +127,13 @@ int prepared(const PrimeCtx& pc, int logn, int dev, Prepared* out) {
 
 }  // namespace
 
+int latency_usable(const PrimeCtx& pc, int logn, int dev, bool* usable) {
+    Prepared P{};
+    const int err = prepared(pc, logn, dev, &P);
+    *usable = err == OK && P.usable;
+    return err;
+}
+
 int latency_mul(const PrimeCtx& pc, int logn, int dev, const ProdJob& job, cudaStream_t st, bool* launched) {
     *launched = false;
     Prepared P;

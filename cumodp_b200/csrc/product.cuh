@@ -49,6 +49,8 @@ void launch_large(const LargeArgs& a, int njobs, cudaStream_t st);
 // at 2^16 the one launch takes 11.5 us and the three-pass kernels 14.8.
 constexpr int kMaxLatencyLog = 16;
 int latency_mul(const PrimeCtx& pc, int logn, int dev, const ProdJob& job, cudaStream_t st, bool* launched);
+// Whether it will run there (its tables are ready then).
+int latency_usable(const PrimeCtx& pc, int logn, int dev, bool* usable);
 // Products of the same lengths mod np (3 or 4) primes: prime r's operands at
 // a + r astride, b + r bstride, its la + lb - 1 residues at h + r hstride.
 int latency_mul_primes(const u32* primes, int np, int dev, const u32* a, int la, long long astride, const u32* b, int lb,

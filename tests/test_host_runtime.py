@@ -270,3 +270,28 @@ calls["bivariate"](s1)
 print(log())
 """)
     assert len(lines) == 4 and all(x.startswith("launch") for x in lines)
+
+
+@pytest.mark.parametrize("what", ["clusters", "pinned_failures"])
+def test_host_products_copy_where_the_one_launch_form_is_not_there(fake, what):
+    """A host product of 2^16 points reads its operands in place only where the one-launch kernel runs and pinned
+    memory is to be had; otherwise its operands are copied to the device, as longer products' are."""
+    fast, slow = fake(f"""
+x = np.ones(30000, np.int32)
+def copies():
+    fake.fake_set(b"clear", 0)
+    cm.fftmul_uni(x, x, P)
+    return [l.split()[1] for l in log() if l.startswith("copy")]
+if {what!r} == "clusters":
+    fake.fake_set(b"clusters", 0)
+    slow = copies(); slow = copies()   # (the first call makes tables)
+    cm.select_device(1)
+    fake.fake_set(b"clusters", 8)
+    fast = copies(); fast = copies()
+else:
+    fake.fake_set(b"pinned_failures", 2)
+    slow = copies(); slow = copies()
+    fast = copies()
+print([fast, slow])
+""")
+    assert fast == [] and sorted(slow) == ["d2h", "h2d", "h2d"]
