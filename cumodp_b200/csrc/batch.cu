@@ -46,7 +46,8 @@ namespace cmb {
 // Results are cached per (device model, kind, logn, job bucket) in memory and,
 // when CUMODP_TUNE_FILE names a file, appended to it and reloaded at start-up;
 // the device model (name, SM count, compute capability) keys the cache, so a
-// file written on one GPU model is not used on another.
+// file written on one GPU model is not used on another, and the number of the
+// kernels it timed, so a file written with other kernels is not used either.
 std::vector<int> legal_row_logs(int logn);
 
 namespace {
@@ -63,13 +64,17 @@ std::mutex g_tune_m;
 std::map<TuneKey, int> g_tune;
 bool g_tune_loaded = false;
 
+// Raised whenever a kernel that the autotuner times is replaced or its plan
+// changes.  1 (not written to files): staged column passes, four-level rows.
+constexpr int kTunedKernels = 2;
+
 int job_bucket(int njobs) {
     int b = 1;
     while (b < njobs && b < 256) b <<= 1;
     return b;
 }
 
-// "name/SMs/sm_major.minor" of device dev (cached).
+// "name/SMs/sm_major.minor/k<kernels>" of device dev (cached).
 const std::string& device_model(int dev) {
     static std::mutex m;
     static std::map<int, std::string> names;
@@ -80,7 +85,8 @@ const std::string& device_model(int dev) {
     std::string key = "unknown";
     if (cudaGetDeviceProperties(&pr, dev) == cudaSuccess) {
         char buf[320];
-        snprintf(buf, sizeof(buf), "%s/%d/sm_%d.%d", pr.name, pr.multiProcessorCount, pr.major, pr.minor);
+        snprintf(buf, sizeof(buf), "%s/%d/sm_%d.%d/k%d", pr.name, pr.multiProcessorCount, pr.major, pr.minor,
+                 kTunedKernels);
         key = buf;
         for (char& c : key)
             if (c == ' ') c = '_';

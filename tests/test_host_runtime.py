@@ -295,3 +295,20 @@ else:
 print([fast, slow])
 """)
     assert fast == [] and sorted(slow) == ["d2h", "h2d", "h2d"]
+
+
+def test_tune_files_of_other_kernels_are_not_used(fake, tmp_path):
+    """A choice in CUMODP_TUNE_FILE counts only for the kernels it was timed with."""
+    f = tmp_path / "tune"
+    f.write_text("0 20 2 14 stand-in/148/sm_10.0\n")  # as written before the key named the kernels
+    code = """
+batch((1 << 19,) * 2)
+print([l for l in log() if l.startswith("launch") and "k_row_mul_f" in l])
+"""
+    timed = fake(code, CUMODP_AUTOTUNE="1", CUMODP_TUNE_FILE=str(f))
+    assert {l2 for l2 in range(9, 15) if any(f"k_row_mul_fILi{l2}E" in x for x in timed)} == set(range(9, 15))
+    lines = f.read_text().splitlines()
+    assert len(lines) == 2
+    again = fake(code, CUMODP_AUTOTUNE="1", CUMODP_TUNE_FILE=str(f))  # and this build's own choice is used
+    assert len({x for x in again}) == 1 and f"k_row_mul_fILi{lines[1].split()[3]}E" in again[0]
+    assert f.read_text().splitlines() == lines
