@@ -531,16 +531,23 @@ int StreamOrder::mark(cudaStream_t st) {
 
 int StreamOrder::enter(cudaStream_t st, bool* replace) {
     if (replace) *replace = false;
+    // one stream alone: nothing to wait for and nothing that leave() would change
+    // (the library's own streams need not be asked for their id)
+    skip_ = used_ && !shared_ && last_own_ && st == last_stream_;
+    if (skip_) return OK;
+    cudaError_t e = cudaStreamGetId(st, &id_);
+    skip_ = e == cudaSuccess && used_ && !shared_ && id_ == last_;
+    if (skip_) return OK;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     // (the legacy stream answers with an error while a blocking stream is captured)
-    skip_ = cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone;
-    if (skip_) {
+    if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) {
         cudaGetLastError();
-        return OK;
+        cs = cudaStreamCaptureStatusActive;
     }
-    cudaError_t e = cudaStreamGetId(st, &id_);
+    skip_ = cs != cudaStreamCaptureStatusNone;
+    if (skip_) return OK;
     if (e == cudaSuccess && replace && used_ && id_ != last_) {
-        if (!marked_ && own_stream(last_stream_)) {
+        if (!marked_ && last_own_) {
             const int err = mark(last_stream_);
             if (err != OK) return err;
         }
@@ -562,7 +569,8 @@ void StreamOrder::leave(cudaStream_t st) {
     marked_ = false;
     last_ = id_;
     last_stream_ = st;
-    if (shared_ && !own_stream(st)) mark(st);
+    last_own_ = own_stream(st);
+    if (shared_ && !last_own_) mark(st);
 }
 
 StreamOrder::~StreamOrder() {

@@ -108,9 +108,10 @@ public:
 private:
     int mark(cudaStream_t st);
     cudaEvent_t ev_ = nullptr;
-    bool used_ = false, marked_ = false, shared_ = false, skip_ = false;
+    bool used_ = false, marked_ = false, shared_ = false, skip_ = false;  // skip_: leave() has nothing to do
     unsigned long long last_ = 0, id_ = 0;  // stream ids of the last user and of the present one
-    cudaStream_t last_stream_ = nullptr;    // looked at only when it is the library's
+    cudaStream_t last_stream_ = nullptr;    // used only when it is the library's (last_own_)
+    bool last_own_ = false;
 };
 
 // Per-device scratch of one call on stream st: each slot is one buffer that
