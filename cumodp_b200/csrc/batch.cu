@@ -68,9 +68,14 @@ bool g_tune_loaded = false;
 // changes.  1 (not written to files): staged column passes, four-level rows.
 constexpr int kTunedKernels = 2;
 
-int job_bucket(int njobs) {
+// The number of products a class of njobs is timed at: its own size rounded up,
+// to a synthetic class of at most 2^25 operand words (512 MiB with workspace).
+// A choice that wins for a few hundred products can lose for thousands: 2^13
+// points take 37.7 us on one CTA each and 35.7 in three passes for 300
+// products, 304 and 389 for 4096.
+int job_bucket(int njobs, int logn) {
     int b = 1;
-    while (b < njobs && b < 256) b <<= 1;
+    while (b < njobs && (long long)b << logn < 1ll << 25) b <<= 1;
     return b;
 }
 
@@ -217,15 +222,13 @@ std::vector<int> legal_row_logs(int logn) {
 int tune_row_log(const PrimeCtx& pc, int logn, int njobs, int dev, cudaStream_t st, bool allow_tuning) {
     const char* off = getenv("CUMODP_AUTOTUNE");
     if (off && off[0] == '0') return default_row_log(logn);
-    const TuneKey key{device_model(dev), 0, logn, job_bucket(njobs)};
+    const TuneKey key{device_model(dev), 0, logn, job_bucket(njobs, logn)};
     int v;
     if (tune_lookup(key, &v)) return v;
     if (!allow_tuning) return default_row_log(logn);
     const std::vector<int> cands = legal_row_logs(logn);
     if (cands.size() <= 1) return cands.empty() ? default_row_log(logn) : cands[0];
-    // timed at the class's own size (its bucket), up to 2^25 operand words: a split that wins for a few
-    // products (many small CTAs) can lose for hundreds
-    const int jobs = std::min(key.bucket, std::max(1, (int)((1ll << 25) >> logn)));
+    const int jobs = key.bucket;
     // a refused launch would count as a slow one
     if (ensure_kernel_attrs(dev) != OK) return default_row_log(logn);
     TuneBufs T(jobs, 1ll << logn, st);
@@ -242,11 +245,11 @@ bool tune_single_cta(const PrimeCtx& pc, int logn, int njobs, int dev, cudaStrea
     if (logn < single_large_min_log() || logn > kMaxSmallLog) return logn <= kMaxSmallLog;
     const char* off = getenv("CUMODP_AUTOTUNE");
     if (off && off[0] == '0') return rule;
-    const TuneKey key{device_model(dev), 1, logn, job_bucket(njobs)};
+    const TuneKey key{device_model(dev), 1, logn, job_bucket(njobs, logn)};
     int v;
     if (tune_lookup(key, &v)) return v != 0;
     if (!allow_tuning) return rule;
-    const int jobs = key.bucket;  // the class's own size (up to 256 products: 64 MiB at 2^14)
+    const int jobs = key.bucket;
     if (ensure_kernel_attrs(dev) != OK) return rule;
     TuneBufs T(jobs, 1ll << logn, st);
     if (!T.ok) return rule;

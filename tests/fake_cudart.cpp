@@ -63,7 +63,7 @@ cudaError_t launch(const void* f, dim3 g, dim3 b, size_t smem, cudaStream_t st) 
         log_op("refused %s dev %d stream %p smem %zu limit %zu", name, g_dev, (void*)st, smem, limit);
         return ret(cudaErrorInvalidValue);
     }
-    log_op("launch %s dev %d stream %p", name, g_dev, (void*)st);
+    log_op("launch %s dev %d grid %u %u %u stream %p", name, g_dev, g.x, g.y, g.z, (void*)st);
     return cudaSuccess;
 }
 
