@@ -86,20 +86,17 @@ __host__ __device__ __forceinline__ u32 col_slot_to_k1(u32 s, const LevelPlan& P
 }
 
 // ------------------------------------------------------ column tiles ----
-// A column CTA owns a tile of TC = col_tile_cols(L1, INV) adjacent columns x n1
-// rows, stored row-major in shared memory (tile_row gives a row's offset).
-// The tile is loaded and stored with 16-byte accesses by all threads at
-// once, so every load of the tile is in flight together; the levels then run
-// on shared memory with lane = column (32-column tiles) or half-warp = task,
-// lane % 16 = column (16-column tiles): conflict-free, and every twiddle is a
-// broadcast to the (half-)warp.
+// A column CTA owns a tile of kColTileCols adjacent columns x n1 rows, stored
+// row-major in shared memory (tile_row gives a row's offset).  The tile is
+// loaded and stored with 16-byte accesses by all threads at once, so every
+// load of the tile is in flight together; the levels then run on shared memory
+// with half-warp = task, lane % 16 = column: conflict-free, and every twiddle
+// is a broadcast to the half-warp.
 
 // Word offset of tile row r.
-template <int L1, int INV>
+template <int L1>
 __host__ __device__ __forceinline__ int tile_row(int r) {
-    constexpr int TC = col_tile_cols(L1, INV);
-    if constexpr (TC == 32) return r * 32;
-    else return (r + (r >> col_pad_log(L1))) * TC;
+    return (r + (r >> col_pad_log(L1))) * kColTileCols;
 }
 
 // tile_row(row0 + TB * m) - tile_row(row0) for element m of a level task
@@ -107,11 +104,10 @@ __host__ __device__ __forceinline__ int tile_row(int r) {
 // the task index): a constant.  Every non-last level of a column plan has TB
 // a multiple of the padding period; the last level has TB = 1 and blocks of
 // exactly one period.
-template <int L1, int INV, int TB>
+template <int L1, int TB>
 __host__ __device__ __forceinline__ constexpr int tile_step(int m) {
-    constexpr int TC = col_tile_cols(L1, INV), PAD = 1 << col_pad_log(L1);
-    if constexpr (TC == 32) return TB * m * 32;
-    else if constexpr (TB % PAD == 0) return TB * m * TC + (TB / PAD) * m * TC;
+    constexpr int TC = kColTileCols, PAD = 1 << col_pad_log(L1);
+    if constexpr (TB % PAD == 0) return TB * m * TC + (TB / PAD) * m * TC;
     else return m * TC;
 }
 
@@ -122,10 +118,10 @@ __host__ __device__ __forceinline__ constexpr int tile_step(int m) {
 // rows entirely past `len` are zero-filled without loads.
 // With ASYNC (and no reduction) the full rows are copied with cp.async,
 // global to shared without a register round trip.
-template <int L1, int INV, int T, bool ASYNC = false>
+template <int L1, int T, bool ASYNC = false>
 __device__ __forceinline__ void tile_load(u32* tile, const u32* __restrict__ src, long long len, int c0, int n2,
                                           bool reduce, const PrimeK& pk) {
-    constexpr int n1 = 1 << L1, TC = col_tile_cols(L1, INV), QR = TC / 4;
+    constexpr int n1 = 1 << L1, TC = kColTileCols, QR = TC / 4;
     constexpr int Q = n1 * QR;  // 16-byte quads in the tile
     const bool vec = ((reinterpret_cast<uintptr_t>(src) & 15) == 0);
     // rows [0, rf) lie fully below len; rows [re, n1) fully at or above it
@@ -136,7 +132,7 @@ __device__ __forceinline__ void tile_load(u32* tile, const u32* __restrict__ src
 #pragma unroll 4
         for (int idx = threadIdx.x; idx < rf * QR; idx += T) {
             const int r = idx / QR, q = idx % QR;
-            const unsigned dst = (unsigned)__cvta_generic_to_shared(tile + tile_row<L1, INV>(r) + 4 * q);
+            const unsigned dst = (unsigned)__cvta_generic_to_shared(tile + tile_row<L1>(r) + 4 * q);
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst),
                          "l"(src + (long long)r * n2 + c0 + 4 * q) : "memory");
         }
@@ -152,7 +148,7 @@ __device__ __forceinline__ void tile_load(u32* tile, const u32* __restrict__ src
             v.z = mul_shoup(v.z, 1u, pk.one_q, pk.p);
             v.w = mul_shoup(v.w, 1u, pk.one_q, pk.p);
         }
-        *reinterpret_cast<uint4*>(tile + tile_row<L1, INV>(r) + 4 * q) = v;
+        *reinterpret_cast<uint4*>(tile + tile_row<L1>(r) + 4 * q) = v;
     }
     for (int idx = rf * QR + threadIdx.x; idx < re * QR; idx += T) {
         const int r = idx / QR, q = idx % QR;
@@ -168,18 +164,18 @@ __device__ __forceinline__ void tile_load(u32* tile, const u32* __restrict__ src
             v.z = mul_shoup(v.z, 1u, pk.one_q, pk.p);
             v.w = mul_shoup(v.w, 1u, pk.one_q, pk.p);
         }
-        *reinterpret_cast<uint4*>(tile + tile_row<L1, INV>(r) + 4 * q) = v;
+        *reinterpret_cast<uint4*>(tile + tile_row<L1>(r) + 4 * q) = v;
     }
     for (int idx = re * QR + threadIdx.x; idx < Q; idx += T)
-        *reinterpret_cast<uint4*>(tile + tile_row<L1, INV>(idx / QR) + 4 * (idx % QR)) = make_uint4(0u, 0u, 0u, 0u);
+        *reinterpret_cast<uint4*>(tile + tile_row<L1>(idx / QR) + 4 * (idx % QR)) = make_uint4(0u, 0u, 0u, 0u);
     if constexpr (ASYNC) asm volatile("cp.async.wait_group 0;\n" ::: "memory");
 }
 
 // Bulk-stores the tile; `final` reduces to [0, p) and stops at `len`.
-template <int L1, int INV, int T>
+template <int L1, int T>
 __device__ __forceinline__ void tile_store(const u32* tile, u32* __restrict__ dst, long long len, int c0, int n2,
                                            bool final, const PrimeK& pk) {
-    constexpr int n1 = 1 << L1, TC = col_tile_cols(L1, INV), QR = TC / 4;
+    constexpr int n1 = 1 << L1, TC = kColTileCols, QR = TC / 4;
     const bool vec = ((reinterpret_cast<uintptr_t>(dst) & 15) == 0);
     const long long lc = len - c0;
     const int rf = vec ? (int)(lc >= TC ? min((long long)n1, (lc - TC) / n2 + 1) : 0) : 0;
@@ -187,7 +183,7 @@ __device__ __forceinline__ void tile_store(const u32* tile, u32* __restrict__ ds
 #pragma unroll 4
     for (int idx = threadIdx.x; idx < rf * QR; idx += T) {
         const int r = idx / QR, q = idx % QR;
-        uint4 v = *reinterpret_cast<const uint4*>(tile + tile_row<L1, INV>(r) + 4 * q);
+        uint4 v = *reinterpret_cast<const uint4*>(tile + tile_row<L1>(r) + 4 * q);
         if (final) {
             v.x = red1(red2(v.x, pk.p2), pk.p);
             v.y = red1(red2(v.y, pk.p2), pk.p);
@@ -199,7 +195,7 @@ __device__ __forceinline__ void tile_store(const u32* tile, u32* __restrict__ ds
     for (int idx = rf * QR + threadIdx.x; idx < re * QR; idx += T) {
         const int r = idx / QR, q = idx % QR;
         const long long gi = (long long)r * n2 + c0 + 4 * q;
-        uint4 v = *reinterpret_cast<const uint4*>(tile + tile_row<L1, INV>(r) + 4 * q);
+        uint4 v = *reinterpret_cast<const uint4*>(tile + tile_row<L1>(r) + 4 * q);
         if (final) {
             v.x = red1(red2(v.x, pk.p2), pk.p);
             v.y = red1(red2(v.y, pk.p2), pk.p);
@@ -213,27 +209,25 @@ __device__ __forceinline__ void tile_store(const u32* tile, u32* __restrict__ ds
     }
 }
 
-// Forward column level LEV, shared memory to shared memory, on a tile of
-// kind KIND (col_tile_cols).
-template <int L1, int LEV, int NW, int KIND = 0>
+// Forward column level LEV, shared memory to shared memory.
+template <int L1, int LEV>
 __device__ __forceinline__ void col_fwd_level(u32* tile, const PrimeK& pk, const Tw* __restrict__ twc) {
     using LV = ColLevel<L1, LEV>;
     constexpr LevelPlan PL = col_plan(L1);
     constexpr int R = LV::R, TB = LV::TB, B = LV::B;
     constexpr bool LAST = LEV + 1 == PL.nlev;
     constexpr int TASKS = (1 << L1) / R;
-    constexpr int INV = KIND;
-    constexpr int TC = col_tile_cols(L1, INV), SUB = 32 / TC;
+    constexpr int TC = kColTileCols, SUB = 32 / TC;
     const u32 p = pk.p, p2 = pk.p2;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int col = lane % TC;
-    for (int id = warp * SUB + lane / TC; id < TASKS; id += NW * SUB) {
+    for (int id = warp * SUB + lane / TC; id < TASKS; id += kColTileWarps * SUB) {
         const int blk = id / TB, o = id % TB;
         const int row0 = blk * B + o;
         u32 x[R];
-        u32* base = tile + tile_row<L1, INV>(row0) + col;
+        u32* base = tile + tile_row<L1>(row0) + col;
 #pragma unroll
-        for (int m = 0; m < R; ++m) x[m] = base[tile_step<L1, INV, TB>(m)];
+        for (int m = 0; m < R; ++m) x[m] = base[tile_step<L1, TB>(m)];
         dif_regs<R, !LAST>(x, pk.rc.f, p, p2);
         if constexpr (!LAST) {
             const Tw* t = twc + LV::TWOFF + o * R;
@@ -244,40 +238,39 @@ __device__ __forceinline__ void col_fwd_level(u32* tile, const PrimeK& pk, const
             }
         }
 #pragma unroll
-        for (int m = 0; m < R; ++m) base[tile_step<L1, INV, TB>(m)] = x[m];
+        for (int m = 0; m < R; ++m) base[tile_step<L1, TB>(m)] = x[m];
     }
 }
 
-template <int L1, int LEV, int NW, int KIND = 0>
+template <int L1, int LEV>
 __device__ __forceinline__ void col_fwd_levels(u32* tile, const PrimeK& pk, const Tw* __restrict__ twc) {
     constexpr LevelPlan PL = col_plan(L1);
     if constexpr (LEV < PL.nlev) {
-        col_fwd_level<L1, LEV, NW, KIND>(tile, pk, twc);
+        col_fwd_level<L1, LEV>(tile, pk, twc);
         __syncthreads();
-        col_fwd_levels<L1, LEV + 1, NW, KIND>(tile, pk, twc);
+        col_fwd_levels<L1, LEV + 1>(tile, pk, twc);
     }
 }
 
 // Inverse column level LEV (pre-twiddle, DIT), shared memory to shared memory.
-template <int L1, int LEV, int NW>
+template <int L1, int LEV>
 __device__ __forceinline__ void col_inv_level(u32* tile, const PrimeK& pk, const Tw* __restrict__ twci) {
     using LV = ColLevel<L1, LEV>;
     constexpr LevelPlan PL = col_plan(L1);
     constexpr int R = LV::R, TB = LV::TB, B = LV::B;
     constexpr bool DEEPEST = LEV + 1 == PL.nlev;
     constexpr int TASKS = (1 << L1) / R;
-    constexpr int INV = 1;
-    constexpr int TC = col_tile_cols(L1, INV), SUB = 32 / TC;
+    constexpr int TC = kColTileCols, SUB = 32 / TC;
     const u32 p = pk.p, p2 = pk.p2;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int col = lane % TC;
-    for (int id = warp * SUB + lane / TC; id < TASKS; id += NW * SUB) {
+    for (int id = warp * SUB + lane / TC; id < TASKS; id += kColTileWarps * SUB) {
         const int blk = id / TB, o = id % TB;
         const int row0 = blk * B + o;
         u32 x[R];
-        u32* base = tile + tile_row<L1, INV>(row0) + col;
+        u32* base = tile + tile_row<L1>(row0) + col;
 #pragma unroll
-        for (int m = 0; m < R; ++m) x[m] = base[tile_step<L1, INV, TB>(m)];
+        for (int m = 0; m < R; ++m) x[m] = base[tile_step<L1, TB>(m)];
         if constexpr (!DEEPEST) {
             const Tw* t = twci + LV::TWOFF + o * R;
 #pragma unroll
@@ -288,23 +281,22 @@ __device__ __forceinline__ void col_inv_level(u32* tile, const PrimeK& pk, const
         }
         dit_regs<R, !DEEPEST>(x, pk.rc.i, p, p2);
 #pragma unroll
-        for (int m = 0; m < R; ++m) base[tile_step<L1, INV, TB>(m)] = x[m];
+        for (int m = 0; m < R; ++m) base[tile_step<L1, TB>(m)] = x[m];
     }
 }
 
-template <int L1, int LEV, int NW>
+template <int L1, int LEV>
 __device__ __forceinline__ void col_inv_levels(u32* tile, const PrimeK& pk, const Tw* __restrict__ twci) {
     if constexpr (LEV >= 0) {
-        col_inv_level<L1, LEV, NW>(tile, pk, twci);
+        col_inv_level<L1, LEV>(tile, pk, twci);
         __syncthreads();
-        col_inv_levels<L1, LEV - 1, NW>(tile, pk, twci);
+        col_inv_levels<L1, LEV - 1>(tile, pk, twci);
     }
 }
 
-// pass A, grid: (n2/TC column tiles, operands, jobs); KIND 0 for a product's
-// operands, 2 for the forward pass of a natural-order transform
-template <int L1, int NW, int KIND = 0>
-__global__ void __launch_bounds__(NW * 32, col_ctas(L1, KIND)) k_col_fwd(const __grid_constant__ LargeArgs A) {
+// pass A, grid: (n2/TC column tiles, operands, jobs)
+template <int L1>
+__global__ void __launch_bounds__(kColTileWarps * 32, 1) k_col_fwd(const __grid_constant__ LargeArgs A) {
     extern __shared__ __align__(16) u32 tile[];
     const LargeJob& J = A.jobs ? A.jobs[blockIdx.z] : A.job0;
     const int op = blockIdx.y;
@@ -312,33 +304,33 @@ __global__ void __launch_bounds__(NW * 32, col_ctas(L1, KIND)) k_col_fwd(const _
     const int len = op ? J.lb : J.la;
     u32* dst = op ? J.wb : J.wa;
     const int n2 = 1 << A.l2;
-    const int c0 = blockIdx.x * col_tile_cols(L1, KIND);
+    const int c0 = blockIdx.x * kColTileCols;
     // the plan's twiddles (broadcast reads) next to the tile
     constexpr int NTW = col_tw_entries(L1);
-    Tw* tws = reinterpret_cast<Tw*>(tile + col_tile_words(L1, KIND));
-    for (int i = threadIdx.x; i < NTW; i += NW * 32) tws[i] = A.twc[i];
+    Tw* tws = reinterpret_cast<Tw*>(tile + col_tile_words(L1));
+    for (int i = threadIdx.x; i < NTW; i += kColTileWarps * 32) tws[i] = A.twc[i];
     // reduced while loaded (an input row half made of padding costs nothing)
-    tile_load<L1, KIND, NW * 32>(tile, src, len, c0, n2, true, A.pkc);
+    tile_load<L1, kColTileWarps * 32>(tile, src, len, c0, n2, true, A.pkc);
     __syncthreads();
-    col_fwd_levels<L1, 0, NW, KIND>(tile, A.pkc, tws);
-    tile_store<L1, KIND, NW * 32>(tile, dst, 1ll << (L1 + A.l2), c0, n2, false, A.pkc);
+    col_fwd_levels<L1, 0>(tile, A.pkc, tws);
+    tile_store<L1, kColTileWarps * 32>(tile, dst, 1ll << (L1 + A.l2), c0, n2, false, A.pkc);
 }
 
 // pass C, grid: (n2/TC column tiles, 1, jobs)
-template <int L1, int NW>
-__global__ void __launch_bounds__(NW * 32, col_ctas(L1, true)) k_col_inv(const __grid_constant__ LargeArgs A) {
+template <int L1>
+__global__ void __launch_bounds__(kColTileWarps * 32, 1) k_col_inv(const __grid_constant__ LargeArgs A) {
     extern __shared__ __align__(16) u32 tile[];
     const LargeJob& J = A.jobs ? A.jobs[blockIdx.z] : A.job0;
     const int n2 = 1 << A.l2;
-    const int c0 = blockIdx.x * col_tile_cols(L1, true);
+    const int c0 = blockIdx.x * kColTileCols;
     constexpr int NTW = col_tw_entries(L1);
-    Tw* tws = reinterpret_cast<Tw*>(tile + col_tile_words(L1, true));
-    for (int i = threadIdx.x; i < NTW; i += NW * 32) tws[i] = A.twc[A.twc_inv + i];
+    Tw* tws = reinterpret_cast<Tw*>(tile + col_tile_words(L1));
+    for (int i = threadIdx.x; i < NTW; i += kColTileWarps * 32) tws[i] = A.twc[A.twc_inv + i];
     pdl_wait();  // pass B's output
-    tile_load<L1, true, NW * 32, true>(tile, J.wa, 1ll << (L1 + A.l2), c0, n2, false, A.pkc);
+    tile_load<L1, kColTileWarps * 32, true>(tile, J.wa, 1ll << (L1 + A.l2), c0, n2, false, A.pkc);
     __syncthreads();
-    col_inv_levels<L1, col_plan(L1).nlev - 1, NW>(tile, A.pkc, tws);
-    tile_store<L1, true, NW * 32>(tile, J.h, J.lh, c0, n2, true, A.pkc);
+    col_inv_levels<L1, col_plan(L1).nlev - 1>(tile, A.pkc, tws);
+    tile_store<L1, kColTileWarps * 32>(tile, J.h, J.lh, c0, n2, true, A.pkc);
 }
 
 // ------------------------------------------------------------- pass B ----

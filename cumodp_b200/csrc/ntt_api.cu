@@ -168,16 +168,6 @@ int rows_and_transpose(const PrimeCtx& pc, const u32* w1, u32* w2, u32* out, int
     return cuda_err(cudaGetLastError());
 }
 
-// Forward-column launchers shared with the product path (single operand).
-template <int L1>
-int launch_colfwd1_t(const LargeArgs& a, int tiles, int dev, cudaStream_t st) {
-    constexpr size_t smem = col_smem_bytes(L1, 2);
-    static DeviceOnce once;
-    const int err = once(dev, [] { return allow_smem(k_col_fwd<L1, col_warps(L1, 2), 2>, smem); });
-    if (err != OK) return err;
-    k_col_fwd<L1, col_warps(L1, 2), 2><<<dim3(tiles, 1, a.njobs), col_warps(L1, 2) * 32, smem, st>>>(a);
-    return OK;
-}
 // w is a primitive 2^k-th root of unity mod p.
 bool root_has_order(u32 w, int k, u32 p) {
     if (w == 0 || w >= p) return false;
@@ -206,8 +196,8 @@ int column_pass(const PrimeCtx& pc, u32 root_c, int l1, int l2, const u32* src, 
     A.jobs = djobs;  // a device job table (a list of transforms), or nullptr: job0
     A.njobs = njobs;
     if ((err = ensure_kernel_attrs(dev)) != OK) return err;
-    if (launch_col_fwd1(A, njobs, st)) return OK;
-    return launch_colfwd1_t<kMaxColLog>(A, (1 << l2) / col_tile_cols(kMaxColLog, 2), dev, st);
+    launch_col_fwd1(A, njobs, st);
+    return OK;
 }
 
 // First radix-2 (decimation-in-frequency) step of a transform of n = 2h
@@ -317,6 +307,7 @@ int ntt_natural_dev(const u32* x_in, u32* x_out, int k, u32 w, u32 p, bool inver
         return cuda_err(cudaGetLastError());
     }
     if (k <= kMaxSmallLog) return row_nat(*pc, x_in, x_out, 1, k, root, sc, 0, dev, st);
+    // the longest rows, and columns for the rest (no other split has been timed)
     const int l1 = std::max(5, k - kMaxRowLog), l2 = k - l1;
     const long long n = 1ll << k;
     const Workspace ws_space(dev, kWsNtt, (size_t)2 * n * sizeof(u32), st, &err);

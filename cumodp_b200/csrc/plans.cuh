@@ -57,57 +57,17 @@ __host__ __device__ constexpr int col_tw_entries(int logl) {
     return n;
 }
 // Column tiles in shared memory (k_col_fwd, k_col_inv: 2^11-row columns;
-// shorter ones are col_direct.cuh's): col_tile_cols adjacent columns x 2^logl
-// rows, processed by col_warps warps, col_ctas resident CTAs per SM, per kind
-// of pass (0: the product's forward pass, 1: the inverse pass, 2: the forward
-// pass of a natural-order transform).  32-column tiles put one column on each
-// lane; 16-column tiles put two tasks on each warp (one per half-warp) and
-// insert a 16-word pad after every 2^col_pad_log rows (the plan's last
-// radix), so that the two half-warps always read opposite halves of the
-// banks.
-__host__ __device__ constexpr int col_tile_cols(int logl, int kind) { return (kind != 0 && logl == 10) || logl >= 11 ? 16 : 32; }
-__host__ __device__ constexpr int col_warps(int logl, int kind) { return logl == 10 && kind == 0 ? 32 : (logl <= 5 ? 1 : (logl <= 6 ? 2 : 16)); }
-__host__ __device__ constexpr int col_ctas(int logl, int kind) { return kind != 0 && logl == 10 ? 2 : 1; }
+// shorter ones are col_direct.cuh's): 16 adjacent columns x 2^logl rows on 16
+// warps, one CTA per SM.  A warp has two tasks, one per half-warp, and a
+// 16-word pad after every 2^col_pad_log rows (the plan's last radix) makes the
+// two half-warps read opposite halves of the banks.
+constexpr int kColTileCols = 16, kColTileWarps = 16;
 __host__ __device__ constexpr int col_pad_log(int logl) { return col_plan(logl).logr[col_plan(logl).nlev - 1]; }
-__host__ __device__ constexpr int col_tile_words(int logl, int kind) {
-    return col_tile_cols(logl, kind) == 32
-               ? (32 << logl)
-               : ((1 << logl) + ((1 << logl) >> col_pad_log(logl))) * col_tile_cols(logl, kind);
+__host__ __device__ constexpr int col_tile_words(int logl) {
+    return ((1 << logl) + ((1 << logl) >> col_pad_log(logl))) * kColTileCols;
 }
-// Whether a column CTA stages its twiddles in shared memory next to the
-// tile (else the levels read them from global memory, as broadcasts).
-__host__ __device__ constexpr bool col_tw_smem(int logl, int kind) { return true; }
 // Dynamic shared memory of a column CTA: the tile and its twiddles.
-__host__ __device__ constexpr int col_smem_bytes(int logl, int kind) {
-    return col_tile_words(logl, kind) * 4 + (col_tw_smem(logl, kind) ? col_tw_entries(logl) * 8 : 0);
-}
-
-// Shared-memory layouts of staged column passes for 2^9- and 2^10-row columns
-// (a tile, a stage of its first n1/2 rows and the level-0 twiddles); the
-// passes run from registers now (col_direct.cuh), the layouts are what
-// tests/index_maps_check.cu checks the tile maps with.
-__host__ __device__ constexpr bool col_pipe_ok(int logl) { return logl == 9 || logl == 10; }
-__host__ __device__ constexpr int col_pipe_kind(int logl) { return logl == 10 ? 2 : 0; }  // tile layout (col_tile_cols)
-__host__ __device__ constexpr int col_pipe_warps(int logl) { return logl == 10 ? 8 : 16; }
-__host__ __device__ constexpr int col_pipe_ctas(int logl) { return logl == 10 ? 2 : 1; }
-__host__ __device__ constexpr int col_pipe_smem_bytes(int logl) {
-    // tile, stage (the tile layout's first n1/2 rows), level-0 twiddles
-    return col_tile_words(logl, col_pipe_kind(logl)) * 4 +
-           (col_tile_cols(logl, col_pipe_kind(logl)) == 32
-                ? (16 << logl)
-                : ((1 << logl) / 2 + ((1 << logl) / 2 >> col_pad_log(logl))) * col_tile_cols(logl, col_pipe_kind(logl))) * 4 +
-           (1 << logl) * 8;
-}
-
-// The same with a stage for a whole tile, inverse and natural-order layouts.
-__host__ __device__ constexpr int col_inv_pipe_warps(int logl) { return 16; }
-__host__ __device__ constexpr int col_inv_pipe_smem_bytes(int logl) {
-    return 2 * col_tile_words(logl, 1) * 4 + (1 << logl) * 8;
-}
-
-__host__ __device__ constexpr int col_pipe1_smem_bytes(int logl) {
-    return 2 * col_tile_words(logl, 2) * 4 + (1 << logl) * 8;
-}
+__host__ __device__ constexpr int col_smem_bytes(int logl) { return col_tile_words(logl) * 4 + col_tw_entries(logl) * 8; }
 
 // A single product (no batch) of transform length 2^logn uses the three-pass
 // kernels from this length on, even where one CTA could hold it: spread over
@@ -130,11 +90,6 @@ __host__ __device__ constexpr int row_threads(int logl) { return logl == 14 ? 10
 // Threads of the split row kernels (one operand row per CTA): one per
 // 32-word row of the last level.
 __host__ __device__ constexpr int rowsplit_threads(int logl) { return logl >= 10 ? (1 << (logl - 5)) : 32; }
-// Shape of one-row CTAs with a thread per 32-word group, 1024 threads per SM
-// (the maps check bounds the row tables' shared memory with it).
-__host__ __device__ constexpr int ntt_row_threads(int logl) { return logl >= 10 ? (1 << (logl - 5)) : 32; }
-__host__ __device__ constexpr int ntt_row_ctas(int logl) { return 1024 / ntt_row_threads(logl) < 32 ? 1024 / ntt_row_threads(logl) : 32; }
-
 // Resident CTAs per SM the split row kernels are compiled for: 1024 threads
 // of 64 registers.
 __host__ __device__ constexpr int rowsplit_ctas(int logl) { return (1024 / rowsplit_threads(logl) < 32 ? 1024 / rowsplit_threads(logl) : 32); }

@@ -55,8 +55,8 @@ void launch_pdl(K kernel, dim3 grid, int threads, size_t smem, cudaStream_t st, 
 
 template <int L1>
 void launch_col_fwd_t(const LargeArgs& a, dim3 grid, cudaStream_t st) {
-    const size_t smem = col_smem_bytes(L1, false);
-    k_col_fwd<L1, col_warps(L1, false)><<<grid, col_warps(L1, false) * 32, smem, st>>>(a);
+    const size_t smem = col_smem_bytes(L1);
+    k_col_fwd<L1><<<grid, kColTileWarps * 32, smem, st>>>(a);
 }
 }  // namespace
 
@@ -75,8 +75,8 @@ namespace {
 
 template <int L1>
 void launch_col_inv_t(const LargeArgs& a, dim3 grid, cudaStream_t st) {
-    const size_t smem = col_smem_bytes(L1, true);
-    launch_pdl(k_col_inv<L1, col_warps(L1, true)>, grid, col_warps(L1, true) * 32, smem, st, a);
+    const size_t smem = col_smem_bytes(L1);
+    launch_pdl(k_col_inv<L1>, grid, kColTileWarps * 32, smem, st, a);
 }
 template <int L2>
 void launch_row_t(const LargeArgs& a, dim3 grid, cudaStream_t st) {
@@ -197,8 +197,8 @@ void attr_small(cudaError_t* e) {
 }
 template <int L1>
 void attr_col(cudaError_t* e) {
-    allow_more(e, k_col_fwd<L1, col_warps(L1, false)>, col_smem_bytes(L1, false));
-    allow_more(e, k_col_inv<L1, col_warps(L1, true)>, col_smem_bytes(L1, true));
+    allow_more(e, k_col_fwd<L1>, col_smem_bytes(L1));
+    allow_more(e, k_col_inv<L1>, col_smem_bytes(L1));
 }
 template <int L2>
 void attr_row(cudaError_t* e) {
@@ -248,9 +248,15 @@ int product_logn(long long la, long long lb) {
 }
 
 int default_row_log(int logn) {
-    // rows of 2^l2 words, columns of 2^(logn-l2): the split with the shortest
-    // single-product time measured on B200 for each length 2^15..2^24 (a
-    // batch's own splits come from the autotuner)
+    // Rows of 2^l2 words, columns of 2^(logn-l2), for a single product of
+    // 2^17..2^24 points (shorter ones are one launch) and for the entries that
+    // do not tune (no-allocation, serving; a batch's own splits come from the
+    // autotuner).  The shortest single-product times of the column passes and
+    // four-level rows that the present kernels replaced.  With the present ones
+    // (us, a batch of one): 2^17 16.6 (rows of 2^11: 14.9), 2^18 18.8 (2^12:
+    // 16.6), 2^19 27.1 (2^11-2^13: 18.8), 2^20 30.4 (2^12: 23.0), 2^21 35.4, 2^22
+    // 64.0, 2^23 135.5 (2^13: 119.7), 2^24 244; 2^15 16.6 (2^11: 13.6), 2^16 15.0
+    // (2^12: 14.4).
     static const int kBest[25] = {7, 7, 7, 7, 7, 7, 7, 7, 7, 7, 7, 7, 7, 7, 7,
                                   7, 11, 12, 13, 14, 10, 11, 12, 14, 14};
     if (logn >= 0 && logn <= 24) return kBest[logn];
@@ -336,14 +342,15 @@ void launch_col_fwd(const LargeArgs& a, int njobs, cudaStream_t st) {
     if (a.l1 <= kMaxDirectColLog)
         kColdFwd[a.l1](a, 2, njobs, st);
     else
-        launch_col_fwd_t<kMaxColLog>(a, dim3((1 << a.l2) / col_tile_cols(kMaxColLog, false), 2, njobs), st);
+        launch_col_fwd_t<kMaxColLog>(a, dim3((1 << a.l2) / kColTileCols, 2, njobs), st);
     if (tr) pass_timing_end(st, kColFwdName[a.l1], e0);
 }
 
-bool launch_col_fwd1(const LargeArgs& a, int njobs, cudaStream_t st) {
-    if (a.l1 > kMaxDirectColLog) return false;
-    kColdFwd[a.l1](a, 1, njobs, st);
-    return true;
+void launch_col_fwd1(const LargeArgs& a, int njobs, cudaStream_t st) {
+    if (a.l1 <= kMaxDirectColLog)
+        kColdFwd[a.l1](a, 1, njobs, st);
+    else
+        launch_col_fwd_t<kMaxColLog>(a, dim3((1 << a.l2) / kColTileCols, 1, njobs), st);
 }
 
 void launch_col_inv(const LargeArgs& a, int njobs, cudaStream_t st) {
@@ -352,7 +359,7 @@ void launch_col_inv(const LargeArgs& a, int njobs, cudaStream_t st) {
     if (a.l1 <= kMaxDirectColLog) {
         kColdInv[a.l1](a, njobs, st);
     } else {
-        launch_col_inv_t<kMaxColLog>(a, dim3((1 << a.l2) / col_tile_cols(kMaxColLog, true), 1, njobs), st);
+        launch_col_inv_t<kMaxColLog>(a, dim3((1 << a.l2) / kColTileCols, 1, njobs), st);
     }
     if (tr) pass_timing_end(st, kColInvName[a.l1], e0);
 }

@@ -34,10 +34,10 @@ int default_row_log(int logn);
 
 int small_args(const PrimeCtx& pc, u32 root, int logn, int dev, SmallArgs* a);
 int large_args(const PrimeCtx& pc, u32 root_n, int logn, int l2, int dev, LargeArgs* a);
-// The forward column pass of every job's two operands; that of operand a alone
-// (false past 2^kMaxDirectColLog rows); the inverse column pass.
+// The forward column pass of every job's two operands; that of operand a alone;
+// the inverse column pass.
 void launch_col_fwd(const LargeArgs& a, int njobs, cudaStream_t st);
-bool launch_col_fwd1(const LargeArgs& a, int njobs, cudaStream_t st);
+void launch_col_fwd1(const LargeArgs& a, int njobs, cudaStream_t st);
 void launch_col_inv(const LargeArgs& a, int njobs, cudaStream_t st);
 void launch_small(int logn, const SmallArgs& a, int njobs, cudaStream_t st);
 void launch_large(const LargeArgs& a, int njobs, cudaStream_t st);

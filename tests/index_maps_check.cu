@@ -7,25 +7,30 @@
 //            products of one and of several operand pairs per CTA) touches
 //            each word of its buffer exactly once, swz_task equals the plain
 //            swizzle, the last level's 16-byte quads tile the buffer, and the
-//            twiddle reads stay inside the plan's table;
-//   columns: for every tile kind and 2^1..2^11 rows, tile_row is injective and
-//            in bounds, tile_step equals tile_row differences for every level
-//            task, and the two half-warps of a 16-column tile read opposite
-//            halves of the banks;
-//   orders:  col_slot_to_k1 and row_pos_to_freq are permutations;
+//            twiddle reads cover the level's entries of the plan's table;
+//   staged columns (2^11 rows): tile_row is injective and in bounds, tile_step
+//            equals tile_row differences for every level task, and the two
+//            half-warps read opposite halves of the banks;
+//   register columns (2^1..2^10 rows): the exchange between the two levels is a
+//            bijection within shared memory, rows are read and written once;
+//   natural-order rows (2^6..2^14 words): every level touches each word once,
+//            outputs are a permutation, shared memory and tables are in bounds;
+//   bivariate rows: the same for the leading level and the levels over x;
+//   orders:  col_slot_to_k1 is bit reversal for every column plan;
 //   row factor tables (rows of 2^11..2^14 words): every level-0 task reads
 //            its two entries inside the table, the two digits recompose the
 //            task index, and the row kernels' shared memory fits the SM;
-//   pipelined column pass: stage, tile and twiddle indexes in bounds;
-//   one-launch products: padded addresses in bounds and distinct, level tasks cover
-//            each block once, twiddle reads in bounds, shared memory fits;
+//   one-launch products and subproduct levels: padded addresses in bounds and
+//            distinct, level tasks cover each block once, twiddle reads in
+//            bounds, shared memory fits; the table builders' exponents;
 //   Shoup quotients from the double estimate equal floor(w 2^32 / p);
-//   the quad-interleaved row spectrum is a permutation with warp-contiguous runs;
-//   the natural-order reorder buffer's swizzle is a bijection without store conflicts.
+//   the quad-interleaved row spectrum is a permutation with warp-contiguous runs.
 #include <cstdio>
 #include <set>
 #include <vector>
 
+#include "../cumodp_b200/csrc/col_direct.cuh"
+#include "../cumodp_b200/csrc/grid_product.cuh"
 #include "../cumodp_b200/csrc/large_product.cuh"
 #include "../cumodp_b200/csrc/latency_product.cuh"
 #include "../cumodp_b200/csrc/row_natural.cuh"
@@ -48,7 +53,7 @@ template <int LOGL, int LEV>
 void row_level(int ppc) {
     using LV = SmallLevel<LOGL, LEV>;
     constexpr int L = 1 << LOGL, R = LV::R, TB = LV::TB, B = LV::B;
-    std::vector<int> seen((size_t)ppc * 2 * L, 0);
+    std::vector<int> seen((size_t)ppc * 2 * L, 0), read((size_t)plan_tw_entries(row_plan(LOGL), LOGL), 0);
     for (int q = 0; q < ppc; ++q)
         for (int op = 0; op < 2; ++op)
             for (int rest = 0; rest < L / R; ++rest) {
@@ -61,11 +66,18 @@ void row_level(int ppc) {
                     CHECK(a >= 0 && a < (int)seen.size(), "row L=%d lev=%d out of range", LOGL, LEV);
                     if (a >= 0 && a < (int)seen.size()) seen[a]++;
                 }
-                // twiddles of this task: o * R + j < the level's B entries
-                CHECK(LV::TWOFF + o * R + R - 1 < plan_tw_entries(row_plan(LOGL), LOGL),
-                      "row L=%d lev=%d twiddle index", LOGL, LEV);
+                // twiddles of this task: slot j at j TB + o (load_tw)
+                for (int j = 0; j < R; ++j) {
+                    const size_t t = (size_t)(LV::TWOFF + j * TB + o);
+                    CHECK(t < read.size(), "row L=%d lev=%d twiddle index", LOGL, LEV);
+                    if (t < read.size()) read[t]++;
+                }
             }
     for (size_t i = 0; i < seen.size(); ++i) CHECK(seen[i] == 1, "row L=%d lev=%d word %zu hit %d", LOGL, LEV, i, seen[i]);
+    // every task of the level reads its own entries, once per block and operand
+    for (size_t t = 0; t < read.size(); ++t)
+        CHECK(read[t] == ((int)t >= LV::TWOFF && (int)t < LV::TWOFF + B ? ppc * 2 * (L / B) : 0),
+              "row L=%d lev=%d twiddle %zu read %d times", LOGL, LEV, t, read[t]);
 }
 
 template <int LOGL, int LEV>
@@ -92,101 +104,189 @@ void row_plan_check() {
                 if (a + k >= 0 && a + k < L) seen[a + k]++;
         }
     for (int i = 0; i < L; ++i) CHECK(seen[i] == 1, "row L=%d last level word %d", LOGL, i);
-    // natural order after the row plan: a permutation
-    if constexpr (LOGL >= 6) {
-        std::vector<int> f(L, 0);
-        for (int P = 0; P < L; ++P) {
-            const u32 v = row_pos_to_freq<LOGL>((u32)P);
-            CHECK(v < (u32)L, "row_pos_to_freq L=%d", LOGL);
-            if (v < (u32)L) f[v]++;
-        }
-        for (int i = 0; i < L; ++i) CHECK(f[i] == 1, "row_pos_to_freq L=%d not a permutation", LOGL);
-    }
 }
 
-template <int L1, int INV, int LEV>
+template <int L1, int LEV>
 void col_level() {
     using LV = ColLevel<L1, LEV>;
     constexpr int R = LV::R, TB = LV::TB, B = LV::B;
-    constexpr int TC = col_tile_cols(L1, INV);
     constexpr int TASKS = (1 << L1) / R;
     for (int id = 0; id < TASKS; ++id) {
         const int blk = id / TB, o = id % TB;
         const int row0 = blk * B + o;
         for (int m = 0; m < R; ++m)
-            CHECK((tile_row<L1, INV>(row0) + tile_step<L1, INV, TB>(m) == tile_row<L1, INV>(row0 + TB * m)),
-                  "col L1=%d kind=%d lev=%d tile_step", L1, INV, LEV);
-        // a 16-column tile puts tasks id (even) and id + 1 on the two half-warps
-        if (TC == 16 && id % 2 == 0 && id + 1 < TASKS) {
+            CHECK((tile_row<L1>(row0) + tile_step<L1, TB>(m) == tile_row<L1>(row0 + TB * m)),
+                  "col L1=%d lev=%d tile_step", L1, LEV);
+        // tasks id (even) and id + 1 are on the two half-warps
+        if (id % 2 == 0 && id + 1 < TASKS) {
             const int blk2 = (id + 1) / TB, o2 = (id + 1) % TB;
             const int row1 = blk2 * B + o2;
             for (int m = 0; m < R; ++m) {
-                const int a = tile_row<L1, INV>(row0 + TB * m), b = tile_row<L1, INV>(row1 + TB * m);
-                CHECK(((a - b) % 32 + 32) % 32 == 16, "col L1=%d kind=%d lev=%d half-warp banks", L1, INV, LEV);
+                const int a = tile_row<L1>(row0 + TB * m), b = tile_row<L1>(row1 + TB * m);
+                CHECK(((a - b) % 32 + 32) % 32 == 16, "col L1=%d lev=%d half-warp banks", L1, LEV);
             }
         }
+        if (LEV + 1 < col_plan(L1).nlev)
+            CHECK(LV::TWOFF + o * R + R - 1 < col_tw_entries(L1), "col L1=%d lev=%d twiddle", L1, LEV);
     }
 }
 
-template <int L1, int INV, int LEV>
+template <int L1, int LEV>
 void col_levels() {
     constexpr LevelPlan PL = col_plan(L1);
     if constexpr (LEV < PL.nlev) {
-        col_level<L1, INV, LEV>();
-        col_levels<L1, INV, LEV + 1>();
+        col_level<L1, LEV>();
+        col_levels<L1, LEV + 1>();
     }
 }
 
-template <int L1, int INV>
-void col_kind_check() {
-    constexpr int n1 = 1 << L1, TC = col_tile_cols(L1, INV);
+// The staged column kernels' tile.
+template <int L1>
+void col_tile_check() {
+    constexpr int n1 = 1 << L1;
     std::set<int> used;
     for (int r = 0; r < n1; ++r)
-        for (int c = 0; c < TC; ++c) {
-            const int a = tile_row<L1, INV>(r) + c;
-            CHECK((a >= 0 && a < col_tile_words(L1, INV)), "col L1=%d kind=%d out of tile", L1, INV);
-            CHECK(used.insert(a).second, "col L1=%d kind=%d collision", L1, INV);
+        for (int c = 0; c < kColTileCols; ++c) {
+            const int a = tile_row<L1>(r) + c;
+            CHECK((a >= 0 && a < col_tile_words(L1)), "col L1=%d out of tile", L1);
+            CHECK(used.insert(a).second, "col L1=%d collision", L1);
         }
     // 16-byte quads of a row stay inside the row and 16-byte aligned
-    for (int r = 0; r < n1; ++r) CHECK((tile_row<L1, INV>(r) % 4 == 0), "col L1=%d kind=%d quad alignment", L1, INV);
-    CHECK((col_smem_bytes(L1, INV) <= 227 * 1024), "col L1=%d kind=%d shared memory", L1, INV);
-    col_levels<L1, INV, 0>();
+    for (int r = 0; r < n1; ++r) CHECK((tile_row<L1>(r) % 4 == 0), "col L1=%d quad alignment", L1);
+    CHECK(col_smem_bytes(L1) <= 227 * 1024, "col L1=%d shared memory", L1);
+    col_levels<L1, 0>();
 }
 
+// Rows leave a column pass in bit-reversed order, whatever its levels.
+void col_order_check(int l1) {
+    for (u32 s = 0; s < (1u << l1); ++s) CHECK(col_slot_to_k1(s, col_plan(l1), l1) == rev_bits(s, l1), "column order L1=%d", l1);
+}
+
+// The register column kernels (k_cold_fwd; k_cold_inv runs the same maps the
+// other way): level 0's task o of column c reads rows o + R1 m and writes slot
+// j to block j, the last level's task b reads its block and writes rows b R1 + m.
 template <int L1>
-void col_plan_check() {
-    col_kind_check<L1, 0>();
-    col_kind_check<L1, 1>();
-    col_kind_check<L1, 2>();
-    const LevelPlan PL = col_plan(L1);
-    std::vector<int> k(1 << L1, 0);
-    for (u32 s = 0; s < (1u << L1); ++s) {
-        const u32 v = col_slot_to_k1(s, PL, L1);
-        CHECK(v < (1u << L1), "col_slot_to_k1 L1=%d", L1);
-        if (v < (1u << L1)) k[v]++;
-    }
-    for (int i = 0; i < (1 << L1); ++i) CHECK(k[i] == 1, "col_slot_to_k1 L1=%d not a permutation", L1);
+void cold_check() {
+    constexpr bool TWO = cold_two(L1);
+    constexpr int n1 = 1 << L1, R0 = cold_r0(L1), R1 = cold_r1(L1), TC = cold_cols(L1), T = cold_threads(L1), BL = cold_block(L1);
+    CHECK(R0 * R1 == n1 && (TWO || R1 == 1), "cold L1=%d radices", L1);
+    CHECK(T % TC == 0 && T <= 1024, "cold L1=%d threads", L1);
+    std::vector<int> in(n1, 0), out(n1, 0), wrote(cold_smem(L1) / 4 + 1, 0), read(cold_smem(L1) / 4 + 1, 0);
+    for (int g = 0; g < T / TC; ++g)
+        for (int o = g; o < R1; o += T / TC)
+            for (int m = 0; m < R0; ++m) {
+                in[o + R1 * m]++;
+                if (!TWO) out[m]++;
+                for (int c = 0; TWO && c < TC; ++c) {
+                    const int a = o * TC + c + m * BL;
+                    CHECK(a >= 0 && a < (int)(cold_smem(L1) / 4), "cold L1=%d tile", L1);
+                    if (a >= 0 && a < (int)(cold_smem(L1) / 4)) wrote[a]++;
+                }
+                if (TWO) CHECK(o * R0 + m < col_tw_entries(L1) && (o * R0) % 2 == 0, "cold L1=%d twiddle", L1);
+            }
+    for (int g = 0; TWO && g < T / TC; ++g)
+        for (int b = g; b < R0; b += T / TC)
+            for (int m = 0; m < R1; ++m) {
+                out[b * R1 + m]++;
+                for (int c = 0; c < TC; ++c) {
+                    const int a = b * BL + c + m * TC;
+                    CHECK(a >= 0 && a < (int)(cold_smem(L1) / 4), "cold L1=%d tile", L1);
+                    if (a >= 0 && a < (int)(cold_smem(L1) / 4)) read[a]++;
+                }
+            }
+    for (int r = 0; r < n1; ++r) CHECK(in[r] == 1 && out[r] == 1, "cold L1=%d row %d", L1, r);
+    for (size_t a = 0; a < wrote.size(); ++a) CHECK(wrote[a] == read[a] && wrote[a] <= 1, "cold L1=%d word %zu", L1, a);
+    if (TWO && TC == 16) CHECK(BL % 32 == 16, "cold L1=%d half-warp banks", L1);
+    CHECK((cold_smem(L1) + 1024) * cold_ctas(L1) <= 228 * 1024, "cold L1=%d shared memory", L1);
 }
 
-// Natural-order reorder of k_row_ntt: swz_nat is a bijection, and the
-// stores of one step (lanes r = 32 w + lane, output j) hit distinct banks.
+// The natural-order row kernel.
 template <int L2>
-void ntt_reorder_check() {
-    constexpr int n2 = 1 << L2;
-    std::vector<int> hit(n2, 0);
-    for (int f = 0; f < n2; ++f) {
-        const int a = swz_nat(f);
-        CHECK((a >= 0 && a < n2), "reorder L2=%d range", L2);
-        if (a >= 0 && a < n2) hit[a]++;
-    }
-    for (int i = 0; i < n2; ++i) CHECK(hit[i] == 1, "reorder L2=%d bijection", L2);
-    for (int w = 0; w * 32 < n2 / 32; ++w)
-        for (int j = 0; j < 32; ++j) {
-            int banks[32] = {0};
-            for (int l = 0; l < 32 && w * 32 + l < n2 / 32; ++l)
-                banks[swz_nat((int)row_pos_to_freq<L2>((u32)((w * 32 + l) * 32 + j))) % 32]++;
-            for (int b = 0; b < 32; ++b) CHECK(banks[b] <= 1, "reorder L2=%d bank conflict", L2);
+void nat_check() {
+    constexpr LevelPlan PL = nat_plan(L2);
+    constexpr bool THREE = PL.nlev == 3;
+    constexpr int n = 1 << L2, TPR = nat_row_threads(L2), S = nat_stride(L2), W = nat_words(L2);
+    constexpr int R0 = 1 << PL.logr[0], TB0 = n / R0, R1 = THREE ? 1 << PL.logr[1] : 1, TB1 = TB0 / R1;
+    constexpr int RL = 1 << PL.logr[PL.nlev - 1];
+    CHECK(R0 * R1 * RL == n && TPR == TB0 && TB1 == RL, "nat L2=%d plan", L2);
+    CHECK(nat_threads(L2) <= 1024 && nat_rows(L2) * W * 4 == (int)nat_smem(L2), "nat L2=%d shape", L2);
+    CHECK((nat_smem(L2) + 1024) * nat_ctas(L2) <= 228 * 1024, "nat L2=%d shared memory", L2);
+    std::vector<int> in(n, 0), out(n, 0), w0(W, 0), w1(W, 0), wl(W, 0), tw(nat_entries(L2), 0);
+    auto hit = [&](std::vector<int>& v, int a) {
+        CHECK(a >= 0 && a < (int)v.size(), "nat L2=%d index", L2);
+        if (a >= 0 && a < (int)v.size()) v[a]++;
+    };
+    for (int t = 0; t < TPR; ++t)
+        for (int k = 0; k < R0; ++k) {
+            hit(in, t + TB0 * k);
+            hit(w0, S * k + t);
+            hit(tw, t + TB0 * k);
         }
+    for (int t = 0; THREE && t < TPR; ++t)
+        for (int id = t; id < R0 * TB1; id += TPR)
+            for (int k = 0; k < R1; ++k) {
+                hit(w1, S * (id / TB1) + id % TB1 + TB1 * k);
+                if (id < TB1) hit(tw, n + id % TB1 + TB1 * k);
+            }
+    for (int t = 0; t < TPR; ++t)
+        for (int id = t; id < n / RL; id += TPR)
+            for (int k = 0; k < RL; ++k) {
+                hit(wl, S * (id % R0) + RL * (id / R0) + k);
+                hit(out, id + (n / RL) * k);
+            }
+    for (int i = 0; i < n; ++i) CHECK(in[i] == 1 && out[i] == 1, "nat L2=%d word %d", L2, i);
+    for (int a = 0; a < W; ++a)
+        CHECK(w0[a] <= 1 && wl[a] == w0[a] && (!THREE || w1[a] == w0[a]), "nat L2=%d exchange word %d", L2, a);
+    for (size_t e = 0; e < tw.size(); ++e) CHECK(tw[e] == 1, "nat L2=%d twiddle %zu", L2, e);
+}
+
+// The row passes of a bivariate product: E bits of y and rows of 2^L2 words.
+template <int E, int L2, int LEV>
+void grid_levels() {
+    constexpr int LT = grid_log(E, L2), N = 1 << LT;
+    constexpr LevelPlan PL = row_plan(L2);
+    if constexpr (LEV + 1 < PL.nlev) {
+        using LV = SmallLevel<L2, LEV>;
+        constexpr int R = LV::R, TB = LV::TB, B = LV::B;
+        std::vector<int> seen(N, 0);
+        for (int id = 0; id < N / R; ++id) {
+            const int o = id % TB, base = (id / TB) * B + o, bs = swz(base);
+            for (int m = 0; m < R; ++m) {
+                const int a = swz_task<TB, B>(base, bs, m);
+                CHECK((a == swz(base + TB * m) && a < N), "grid E=%d L2=%d lev=%d", E, L2, LEV);
+                if (a >= 0 && a < N) seen[a]++;
+                CHECK(LV::TWOFF + m * TB + o < plan_tw_entries(PL, L2), "grid E=%d L2=%d lev=%d twiddle", E, L2, LEV);
+            }
+        }
+        for (int a = 0; a < N; ++a) CHECK(seen[a] == 1, "grid E=%d L2=%d lev=%d word %d", E, L2, LEV, a);
+        grid_levels<E, L2, LEV + 1>();
+    }
+}
+
+template <int E, int L2>
+void grid_check() {
+    constexpr int LT = grid_log(E, L2), N = 1 << LT;
+    CHECK(grid_threads(LT) * 32 == N && (N * 4 + 1024) * grid_ctas(LT) <= 228 * 1024, "grid E=%d L2=%d shape", E, L2);
+    if constexpr (E > 0) {
+        // the level over y0: words 2^L2 apart, slot block (N / B) + blk's factors
+        constexpr int R = 1 << E, TB = 1 << L2, B = TB << E;
+        for (int slots = 1 << (LT - E - L2); slots <= 1 << 11; slots *= 2) {
+            const int blocks = (int)(((long long)slots << (E + L2)) >> LT);
+            CHECK(blocks >= 1 && ((long long)blocks << LT) == (long long)slots << (E + L2), "grid E=%d L2=%d blocks", E, L2);
+            CHECK((blocks - 1) * (N / B) + N / B - 1 == slots - 1, "grid E=%d L2=%d slots", E, L2);
+        }
+        std::vector<int> seen(N, 0);
+        for (int id = 0; id < N / R; ++id) {
+            const int o = id % TB, base = (id / TB) * B + o, bs = swz(base);
+            for (int m = 0; m < R; ++m) {
+                const int a = swz_task<TB, B>(base, bs, m);
+                CHECK((a == swz(base + TB * m) && a < N), "grid E=%d L2=%d leading level", E, L2);
+                if (a >= 0 && a < N) seen[a]++;
+            }
+        }
+        for (int a = 0; a < N; ++a) CHECK(seen[a] == 1, "grid E=%d L2=%d leading word %d", E, L2, a);
+    }
+    grid_levels<E, L2, 0>();
 }
 
 // G's row spectrum between the row kernels: quad c of 32-word group r at
@@ -230,7 +330,7 @@ void row_tab_check() {
         CHECK(at >= 0 && at < RT::ENTRIES, "rowtab L2=%d build slot", L2);
         if (at >= 0 && at < RT::ENTRIES) hit[at]++;
         CHECK(w >= 0 && w < RT::NPOW, "rowtab L2=%d build power", L2);
-        CHECK(e * RT::R0 + j < plan_tw_entries(row_plan(L2), L2), "rowtab L2=%d build twiddle", L2);
+        CHECK(j * RT::TB0 + e < 1 << L2 && e < RT::TB0, "rowtab L2=%d build twiddle", L2);
         // the slot the level reads for (o, j) has exponent o mod NA, resp. NA (o div NA)
         if (q < RT::R0 * RT::NA) CHECK(at % RT::NA == e && at / RT::NA == j, "rowtab L2=%d A exponent", L2);
         else CHECK((at - RT::R0 * RT::NA) % RT::NB * RT::NA == e, "rowtab L2=%d B exponent", L2);
@@ -239,77 +339,7 @@ void row_tab_check() {
     // shared memory of the split row kernels (+1 KiB reserved per CTA)
     const long long smem = (long long)(1 << L2) * 4 + (long long)RT::TABW * 8 + (long long)RT::NPOW * 4 + 2 * RT::R0 * 8;
     CHECK((RT::TABW * 8) % 16 == 0, "rowtab L2=%d table not a whole number of 16-byte copies", L2);
-    // the natural-order row kernel holds the row and the forward table
-    CHECK(((long long)(1 << L2) * 4 + (long long)RT::TABW * 8 + RT::R0 * 8 + 1024) * ntt_row_ctas(L2) <= 228 * 1024,
-          "ntt row L2=%d shared memory", L2);
     CHECK((smem + 1024) * rowsplit_ctas(L2) <= 228 * 1024, "rowsplit L2=%d shared memory", L2);
-}
-
-template <int L1, int KIND>
-void col_pipe_check() {
-    constexpr LevelPlan PL = col_plan(L1);
-    constexpr int n1 = 1 << L1, HALF = n1 / 2, R0 = 1 << PL.logr[0], R1 = 1 << PL.logr[1];
-    constexpr int TC = col_tile_cols(L1, KIND), QR = TC / 4;
-    constexpr int TW = col_tile_words(L1, KIND);
-    const int SW = tile_row<L1, KIND>(HALF);
-    CHECK(PL.nlev == 2 && R0 * R1 == n1, "colpipe L1=%d plan", L1);
-    // stage copies of rows [0, HALF) and tile copies of rows [HALF, n1)
-    for (int idx = 0; idx < n1 * QR; ++idx) {
-        const int r = idx / QR, q = idx % QR;
-        const int a = tile_row<L1, KIND>(r) + 4 * q;
-        CHECK((a % 4 == 0 && a + 3 < (r < HALF ? SW : TW)), "colpipe L1=%d kind=%d copy", L1, KIND);
-    }
-    for (int o = 0; o < R1; ++o)
-        for (int m = 0; m < R0; ++m) {
-            const int row = o + R1 * m;
-            CHECK((tile_row<L1, KIND>(o) + tile_step<L1, KIND, R1>(m) == tile_row<L1, KIND>(row)), "colpipe L1=%d level-0 step", L1);
-            if (m < R0 / 2) CHECK((row < HALF && tile_row<L1, KIND>(row) + TC <= SW), "colpipe L1=%d stage row", L1);
-            else CHECK(row >= HALF, "colpipe L1=%d upper row", L1);
-            CHECK(o * R0 + m < col_tw_entries(L1), "colpipe L1=%d twiddle", L1);
-        }
-    for (int blk = 0; blk < R0; ++blk)
-        for (int m = 0; m < R1; ++m)
-            CHECK((tile_row<L1, KIND>(blk * R1) + tile_step<L1, KIND, 1>(m) == tile_row<L1, KIND>(blk * R1 + m)), "colpipe L1=%d level-1 step", L1);
-    if (KIND == col_pipe_kind(L1)) {
-        CHECK(col_pipe_smem_bytes(L1) == TW * 4 + SW * 4 + col_tw_entries(L1) * 8, "colpipe L1=%d layout", L1);
-        CHECK((col_pipe_smem_bytes(L1) + 1024) * col_pipe_ctas(L1) <= 228 * 1024, "colpipe L1=%d shared memory", L1);
-    }
-}
-
-template <int L1>
-void col_inv_pipe_check() {
-    constexpr LevelPlan PL = col_plan(L1);
-    constexpr int n1 = 1 << L1, R0 = 1 << PL.logr[0], R1 = 1 << PL.logr[1];
-    constexpr int TC = col_tile_cols(L1, 1), QR = TC / 4, TW = col_tile_words(L1, 1);
-    // stage copies: every 16-byte quad of every row inside the stage, aligned
-    for (int idx = 0; idx < n1 * QR; ++idx) {
-        const int r = idx / QR, q = idx % QR;
-        const int a = tile_row<L1, 1>(r) + 4 * q;
-        CHECK((a % 4 == 0 && a + 3 < TW), "colinvpipe L1=%d stage quad", L1);
-    }
-    // deepest level (blocks of R1 rows) and level 0 (rows o + R1 m): in the tile
-    for (int id = 0; id < R0; ++id)
-        for (int m = 0; m < R1; ++m)
-            CHECK((tile_row<L1, 1>(id * R1) + tile_step<L1, 1, 1>(m) == tile_row<L1, 1>(id * R1 + m)), "colinvpipe L1=%d deep", L1);
-    for (int o = 0; o < R1; ++o)
-        for (int m = 0; m < R0; ++m) {
-            CHECK((tile_row<L1, 1>(o) + tile_step<L1, 1, R1>(m) == tile_row<L1, 1>(o + R1 * m)), "colinvpipe L1=%d lvl0", L1);
-            CHECK(o * R0 + m < n1, "colinvpipe L1=%d twiddle", L1);
-        }
-    CHECK(col_inv_pipe_smem_bytes(L1) + 1024 <= 228 * 1024, "colinvpipe L1=%d shared memory", L1);
-    // per-warp refill: warp w's deepest-level blocks are exactly the rows it
-    // copies, [w SUB R1, (w + 1) SUB R1), and the warps cover all n1 rows once
-    constexpr int NW = col_inv_pipe_warps(L1), SUB = 32 / TC;
-    CHECK(NW * SUB == R0, "colinvpipe L1=%d one block set per warp", L1);
-    std::vector<int> rows(n1, 0);
-    for (int w = 0; w < NW; ++w)
-        for (int l = 0; l < 32; ++l) {
-            const int blk = w * SUB + l / TC;
-            CHECK((blk * R1 >= w * SUB * R1 && (blk + 1) * R1 <= (w + 1) * SUB * R1), "colinvpipe L1=%d warp blocks", L1);
-            for (int r = w * SUB * R1 + l / QR; r < (w + 1) * SUB * R1; r += 32 / QR)
-                if (l % QR == 0) rows[r]++;
-        }
-    for (int r = 0; r < n1; ++r) CHECK(rows[r] == 1, "colinvpipe L1=%d refill row %d copied %d times", L1, r, rows[r]);
 }
 
 void shoup_quot_check() {
@@ -371,6 +401,15 @@ void latency_check(int cluster) {
     }
 }
 
+// The subproduct level kernel: the same blocks on its own CTA shape.
+template <int LOGL>
+void level_check() {
+    constexpr int L = 1 << LOGL, T = level_threads(LOGL);
+    latency_check<LOGL>(1);
+    CHECK(2 * L % T == 0 && T <= 1024, "level L=%d load loop", LOGL);
+    CHECK(T * level_ctas(LOGL) <= 2048 && level_ctas(LOGL) <= 32, "level L=%d residency", LOGL);
+}
+
 // latency_tables' exponents: entry (o, j) of a level of blocks of B = 2^lb
 // words is (w^(2^(logn - lb)))^(+-o bitrev(j)), where the kernels read it.
 template <int LOGL>
@@ -426,13 +465,14 @@ int main() {
     slot_exponent_check<13>(5);
     slot_exponent_check<14>(10);
     slot_exponent_check<14>(11);
-    latency_check<5>(1);
-    latency_check<6>(1);
-    latency_check<7>(1);
-    latency_check<8>(1);
-    latency_check<9>(1);
-    latency_check<10>(1);
-    latency_check<11>(1);
+    level_check<5>();
+    level_check<6>();
+    level_check<7>();
+    level_check<8>();
+    level_check<9>();
+    level_check<10>();
+    level_check<11>();
+    level_check<12>();
     latency_check<8>(16);
     latency_check<9>(16);
     latency_check<10>(16);
@@ -448,36 +488,61 @@ int main() {
     row_plan_check<12>();
     row_plan_check<13>();
     row_plan_check<14>();
-    col_plan_check<1>();
-    col_plan_check<2>();
-    col_plan_check<3>();
-    col_plan_check<4>();
-    col_plan_check<5>();
-    col_plan_check<6>();
-    col_plan_check<7>();
-    col_plan_check<8>();
-    col_plan_check<9>();
-    col_plan_check<10>();
-    col_plan_check<11>();
-    ntt_reorder_check<10>();
-    ntt_reorder_check<11>();
-    ntt_reorder_check<12>();
-    ntt_reorder_check<13>();
-    ntt_reorder_check<14>();
+    for (int l1 = 1; l1 <= 11; ++l1) col_order_check(l1);
+    col_tile_check<11>();
+    cold_check<1>();
+    cold_check<2>();
+    cold_check<3>();
+    cold_check<4>();
+    cold_check<5>();
+    cold_check<6>();
+    cold_check<7>();
+    cold_check<8>();
+    cold_check<9>();
+    cold_check<10>();
+    nat_check<6>();
+    nat_check<7>();
+    nat_check<8>();
+    nat_check<9>();
+    nat_check<10>();
+    nat_check<11>();
+    nat_check<12>();
+    nat_check<13>();
+    nat_check<14>();
+    grid_check<0, 6>();
+    grid_check<0, 7>();
+    grid_check<0, 8>();
+    grid_check<0, 9>();
+    grid_check<0, 10>();
+    grid_check<0, 11>();
+    grid_check<0, 12>();
+    grid_check<0, 13>();
+    grid_check<0, 14>();
+    grid_check<1, 6>();
+    grid_check<1, 7>();
+    grid_check<1, 8>();
+    grid_check<1, 9>();
+    grid_check<1, 10>();
+    grid_check<1, 11>();
+    grid_check<1, 12>();
+    grid_check<1, 13>();
+    grid_check<2, 6>();
+    grid_check<2, 7>();
+    grid_check<2, 8>();
+    grid_check<2, 9>();
+    grid_check<2, 10>();
+    grid_check<2, 11>();
+    grid_check<2, 12>();
     spectrum_layout_check<6>();
     spectrum_layout_check<10>();
+    spectrum_layout_check<11>();
+    spectrum_layout_check<12>();
+    spectrum_layout_check<13>();
     spectrum_layout_check<14>();
     row_tab_check<11>();
     row_tab_check<12>();
     row_tab_check<13>();
     row_tab_check<14>();
-    col_pipe_check<9, 0>();
-    col_pipe_check<10, 0>();
-    col_pipe_check<10, 2>();
-    CHECK(col_pipe1_smem_bytes(10) + 1024 <= 228 * 1024, "colpipe1 shared memory");
-    CHECK(col_pipe1_smem_bytes(10) == 2 * col_tile_words(10, 2) * 4 + 1024 * 8, "colpipe1 layout");
-    col_inv_pipe_check<9>();
-    col_inv_pipe_check<10>();
     shoup_quot_check();
     std::printf("%s: %d failures\n", failures ? "FAILED" : "OK", failures);
     return failures ? 1 : 0;

@@ -2,10 +2,11 @@
 
 Compiles tests/index_maps_check.cu (the kernels' own __host__ __device__ index
 functions, compiled for the host) with nvcc and runs it: every level of every
-row and column plan touches each shared-memory word exactly once, the fast
-address paths equal the plain swizzle, twiddle reads stay in their tables,
-16-column tiles keep their half-warps on opposite bank halves, and the
-digit-reversal maps are permutations.  No GPU is involved.
+row, column, natural-order, bivariate and one-launch plan touches each
+shared-memory word exactly once, the fast address paths equal the plain
+swizzle, twiddle reads stay in their tables, 16-column tiles keep their
+half-warps on opposite bank halves, and the output orders are permutations.
+No GPU is involved.
 """
 import os
 import shutil

@@ -216,9 +216,10 @@ def test_inputs_above_p_are_reduced(cm, oracle_mod):
 
 
 def test_comparison_switches_give_the_same_products(cm):
-    """CUMODP_COL_PIPE=0 (one-tile-per-CTA column passes) and CUMODP_ROWTAB=0
-    (factor tables built inside every row CTA) select other kernels for the
-    same products: a 2^21 and a 2^23 product must come out identical."""
+    """CUMODP_ROWTAB=0 (factor tables built inside every row CTA) and
+    CUMODP_ROW_FUSED=1 (both row passes in one CTA) select other kernels for the
+    same products: 2^21 and 2^23 products (rows of 2^11 and 2^14 words) must come
+    out identical."""
     import os
     import subprocess
     import sys
@@ -234,12 +235,12 @@ def test_comparison_switches_give_the_same_products(cm):
         "print(out)\n")
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     res = []
-    for extra in ({}, {"CUMODP_COL_PIPE": "0", "CUMODP_ROWTAB": "0"}):
+    for extra in ({}, {"CUMODP_ROWTAB": "0"}, {"CUMODP_ROW_FUSED": "1"}):
         env = dict(os.environ, PYTHONPATH=root, **extra)
         out = subprocess.run([sys.executable, "-c", code], env=env, capture_output=True, text=True, timeout=300)
         assert out.returncode == 0, out.stderr[-2000:]
         res.append(out.stdout.strip().splitlines()[-1])
-    assert res[0] == res[1]
+    assert res[0] == res[1] == res[2]
 
 
 _FIRST_USE = r"""
