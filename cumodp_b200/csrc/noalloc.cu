@@ -60,10 +60,11 @@ struct NaDevice {
 std::mutex g_na_m;
 NaDevice g_na[64];
 
-// One plan's level tables (the layout of level_tables_into: per level i,
-// task o and slot j at off_i + j TB_i + o (row plans) or off_i + o R_i + j
-// (column plans) hold w_B^(o bitrev(j)) in Shoup form, the forward tables first and the inverse ones nf entries later, then
-// two zero words), with w_B and w_B^-1 of every level in Montgomery form.
+// One plan's level tables (the layout of level_tables_into: per level i, task o
+// and slot j at off_i + j TB_i + o (row plans) or off_i + o R_i + j (column
+// plans) hold w_B^(o bitrev(j)) in Shoup form, the forward tables first and the
+// inverse ones nf entries later, then two zero words), with w_B and w_B^-1 of
+// every level in Montgomery form.
 struct NaPlan {
     Tw* out;
     LevelPlan pl;
@@ -106,8 +107,8 @@ __device__ __forceinline__ Tw na_level_entry(const NaPlan& P, int t, u32 one_m, 
 // inter-pass seeds (seeds_into's layout: lo[e] = w^e 2^32 for e < nlo, then
 // hi[e] = w^(4096 e) 2^32 for e < nhi, forward then inverse; wm, wim, w4m,
 // wi4m: w, w^-1, w^4096, w^-4096 in Montgomery form).
-__global__ void k_na_tables(const NaPlan row, const NaPlan col, u32* seeds, u32 nlo, u32 nhi, u32 wm, u32 wim,
-                            u32 w4m, u32 wi4m, u32 p, u32 pinv, u32 one_m) {
+__global__ void k_na_tables(const __grid_constant__ NaPlan row, const __grid_constant__ NaPlan col, u32* seeds,
+                            u32 nlo, u32 nhi, u32 wm, u32 wim, u32 w4m, u32 wi4m, u32 p, u32 pinv, u32 one_m) {
     const int nr = row.out ? 2 * row.nf + 2 : 0, nc = col.out ? 2 * col.nf + 2 : 0;
     const int ns = seeds ? (int)(2 * (nlo + nhi)) : 0;
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nr + nc + ns; t += gridDim.x * blockDim.x) {
