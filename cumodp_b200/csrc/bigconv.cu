@@ -253,7 +253,8 @@ __global__ void k_big_crt(const __grid_constant__ BigCrtArgs A) {
 // 32 at a time with ballots.  One thread per coefficient ran a serial chain of
 // 2K-1 lifts with 64-bit divisions and two accumulators in local memory; with
 // this sum and the split in one launch the 1024-term 1024-bit product went
-// from 194 to 42 us (its three 2^17-point products, 17 us each on side
+// from 194 to 42 us, and to 32-34 us with the register column passes and
+// three-level rows (its three 2^17-point products, 15-17 us each on side
 // streams, are most of what is left).
 constexpr int kBigThreadK = 4;
 constexpr int kBigWarps = 4;

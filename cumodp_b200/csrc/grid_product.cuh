@@ -14,9 +14,10 @@
 // (k_grid_mul_f), inverse columns.  With E, grids of up to 2^13 rows use the
 // 2^10- and 2^11-row column kernels.
 // Bound by integer issue like the univariate row kernels (k_row_fwd_g,
-// k_row_mul_f), whose levels these are.  Measured on B200, 2^12 x 2^12: 290 us
-// (columns 97, G's rows 52, F's rows 107, inverse columns 40); row and column
-// list transforms around two transposes took 543.
+// k_row_mul_f), whose levels these are.  Measured on B200, 2^12 x 2^12, without
+// copies: 249 us (with an event pair around each kernel: columns 77, G's rows
+// 53, F's rows 101, inverse columns 39); row and column list transforms around
+// two transposes took 543.
 #pragma once
 #include "large_product.cuh"
 

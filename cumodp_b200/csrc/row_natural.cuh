@@ -45,7 +45,10 @@ __host__ __device__ constexpr int nat_row_threads(int logl) { return 1 << (logl 
 __host__ __device__ constexpr int nat_rows(int logl) { return nat_row_threads(logl) >= 128 ? 1 : 128 / nat_row_threads(logl); }
 __host__ __device__ constexpr int nat_threads(int logl) { return nat_rows(logl) * nat_row_threads(logl); }
 // Words of shared memory between two k0 blocks: the last level's tasks step
-// through k0, so an odd step puts consecutive tasks into different banks.
+// through k0, so an odd step puts consecutive tasks into different banks (two
+// ways for rows of 2^10).  The middle level's warps cover two k0 blocks one bank
+// apart: two ways in every access (four for 2^9), 2^20 conflicts in a 2^24-point
+// transform's rows.
 __host__ __device__ constexpr int nat_stride(int logl) { return nat_row_threads(logl) + 1; }
 __host__ __device__ constexpr int nat_words(int logl) { return nat_stride(logl) << nat_plan(logl).logr[0]; }
 __host__ __device__ constexpr size_t nat_smem(int logl) { return (size_t)nat_rows(logl) * nat_words(logl) * sizeof(u32); }
