@@ -366,6 +366,7 @@ int build_plan(BatchPlan& P, const PrimeCtx& pc, cudaStream_t st) {
         return OUT_OF_MEMORY;
     }
     P.bytes += P.jobs_bytes;
+    account_bytes((long long)P.jobs_bytes);
     P.hjobs.assign(P.jobs_bytes, 0);
     P.ws_words = ws;
     if (ws) {
@@ -374,8 +375,8 @@ int build_plan(BatchPlan& P, const PrimeCtx& pc, cudaStream_t st) {
             return OUT_OF_MEMORY;
         }
         P.bytes += ws * sizeof(u32);
+        account_bytes((long long)(ws * sizeof(u32)));
     }
-    account_bytes((long long)P.bytes);
     return OK;
 }
 

@@ -8,7 +8,8 @@
 //   * the order of operations: every launch, copy, event record and wait goes to
 //     a log with its stream.
 // Two devices.  fake_set("clusters", 0) makes clusters unlaunchable,
-// fake_set("pinned_failures", n) fails the next n pinned allocations.
+// fake_set("pinned_failures", n) fails the next n pinned allocations,
+// fake_set("malloc_failure_at", n) the n-th device allocation from then on.
 #include <cuda_runtime_api.h>
 
 #include <cstdarg>
@@ -24,7 +25,7 @@
 namespace {
 
 std::recursive_mutex m;
-int g_dev = 0, g_clusters = 8, g_pinned_failures = 0;
+int g_dev = 0, g_clusters = 8, g_pinned_failures = 0, g_malloc_failure_at = 0;
 cudaError_t g_last = cudaSuccess;
 std::map<const void*, std::string> g_names;
 std::map<const void*, size_t> g_vars;
@@ -78,6 +79,7 @@ void fake_set(const char* what, int v) {
     L;
     if (!strcmp(what, "clusters")) g_clusters = v;
     if (!strcmp(what, "pinned_failures")) g_pinned_failures = v;
+    if (!strcmp(what, "malloc_failure_at")) g_malloc_failure_at = v;
     if (!strcmp(what, "clear")) g_log.clear();
 }
 int fake_log_size() { L; return (int)g_log.size(); }
@@ -125,6 +127,7 @@ cudaError_t cudaDeviceSynchronize(void) { L; log_op("devicesync dev %d", g_dev);
 cudaError_t cudaMalloc(void** p, size_t n) {
     L;
     log_op("malloc bytes %zu", n);
+    if (g_malloc_failure_at > 0 && --g_malloc_failure_at == 0) return ret(cudaErrorMemoryAllocation);
     return (*p = malloc(n)) ? cudaSuccess : ret(cudaErrorMemoryAllocation);
 }
 cudaError_t cudaMallocAsync(void** p, size_t n, cudaStream_t) { return cudaMalloc(p, n); }

@@ -326,3 +326,21 @@ print([l for l in log() if l.startswith("launch")])
     assert any("k_small_productILi13" in n and g[0] == 4096 for n, g in grids)
     assert all(g[1] in (1, 3, 4, 4000, 4096) for n, g in grids if "k_row_mul_f" in n)
     assert any("k_row_mul_f" in n and g[1] == 4 for n, g in grids)  # three products: a bucket of four
+
+
+def test_failed_batch_plans_leave_the_byte_count(fake):
+    """A batch whose plan runs out of memory half-way gives back what it took, and counts it so."""
+    before, after, code = fake("""
+L.cumodp_inject_alloc_failures.argtypes = [ctypes.c_int]
+batch((4096,) * 3)                      # tables
+batch((1 << 16,) * 2)
+before = cm.device_bytes_in_use()
+fake.fake_set(b"malloc_failure_at", 2)  # the plan's job table is had, its workspace is not
+try:
+    batch((1 << 16,) * 3)
+    code = 0
+except cm.CumodpError as e:
+    code = e.code
+print([before, cm.device_bytes_in_use(), code])
+""", CUMODP_AUTOTUNE="0")
+    assert code == 0x401 and after == before
