@@ -68,14 +68,15 @@ bool g_tune_loaded = false;
 // changes.  1 (not written to files): staged column passes, four-level rows.
 constexpr int kTunedKernels = 2;
 
-// The number of products a class of njobs is timed at: its own size rounded up,
-// to a synthetic class of at most 2^25 operand words (512 MiB with workspace).
-// A choice that wins for a few hundred products can lose for thousands: 2^13
-// points take 37.7 us on one CTA each and 35.7 in three passes for 300
-// products, 304 and 389 for 4096.
-int job_bucket(int njobs, int logn) {
+// The number of products a class of njobs is timed at: its own size rounded up
+// to a power of two, at most 256 for the splits (kind 0) and 1024 for one CTA
+// against three passes (kind 1), where what wins for a few hundred products can
+// lose for more: 2^13 points take 37.7 us on one CTA each and 35.7 in three
+// passes for 300 products, 79 and 98 for 1024, 304 and 389 for 4096.
+int job_bucket(int kind, int njobs) {
+    const int cap = kind == 0 ? 256 : 1024;
     int b = 1;
-    while (b < njobs && (long long)b << logn < 1ll << 25) b <<= 1;
+    while (b < njobs && b < cap) b <<= 1;
     return b;
 }
 
@@ -222,13 +223,15 @@ std::vector<int> legal_row_logs(int logn) {
 int tune_row_log(const PrimeCtx& pc, int logn, int njobs, int dev, cudaStream_t st, bool allow_tuning) {
     const char* off = getenv("CUMODP_AUTOTUNE");
     if (off && off[0] == '0') return default_row_log(logn);
-    const TuneKey key{device_model(dev), 0, logn, job_bucket(njobs, logn)};
+    const TuneKey key{device_model(dev), 0, logn, job_bucket(0, njobs)};
     int v;
     if (tune_lookup(key, &v)) return v;
     if (!allow_tuning) return default_row_log(logn);
     const std::vector<int> cands = legal_row_logs(logn);
     if (cands.size() <= 1) return cands.empty() ? default_row_log(logn) : cands[0];
-    const int jobs = key.bucket;
+    // timed at the class's own size (its bucket), up to 2^25 operand words: a split that wins for a few
+    // products (many small CTAs) can lose for hundreds
+    const int jobs = std::min(key.bucket, std::max(1, (int)((1ll << 25) >> logn)));
     // a refused launch would count as a slow one
     if (ensure_kernel_attrs(dev) != OK) return default_row_log(logn);
     TuneBufs T(jobs, 1ll << logn, st);
@@ -245,11 +248,11 @@ bool tune_single_cta(const PrimeCtx& pc, int logn, int njobs, int dev, cudaStrea
     if (logn < single_large_min_log() || logn > kMaxSmallLog) return logn <= kMaxSmallLog;
     const char* off = getenv("CUMODP_AUTOTUNE");
     if (off && off[0] == '0') return rule;
-    const TuneKey key{device_model(dev), 1, logn, job_bucket(njobs, logn)};
+    const TuneKey key{device_model(dev), 1, logn, job_bucket(1, njobs)};
     int v;
     if (tune_lookup(key, &v)) return v != 0;
     if (!allow_tuning) return rule;
-    const int jobs = key.bucket;
+    const int jobs = key.bucket;  // up to 1024 products: 128 MiB of operands and workspace at 2^13, 256 at 2^14
     if (ensure_kernel_attrs(dev) != OK) return rule;
     TuneBufs T(jobs, 1ll << logn, st);
     if (!T.ok) return rule;
