@@ -531,12 +531,9 @@ int StreamOrder::mark(cudaStream_t st) {
 
 int StreamOrder::enter(cudaStream_t st, bool* replace) {
     if (replace) *replace = false;
-    // one stream alone: nothing to wait for and nothing that leave() would change
-    // (the library's own streams need not be asked for their id)
+    // one of the library's own streams alone: nothing to wait for and nothing
+    // that leave() would change
     skip_ = used_ && !shared_ && last_own_ && st == last_stream_;
-    if (skip_) return OK;
-    cudaError_t e = cudaStreamGetId(st, &id_);
-    skip_ = e == cudaSuccess && used_ && !shared_ && id_ == last_;
     if (skip_) return OK;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     // (the legacy stream answers with an error while a blocking stream is captured)
@@ -545,6 +542,9 @@ int StreamOrder::enter(cudaStream_t st, bool* replace) {
         cs = cudaStreamCaptureStatusActive;
     }
     skip_ = cs != cudaStreamCaptureStatusNone;
+    if (skip_) return OK;
+    cudaError_t e = cudaStreamGetId(st, &id_);  // (ends a capture: not before the question above)
+    skip_ = e == cudaSuccess && used_ && !shared_ && id_ == last_;
     if (skip_) return OK;
     if (e == cudaSuccess && replace && used_ && id_ != last_) {
         if (!marked_ && last_own_) {

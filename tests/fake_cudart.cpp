@@ -177,6 +177,10 @@ cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) {
 cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaStreamGetId(cudaStream_t s, unsigned long long* id) {
     L;
+    if (g_capturing[s]) {  // as the runtime does: the query ends the capture
+        log_op("capture of stream %p invalidated", (void*)s);
+        return ret(cudaErrorStreamCaptureUnsupported);
+    }
     if (!g_stream_ids.count(s)) g_stream_ids[s] = g_next++;
     *id = g_stream_ids[s];
     return cudaSuccess;

@@ -97,3 +97,22 @@ def test_interleaved_calls_on_two_streams(cm, kinds):
     torch.cuda.synchronize()
     for (_, out), w in zip(jobs, want):
         assert torch.equal(out, w)
+
+
+@pytest.mark.parametrize("kind", ["product", "fft", "bivariate", "exact"])
+def test_captured_calls_replay(cm, kind):
+    """After a first call the others can be captured into a graph, scratch and all; replays give the same result."""
+    s = torch.cuda.Stream()
+    run, out = _make(cm, kind, 3)
+    run(s.cuda_stream)
+    torch.cuda.synchronize()
+    want = out.clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=s):
+        run(s.cuda_stream)
+        run(s.cuda_stream)
+    out.fill_(-1)
+    for _ in range(3):
+        graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, want)
