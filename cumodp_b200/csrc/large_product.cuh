@@ -728,11 +728,16 @@ __global__ void __launch_bounds__(rowsplit_threads(L2), rowsplit_ctas(L2)) k_row
     const u32 k1 = col_slot_to_k1(s, A.colpl, A.l1);
     const u32 p = A.pk.p, p2 = A.pk.p2;
     u32* row = J.wb + (size_t)s * n2;
+    // F's row kernel reads pass A's columns of F before its own wait, so its
+    // launch is allowed only after a wait for them here; one thread does, before
+    // its share of the tables
+    if (threadIdx.x == 0) {
+        pdl_wait();
+        pdl_trigger();
+    }
     if constexpr (RowTab<L2>::USE) row_tab_fetch<L2, T>(tab, wp, A, s, k1, false);
     else row_slot_factors<L2>(A, k1, bf, nullptr);
     pdl_wait();  // pass A's columns of G
-    // after the wait: F's row kernel reads pass A's columns of F before its own
-    pdl_trigger();
     if constexpr (RowTab<L2>::USE) {
         row_level0_fwd<L2, T>(sm, row, A, tab);
     } else {

@@ -87,8 +87,8 @@ int seeds_into(u32 p, u32 root, int logn, u32* out, size_t cap);
 // come on different streams.  enter() makes st follow the user before, leave()
 // marks where this one's work on st ends.  A stream needs no wait for itself
 // (streams are told apart by their id, which a destroyed stream's handle does
-// not carry on), and a program with one stream pays nothing: an event after
-// every call cost the calls of 17-40 us on one stream 0.5-1.5 us each.  So the
+// not carry on), and a program with one stream pays two queries of it (0.2 us):
+// an event after every call cost the calls of 17-40 us 0.5-1.5 us each.  So the
 // first user's calls are not marked, and when another stream comes they cannot
 // be waited for any more (their stream may be gone): enter() then sets
 // *replace, the caller gives st another copy of the thing (or waits for the
