@@ -127,6 +127,22 @@ int prepared(const PrimeCtx& pc, int logn, int dev, Prepared* out) {
 
 }  // namespace
 
+namespace {
+
+// The library code of a launch; one that was refused for resources (the room
+// the set-up found for a cluster is gone) leaves *launched false and no error,
+// and the caller takes the other kernels.
+int launch_result(cudaError_t e, bool* launched) {
+    *launched = e == cudaSuccess;
+    if (e == cudaErrorLaunchOutOfResources || e == cudaErrorInvalidClusterSize) {
+        cudaGetLastError();
+        return OK;
+    }
+    return cuda_err(e);
+}
+
+}  // namespace
+
 int latency_usable(const PrimeCtx& pc, int logn, int dev, bool* usable) {
     Prepared P{};
     const int err = prepared(pc, logn, dev, &P);
@@ -145,8 +161,7 @@ int latency_mul(const PrimeCtx& pc, int logn, int dev, const ProdJob& job, cudaS
     const bool tr = pass_timing_begin(st, &e0);
     const cudaError_t ce = kForms[logn - kMinLog].one(a, st);
     if (tr) pass_timing_end(st, kName[logn - kMinLog], e0);
-    *launched = ce == cudaSuccess;
-    return cuda_err(ce);
+    return launch_result(ce, launched);
 }
 
 namespace {
@@ -184,8 +199,7 @@ int latency_mul_primes(const u32* primes, int np, int dev, const u32* a, int la,
     if (np == 4 && ce == cudaSuccess)
         ce = form.one(LatArgs<1>{{P[3].pr}, a + 3 * astride, b + 3 * bstride, h + 3 * hstride, la, lb, lh, 0, 0, 0}, st);
     if (tr) pass_timing_end(st, kName[logn - kMinLog], e0);
-    *launched = ce == cudaSuccess;
-    return cuda_err(ce);
+    return launch_result(ce, launched);
 }
 
 int latency_mul_i64(const u32* primes, int np, int dev, const long long* a, int la, const long long* b, int lb, u32* h,
@@ -204,8 +218,7 @@ int latency_mul_i64(const u32* primes, int np, int dev, const long long* a, int 
         np == 2 ? form.wide2(LatArgs<2>{{P[0].pr, P[1].pr}, a, b, h, la, lb, lh, 0, 0, lh}, st)
                 : form.wide3(LatArgs<3>{{P[0].pr, P[1].pr, P[2].pr}, a, b, h, la, lb, lh, 0, 0, lh}, st);
     if (tr) pass_timing_end(st, kName[logn - kMinLog], e0);
-    *launched = ce == cudaSuccess;
-    return cuda_err(ce);
+    return launch_result(ce, launched);
 }
 
 namespace {

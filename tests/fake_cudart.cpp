@@ -7,7 +7,8 @@
 //     for that kernel (48 KiB unless raised) is refused;
 //   * the order of operations: every launch, copy, event record and wait goes to
 //     a log with its stream.
-// Two devices.  fake_set("clusters", 0) makes clusters unlaunchable,
+// Two devices.  fake_set("clusters", 0) makes clusters unlaunchable by the
+// occupancy query, fake_set("refuse_clusters", 1) their launches alone,
 // fake_set("pinned_failures", n) fails the next n pinned allocations,
 // fake_set("malloc_failure_at", n) the n-th device allocation from then on.
 #include <cuda_runtime_api.h>
@@ -25,7 +26,7 @@
 namespace {
 
 std::recursive_mutex m;
-int g_dev = 0, g_clusters = 8, g_pinned_failures = 0, g_malloc_failure_at = 0;
+int g_dev = 0, g_clusters = 8, g_pinned_failures = 0, g_malloc_failure_at = 0, g_refuse_clusters = 0;
 cudaError_t g_last = cudaSuccess;
 std::map<const void*, std::string> g_names;
 std::map<const void*, size_t> g_vars;
@@ -79,6 +80,7 @@ void fake_set(const char* what, int v) {
     L;
     if (!strcmp(what, "clusters")) g_clusters = v;
     if (!strcmp(what, "pinned_failures")) g_pinned_failures = v;
+    if (!strcmp(what, "refuse_clusters")) g_refuse_clusters = v;
     if (!strcmp(what, "malloc_failure_at")) g_malloc_failure_at = v;
     if (!strcmp(what, "clear")) g_log.clear();
 }
@@ -250,6 +252,8 @@ cudaError_t cudaLaunchKernel(const void* f, dim3 g, dim3 b, void**, size_t smem,
 }
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void**) {
     L;
+    for (unsigned i = 0; g_refuse_clusters && i < c->numAttrs; ++i)
+        if (c->attrs[i].id == cudaLaunchAttributeClusterDimension) return ret(cudaErrorLaunchOutOfResources);
     return launch(f, c->gridDim, c->blockDim, c->dynamicSmemBytes, c->stream);
 }
 }

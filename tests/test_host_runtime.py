@@ -344,3 +344,22 @@ except cm.CumodpError as e:
 print([before, cm.device_bytes_in_use(), code])
 """, CUMODP_AUTOTUNE="0")
     assert code == 0x401 and after == before
+
+
+def test_refused_cluster_launches_fall_back(fake):
+    """Where the set-up found room for a cluster and its launch is refused for resources all the same, the other
+    kernels take the product."""
+    log = fake("""
+product(14)
+fake.fake_set(b"refuse_clusters", 1)
+fake.fake_set(b"clear", 0)
+product(14)
+exact(8192)
+big(400, 4)
+x = np.ones(30000, np.int32)
+cm.fftmul_uni(x, x, P)
+print(log())
+""")
+    names = " ".join(x for x in log if x.startswith("launch"))
+    assert "k_row_mul_f" in names and "k_residues" in names and "ELi16ELi" not in names  # no 16-CTA form
+    assert any(x.startswith("graph") for x in log)
